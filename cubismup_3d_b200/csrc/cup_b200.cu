@@ -26,6 +26,7 @@
 #include "advect_f2.cuh"
 #include "common.cuh"
 #include "dht.cuh"
+#include "pfft.cuh"
 #include "pressure_zq.cuh"
 #include "ops.cuh"
 #include "stencil.cuh"
@@ -708,36 +709,49 @@ int ilog2(int n) {
 }
 bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
+const long double kPi = 3.141592653589793238462643383279502884L;
+
 template <int M>
-void build_table_M(std::vector<double2>& t64, std::vector<float2>& t32) {
+void build_table_M(std::vector<double2>& t64) {
   using Pl = FFTPlan<M>;
-  const int L = Pl::table_len();
-  t64.assign(L, double2{0, 0});
-  t32.assign(L, float2{0, 0});
-  const long double PI = 3.141592653589793238462643383279502884L;
-  auto put = [&](int i, long double ang) {
-    t64[i] = double2{(double)cosl(ang), (double)sinl(ang)};
-    t32[i] = float2{(float)cosl(ang), (float)sinl(ang)};
-  };
+  t64.assign(Pl::table_len(), double2{0, 0});
+  auto put = [&](int i, long double ang) { t64[i] = double2{(double)cosl(ang), (double)sinl(ang)}; };
   for (int s = 1; s < Pl::nstages; ++s) {
     const int R = Pl::radix(s), Ns = Pl::ns(s), off = Pl::tw_off(s);
     for (int r = 0; r < R; ++r)
-      for (int j = 0; j < Ns; ++j) put(off + r * Ns + j, -2.0L * PI * r * j / ((long double)Ns * R));
+      for (int j = 0; j < Ns; ++j) put(off + r * Ns + j, -2.0L * kPi * r * j / ((long double)Ns * R));
   }
-  for (int k = 0; k <= M / 2; ++k) put(Pl::post_off() + k, -2.0L * PI * k / (2.0L * M));
+  for (int k = 0; k <= M / 2; ++k) put(Pl::post_off() + k, -2.0L * kPi * k / (2.0L * M));
   if (M == 128)
     for (int r = 0; r < 8; ++r)
-      for (int j = 0; j < 16; ++j) put(Pl::r16_off() + 16 * r + j, -2.0L * PI * r * j / (long double)M);
+      for (int j = 0; j < 16; ++j) put(Pl::r16_off() + 16 * r + j, -2.0L * kPi * r * j / (long double)M);
 }
 
-void build_table(int N, std::vector<double2>& t64, std::vector<float2>& t32) {
+// Tables of the packed transforms (pfft.cuh): the twiddles W_M^(k1 t) and
+// cos(2 pi k / M) of the bin at each position (rows: the swizzled order); c is
+// the reference's cos(4 pi k / N), k < N.
+template <int M>
+void build_ptable_M(const std::vector<double>& c, bool rows, std::vector<double2>& t64, std::vector<float2>& t32,
+                    std::vector<double>& pc) {
+  using P = PPlan<M>;
+  t64.resize(M), t32.resize(M), pc.resize(M);
+  for (int k1 = 0; k1 < P::R1; ++k1)
+    for (int t = 0; t < P::R2; ++t) {
+      const long double a = -2.0L * kPi * k1 * t / (long double)M;
+      t64[k1 * P::R2 + t] = double2{(double)cosl(a), (double)sinl(a)};
+      t32[k1 * P::R2 + t] = float2{(float)cosl(a), (float)sinl(a)};
+    }
+  for (int i = 0; i < M; ++i) pc[i] = c[rows ? P::row_bin(i) : P::bin(i)];
+}
+
+void build_tables(int N, const std::vector<double>& c, bool rows, std::vector<double2>& t64, std::vector<double2>& p64,
+                  std::vector<float2>& p32, std::vector<double>& pc) {
   switch (N / 2) {
-    case 8: build_table_M<8>(t64, t32); break;
-    case 16: build_table_M<16>(t64, t32); break;
-    case 32: build_table_M<32>(t64, t32); break;
-    case 64: build_table_M<64>(t64, t32); break;
-    case 128: build_table_M<128>(t64, t32); break;
-    case 256: build_table_M<256>(t64, t32); break;
+    case 8: build_table_M<8>(t64), build_ptable_M<8>(c, rows, p64, p32, pc); break;
+    case 16: build_table_M<16>(t64), build_ptable_M<16>(c, rows, p64, p32, pc); break;
+    case 32: build_table_M<32>(t64), build_ptable_M<32>(c, rows, p64, p32, pc); break;
+    case 64: build_table_M<64>(t64), build_ptable_M<64>(c, rows, p64, p32, pc); break;
+    case 128: build_table_M<128>(t64), build_ptable_M<128>(c, rows, p64, p32, pc); break;
     default: break;
   }
 }
@@ -776,9 +790,16 @@ struct cup_handle {
   int* derr = nullptr;
   // FFT tables (per axis) and spectral cos tables
   double2* tw64[3] = {nullptr, nullptr, nullptr};
-  float2* tw32[3] = {nullptr, nullptr, nullptr};
+  // packed transforms of the pressure solve (pfft.cuh): twiddles and the
+  // cosines in spectrum order, per axis
+  double2* ptw64[3] = {nullptr, nullptr, nullptr};
+  float2* ptw32[3] = {nullptr, nullptr, nullptr};
+  double* pcos[3] = {nullptr, nullptr, nullptr};
   double *cosx = nullptr, *cosy = nullptr, *cosz = nullptr;
   double norm_factor = 0;
+  double pnorm = 0;  // of the packed transforms: 4 / h / (Mx My Mz)
+  void* tables = nullptr;       // the one allocation behind the tables above
+  double* cosy_win = nullptr;   // cosy of cup_set_spectral_window
   // spectral window of a y-split pencil of a decomposed grid (cup_set_spectral_window):
   // the global y length of the cos table and of the null modes, and this handle's first y
   int spec_ny = 0, spec_y0 = 0;
@@ -1017,63 +1038,17 @@ int launch_stream(cup_handle* H, const char* name, const void* const* fields, co
   return CUP_OK;
 }
 
-template <typename R>
-const typename Cplx<R>::T* table(cup_handle* H, int axis);
-template <>
-const double2* table<double>(cup_handle* H, int axis) {
-  return H->tw64[axis];
-}
-template <>
-const float2* table<float>(cup_handle* H, int axis) {
-  return H->tw32[axis];
-}
-
-template <int M, typename R, class Prod, class Cons>
-int launch_rows_M(cup_handle* H, const char* name, const Prod& prod, const Cons& cons, const int* skip) {
+// Pipelined Hartley x pass (k_dht_rows_pipe): rows of `buf` transformed in place.
+template <int M>
+int launch_rows_pipe_M(cup_handle* H, const char* name, double* buf) {
   constexpr int N = 2 * M, TPL = M / 8;
   constexpr bool PAD = FFTPlan<M>::nstages > 1;
-  // 256 threads per CTA (16 rows of 256-long lines; 8- and 4-row tiles measured no faster)
+  constexpr int NB = 2;
   const int lpc = 256 / TPL;
   const int nrows = H->ny * H->nz;
-  const size_t smem = (size_t)lpc * N * sizeof(R) + (PAD ? (size_t)lpc * 2 * (M + M / 8) * sizeof(R) : 0) +
-                      FFTPlan<M>::rows_table_len() * sizeof(typename Cplx<R>::T) + 128;
-  auto kern = k_dht_rows<M, R, Prod, Cons>;
-  int bpsm = 0;
-  int rc = prepare_kernel(H, kern, smem, lpc * TPL, &bpsm);
-  if (rc) return rc;
-  const int grid = (nrows + lpc - 1) / lpc;
-  return launch_named(H, name, [&]() -> int {
-    klaunch(H, kern, grid, lpc * TPL, smem, prod, cons, nrows, lpc, table<R>(H, 0), H->derr, skip);
-    CKL();
-    return CUP_OK;
-  });
-}
-
-template <typename R, class Prod, class Cons>
-int launch_rows(cup_handle* H, const char* name, const Prod& prod, const Cons& cons, const int* skip) {
-  switch (H->nx / 2) {
-    case 8: return launch_rows_M<8, R>(H, name, prod, cons, skip);
-    case 16: return launch_rows_M<16, R>(H, name, prod, cons, skip);
-    case 32: return launch_rows_M<32, R>(H, name, prod, cons, skip);
-    case 64: return launch_rows_M<64, R>(H, name, prod, cons, skip);
-    case 128: return launch_rows_M<128, R>(H, name, prod, cons, skip);
-    case 256: return launch_rows_M<256, R>(H, name, prod, cons, skip);
-  }
-  return fail(H, CUP_ERR_ARG, "unsupported nx %d", H->nx);
-}
-
-// Pipelined x pass (k_dht_rows_pipe): rows of `in` transformed into `out`.
-// FP32: three tile buffers; FP64: two.
-template <int M, typename R>
-int launch_rows_pipe_M(cup_handle* H, const char* name, const R* in, R* out, const int* skip) {
-  constexpr int N = 2 * M, TPL = M / 8;
-  constexpr bool PAD = FFTPlan<M>::nstages > 1;
-  constexpr int NB = sizeof(R) == 4 ? 3 : 2;
-  const int lpc = 256 / TPL;  // (8- and 4-row tiles measured 37.4 and 38.6 against 37.3 us at 256^3, FP32)
-  const int nrows = H->ny * H->nz;
-  const size_t smem = (size_t)NB * lpc * N * sizeof(R) + (PAD ? (size_t)lpc * 2 * (M + M / 8) * sizeof(R) : 0) +
-                      FFTPlan<M>::rows_table_len() * sizeof(typename Cplx<R>::T) + NB * sizeof(uint64_t) + 128;
-  auto kern = k_dht_rows_pipe<M, R, NB>;
+  const size_t smem = (size_t)NB * lpc * N * sizeof(double) + (PAD ? (size_t)lpc * 2 * (M + M / 8) * sizeof(double) : 0) +
+                      FFTPlan<M>::rows_table_len() * sizeof(double2) + NB * sizeof(uint64_t) + 128;
+  auto kern = k_dht_rows_pipe<M, double, NB>;
   const int threads = lpc * TPL;
   int bpsm = 0;
   int rc = prepare_kernel(H, kern, smem, threads, &bpsm);
@@ -1081,88 +1056,39 @@ int launch_rows_pipe_M(cup_handle* H, const char* name, const R* in, R* out, con
   const int ntiles = (nrows + lpc - 1) / lpc;
   const int grid = std::min(ntiles, bpsm * H->num_sms);
   return launch_named(H, name, [&]() -> int {
-    klaunch(H, kern, grid, threads, smem, in, out, nrows, lpc, table<R>(H, 0), H->derr, skip);
+    klaunch(H, kern, grid, threads, smem, (const double*)buf, buf, nrows, lpc, (const double2*)H->tw64[0], H->derr,
+            (const int*)nullptr);
     CKL();
     return CUP_OK;
   });
 }
 
-template <typename R>
-int launch_rows_pipe(cup_handle* H, const char* name, const R* in, R* out, const int* skip) {
+int launch_rows_pipe(cup_handle* H, const char* name, double* buf) {
   switch (H->nx / 2) {
-    case 8: return launch_rows_pipe_M<8, R>(H, name, in, out, skip);
-    case 16: return launch_rows_pipe_M<16, R>(H, name, in, out, skip);
-    case 32: return launch_rows_pipe_M<32, R>(H, name, in, out, skip);
-    case 64: return launch_rows_pipe_M<64, R>(H, name, in, out, skip);
-    case 128: return launch_rows_pipe_M<128, R>(H, name, in, out, skip);
-    case 256: return launch_rows_pipe_M<256, R>(H, name, in, out, skip);
+    case 8: return launch_rows_pipe_M<8>(H, name, buf);
+    case 16: return launch_rows_pipe_M<16>(H, name, buf);
+    case 32: return launch_rows_pipe_M<32>(H, name, buf);
+    case 64: return launch_rows_pipe_M<64>(H, name, buf);
+    case 128: return launch_rows_pipe_M<128>(H, name, buf);
   }
   return fail(H, CUP_ERR_ARG, "unsupported nx %d", H->nx);
 }
 
-// Pipelined last x pass of a correction solve (k_dht_rows_addp_pipe): the
-// FP64 inverse of `in` added into p minus the class means of p.
-template <int M>
-int launch_rows_addp_M(cup_handle* H, const char* name, const double* in, double* p, const int* skip) {
-  constexpr int N = 2 * M, TPL = M / 8, NB = 2;
-  constexpr bool PAD = FFTPlan<M>::nstages > 1;
-  // 64 threads per CTA (4 rows of 256-long lines, several CTAs per SM): 74 us at
-  // 256^3 against 81 us with 8-row and 88 us with 16-row tiles
-  const int lpc = std::max(1, 64 / TPL);
-  const int nrows = H->ny * H->nz;
-  const size_t smem = (size_t)2 * NB * lpc * N * sizeof(double) +
-                      (PAD ? (size_t)lpc * 2 * (M + M / 8) * sizeof(double) : 0) +
-                      FFTPlan<M>::rows_table_len() * sizeof(double2) + NB * sizeof(uint64_t) + 8 * sizeof(double) + 128;
-  auto kern = k_dht_rows_addp_pipe<M, NB>;
-  const int threads = lpc * TPL;
-  int bpsm = 0;
-  int rc = prepare_kernel(H, kern, smem, threads, &bpsm);
-  if (rc) return rc;
-  const int ntiles = (nrows + lpc - 1) / lpc;
-  const int grid = std::min(ntiles, bpsm * H->num_sms);
-  return launch_named(H, name, [&]() -> int {
-    klaunch(H, kern, grid, threads, smem, in, p, (const double*)H->dstate->cmean, ilog2(H->ny), nrows, lpc,
-            table<double>(H, 0), H->derr, skip);
-    CKL();
-    return CUP_OK;
-  });
-}
-
-int launch_rows_addp(cup_handle* H, const char* name, const double* in, double* p, const int* skip) {
-  switch (H->nx / 2) {
-    case 8: return launch_rows_addp_M<8>(H, name, in, p, skip);
-    case 16: return launch_rows_addp_M<16>(H, name, in, p, skip);
-    case 32: return launch_rows_addp_M<32>(H, name, in, p, skip);
-    case 64: return launch_rows_addp_M<64>(H, name, in, p, skip);
-    case 128: return launch_rows_addp_M<128>(H, name, in, p, skip);
-  }
-  return fail(H, CUP_ERR_ARG, "unsupported nx %d", H->nx);
-}
-
-template <int M, typename R, int AXIS, bool DIVIDE, typename RIN = R>
-int launch_cols_M(cup_handle* H, RIN* in, R* out, const int* skip) {
-  // W x-columns per tile (FP32: 128-B rows of a tile, FP64: 128 B), NB = 3 tile buffers
-  // 256-long lines: the 8-thread plan (radix 16, then radix 8 fused with the
-  // split), also for the mixed-precision z pass (the 16-thread plan measured
-  // 89 against 75 us there at 256^3; that pass now runs k_dht_z_mixed for
-  // 256-long lines, this kernel for shorter ones)
+// Hartley y or z pass (z: with the spectral divide and the inverse when DIVIDE), in place on buf.
+template <int M, int AXIS, bool DIVIDE>
+int launch_cols_M(cup_handle* H, double* buf) {
+  // 16 x-columns per tile (128-B rows), NB tile buffers; 256-long lines: the
+  // 8-thread plan (radix 16, then radix 8 fused with the split)
   constexpr bool T8 = M == 128;
-  // (a 3-deep ring for the mixed z pass, 2 CTAs per SM: 85 against 70 us)
-  constexpr int N = 2 * M, TPL = T8 ? 8 : M / 8, NB = T8 ? 2 : 3;
-  // (8-column FP64 tiles measured slower: 90 against 70 us for the mixed z pass, 58 against 50 for the y pass)
-  constexpr int W = sizeof(R) == 4 ? 32 : 16;
+  constexpr int N = 2 * M, TPL = T8 ? 8 : M / 8, NB = T8 ? 2 : 3, W = 16;
   if (AXIS == 2 && H->cfg.z_halo)
     return fail(H, CUP_ERR_STATE, "a z-slab handle has no z transform (the Poisson solve runs over the ranks)");
-  if (H->nx % W) return fail(H, CUP_ERR_ARG, "nx must be a multiple of %d for this precision", W);
-  CUtensorMap map_in, map_out;
-  int rc = make_map(H, &map_in, in, tma_dtype<RIN>(), sizeof(RIN), W, AXIS == 1 ? N : 1, AXIS == 2 ? N : 1);
-  if (!rc) rc = make_map(H, &map_out, out, tma_dtype<R>(), sizeof(R), W, AXIS == 1 ? N : 1, AXIS == 2 ? N : 1);
+  CUtensorMap map;
+  int rc = make_map(H, &map, buf, tma_dtype<double>(), sizeof(double), W, AXIS == 1 ? N : 1, AXIS == 2 ? N : 1);
   if (rc) return rc;
-  constexpr bool WIDEN = sizeof(RIN) < sizeof(R);
-  const size_t smem = (size_t)NB * N * W * sizeof(R) + FFTPlan<M>::table_len() * sizeof(typename Cplx<R>::T) +
-                      (WIDEN ? FFTPlan<M>::table_len() * sizeof(typename Cplx<RIN>::T) : 0) +
+  const size_t smem = (size_t)NB * N * W * sizeof(double) + FFTPlan<M>::table_len() * sizeof(double2) +
                       NB * sizeof(uint64_t) + (DIVIDE ? (M / 2 + 1) * sizeof(double) : 0) + 128;
-  auto kern = k_dht_cols_pipe<M, R, AXIS, DIVIDE, W, NB, RIN, T8>;
+  auto kern = k_dht_cols_pipe<M, double, AXIS, DIVIDE, W, NB, T8>;
   const int threads = W * TPL;
   int bpsm = 0;
   rc = prepare_kernel(H, kern, smem, threads, &bpsm);
@@ -1171,109 +1097,200 @@ int launch_cols_M(cup_handle* H, RIN* in, R* out, const int* skip) {
   const int ntiles = ntx * (AXIS == 1 ? H->nz : H->ny);
   const int grid = std::min(ntiles, bpsm * H->num_sms);
   SpectralParams sp{H->cosx, H->cosy, H->cosz, H->norm_factor, H->nx, H->spec_ny, H->nz, H->spec_y0};
-  const bool inv64 = H->fp32 && sizeof(R) == 8;  // FP64 inverse pass of a mixed-precision correction solve
-  const char* name = AXIS == 1 ? (inv64 ? "dht_y_f64" : "dht_y")
-                               : (sizeof(RIN) < sizeof(R) ? "dht_z_solve_mixed" : "dht_z_solve");
-  return launch_named(H, name, [&]() -> int {
-    klaunch(H, kern, grid, threads, smem, map_in, map_out, ntx, ntiles, table<R>(H, AXIS), table<RIN>(H, AXIS),
-                                             sp, H->derr, skip);
+  return launch_named(H, AXIS == 1 ? "dht_y" : "dht_z_solve", [&]() -> int {
+    klaunch(H, kern, grid, threads, smem, map, ntx, ntiles, (const double2*)H->tw64[AXIS], sp, H->derr,
+            (const int*)nullptr);
     CKL();
     return CUP_OK;
   });
 }
 
-template <typename R, int AXIS, bool DIVIDE, typename RIN = R>
-int launch_cols(cup_handle* H, RIN* in, R* out, const int* skip) {
+template <int AXIS, bool DIVIDE>
+int launch_cols(cup_handle* H, double* buf) {
   const int N = AXIS == 1 ? H->ny : H->nz;
   switch (N / 2) {
-    case 8: return launch_cols_M<8, R, AXIS, DIVIDE, RIN>(H, in, out, skip);
-    case 16: return launch_cols_M<16, R, AXIS, DIVIDE, RIN>(H, in, out, skip);
-    case 32: return launch_cols_M<32, R, AXIS, DIVIDE, RIN>(H, in, out, skip);
-    case 64: return launch_cols_M<64, R, AXIS, DIVIDE, RIN>(H, in, out, skip);
-    case 128: return launch_cols_M<128, R, AXIS, DIVIDE, RIN>(H, in, out, skip);
+    case 8: return launch_cols_M<8, AXIS, DIVIDE>(H, buf);
+    case 16: return launch_cols_M<16, AXIS, DIVIDE>(H, buf);
+    case 32: return launch_cols_M<32, AXIS, DIVIDE>(H, buf);
+    case 64: return launch_cols_M<64, AXIS, DIVIDE>(H, buf);
+    case 128: return launch_cols_M<128, AXIS, DIVIDE>(H, buf);
   }
   return fail(H, CUP_ERR_ARG, "unsupported line length %d", N);
 }
 
-// Mixed-precision z pass of 256-long lines with a narrow input ring
-// (k_dht_z_mixed): W columns per tile, NBN FP32 input buffers and one FP64
-// buffer per CTA. Measured at 256^3: 58.2 us with W = 32, NBN = 1 (two CTAs
-// per SM), 64.2 with W = 16, NBN = 1 (four), 69.2 with W = 16, NBN = 2
-// (three), against 70.4 for the two-FP64-buffer ring of k_dht_cols_pipe.
-template <int W, int NBN>
-int launch_z_mixed(cup_handle* H, float* in, double* out, const int* skip) {
-  constexpr int M = 128, N = 2 * M;
-  using Pl = FFTPlan<M>;
-  if (H->cfg.z_halo)
-    return fail(H, CUP_ERR_STATE, "a z-slab handle has no z transform (the Poisson solve runs over the ranks)");
-  if (H->nz != N) return fail(H, CUP_ERR_ARG, "the narrow-ring z pass needs 256-long z lines");
-  if (H->nx % W) return fail(H, CUP_ERR_ARG, "nx must be a multiple of %d for this precision", W);
-  CUtensorMap map_in, map_out;
-  int rc = make_map(H, &map_in, in, tma_dtype<float>(), sizeof(float), W, 1, N);
-  if (!rc) rc = make_map(H, &map_out, out, tma_dtype<double>(), sizeof(double), W, 1, N);
-  if (rc) return rc;
-  constexpr int TN = Pl::table_len() - Pl::post_off();
-  const size_t smem = (size_t)N * W * sizeof(double) + (size_t)NBN * N * W * sizeof(float) +
-                      (size_t)TN * (sizeof(double2) + sizeof(float2)) + NBN * sizeof(uint64_t) +
-                      (M / 2 + 1) * sizeof(double) + 128;
-  auto kern = k_dht_z_mixed<W, NBN>;
-  const int threads = W * 8;
+// ---- the pressure solve's passes (pfft.cuh) --------------------------------
+// Calls fn<M>() for the line length N = 2 M.
+#define PFFT_DISPATCH(N, call)                                          \
+  switch ((N) / 2) {                                                    \
+    case 8: { constexpr int M = 8; return call; }                       \
+    case 16: { constexpr int M = 16; return call; }                     \
+    case 32: { constexpr int M = 32; return call; }                     \
+    case 64: { constexpr int M = 64; return call; }                     \
+    case 128: { constexpr int M = 128; return call; }                   \
+  }                                                                     \
+  return fail(H, CUP_ERR_ARG, "unsupported line length %d", (int)(N))
+
+template <typename S>
+const typename Cplx<S>::T* ptable(cup_handle* H, int axis) {
+  if constexpr (sizeof(S) == 8) return H->ptw64[axis];
+  else return H->ptw32[axis];
+}
+
+// x pass: MODE as k_pfft_x; rev walks the tiles backwards (a pass that starts
+// where the pass before it ended finds that part of the array in L2: at 256^3
+// FP64 the y pass took 43.0 against 47.1 us and the last x pass 45.2 against 51.1).
+// Warps per CTA and buffers per warp as measured at 256^3: FP32 forward 27.4 us
+// (2 to 8 warps and 2 to 4 buffers within 1 us), FP64 45 us, with p 65.5 us.
+template <int M, typename S, int MODE>
+int launch_pfft_x_M(cup_handle* H, const char* name, const S* in, S* out, S* out2, int rev, const int* skip) {
+  constexpr bool ADDP = MODE == PROW_INV_ADDP;
+  constexpr int NB = sizeof(S) == 4 ? 3 : 2, WARPS = ADDP ? 2 : 4;
+  constexpr bool LATE = sizeof(S) == 4 || ADDP;
+  using Rw = PRows<M>;
+  const size_t smem = (size_t)WARPS * NB * Rw::ELEMS * (ADDP ? 2 : 1) * sizeof(S) + M * sizeof(typename Cplx<S>::T) +
+                      WARPS * NB * sizeof(uint64_t) + 8 * sizeof(double) + 128;
+  auto kern = k_pfft_x<M, S, MODE, NB, WARPS, LATE>;
   int bpsm = 0;
-  rc = prepare_kernel(H, kern, smem, threads, &bpsm);
+  int rc = prepare_kernel(H, kern, smem, 32 * WARPS, &bpsm);
   if (rc) return rc;
-  const int ntx = H->nx / W;
-  const int ntiles = ntx * H->ny;
-  const int grid = std::min(ntiles, bpsm * H->num_sms);
-  SpectralParams sp{H->cosx, H->cosy, H->cosz, H->norm_factor, H->nx, H->spec_ny, H->nz, H->spec_y0};
-  return launch_named(H, "dht_z_solve_mixed", [&]() -> int {
-    klaunch(H, kern, grid, threads, smem, map_in, map_out, ntx, ntiles, table<double>(H, 2), table<float>(H, 2), sp,
-            H->derr, skip);
+  const int ntiles = H->ny * H->nz / Rw::ROWS;
+  const int grid = std::min((ntiles + WARPS - 1) / WARPS, bpsm * H->num_sms);
+  return launch_named(H, name, [&]() -> int {
+    klaunch(H, kern, grid, 32 * WARPS, smem, in, out, out2, (const double*)H->dstate->cmean, ilog2(H->ny), ntiles, rev,
+            ptable<S>(H, 0), H->derr, skip);
     CKL();
     return CUP_OK;
   });
 }
+template <typename S, int MODE>
+int launch_pfft_x(cup_handle* H, const char* name, const S* in, S* out, S* out2, int rev, const int* skip) {
+  PFFT_DISPATCH(H->nx, (launch_pfft_x_M<M, S, MODE>(H, name, in, out, out2, rev, skip)));
+}
 
-// p = H(f . H(work)) over the three axes, in place on `work`; the last x
-// pass writes to `out` (may equal work).
-// The y, z (+ divide + inverse) and y passes, in place on `work`.
-template <typename R>
-int fft_middle(cup_handle* H, R* work, const int* skip) {
+// y pass in place. L: double (16-column tiles) or F2 (FP32, 32 columns in pairs).
+template <int M, typename L, bool INV>
+int launch_pfft_y_M(cup_handle* H, const char* name, typename Lane<L>::S* buf, int rev, const int* skip) {
+  using S = typename Lane<L>::S;
+  constexpr int W = sizeof(S) == 8 ? 16 : 32, NB = 2, N = 2 * M;
+  using Tile = PTile<M, L, W>;
+  if (H->nx % W) return fail(H, CUP_ERR_ARG, "nx must be a multiple of %d for this precision", W);
+  CUtensorMap map;
+  int rc = make_map(H, &map, buf, tma_dtype<S>(), sizeof(S), W, N, Tile::P);
+  if (rc) return rc;
+  const size_t smem = (size_t)NB * N * W * Tile::P * sizeof(S) + M * sizeof(typename Cplx<S>::T) +
+                      NB * sizeof(uint64_t) + 128;
+  auto kern = k_pfft_y<M, L, INV, W, NB>;
+  int bpsm = 0;
+  if ((rc = prepare_kernel(H, kern, smem, Tile::THREADS, &bpsm))) return rc;
+  const int ntx = H->nx / W, ntiles = ntx * (H->nz / Tile::P);
+  const int grid = std::min(ntiles, bpsm * H->num_sms);
+  return launch_named(H, name, [&]() -> int {
+    klaunch(H, kern, grid, Tile::THREADS, smem, map, ntx, ntiles, rev, ptable<S>(H, 1), H->derr, skip);
+    CKL();
+    return CUP_OK;
+  });
+}
+template <typename L, bool INV>
+int launch_pfft_y(cup_handle* H, const char* name, typename Lane<L>::S* buf, int rev, const int* skip) {
+  PFFT_DISPATCH(H->ny, (launch_pfft_y_M<M, L, INV>(H, name, buf, rev, skip)));
+}
+
+// z pass with the spectral divide, from `in` to `out` (FP64: the same array).
+template <int M, typename T>
+int launch_pfft_z_M(cup_handle* H, const char* name, T* in, double* out, const int* skip) {
+  constexpr bool MIXED = sizeof(T) == 4;
+  constexpr int W = 16, NB = 2, N = 2 * M;
+  using Tile = PTile<M, T, W>;
+  constexpr size_t ELEMS = (size_t)N * W * Tile::P;
+  CUtensorMap map_in, map_out;
+  int rc = make_map(H, &map_in, in, tma_dtype<T>(), sizeof(T), W, Tile::P, N);
+  if (!rc) rc = make_map(H, &map_out, out, tma_dtype<double>(), sizeof(double), W, Tile::P, N);
+  if (rc) return rc;
+  const size_t smem = NB * ELEMS * sizeof(T) + (MIXED ? ELEMS * sizeof(double) : 0) +
+                      M * (sizeof(double2) + sizeof(double) + (MIXED ? sizeof(float2) : 0)) + NB * sizeof(uint64_t) + 128;
+  auto kern = k_pfft_z<M, T, W, NB>;
+  int bpsm = 0;
+  if ((rc = prepare_kernel(H, kern, smem, Tile::THREADS, &bpsm))) return rc;
+  const int ntx = H->nx / W, ntiles = ntx * (H->ny / Tile::P);
+  const int grid = std::min(ntiles, bpsm * H->num_sms);
+  const PSpectral sp{H->pcos[0], H->pcos[1], H->pcos[2], H->pnorm};
+  return launch_named(H, name, [&]() -> int {
+    klaunch(H, kern, grid, Tile::THREADS, smem, map_in, map_out, ntx, ntiles, 0, ptable<T>(H, 2),
+            (const double2*)H->ptw64[2], sp, H->derr, skip);
+    CKL();
+    return CUP_OK;
+  });
+}
+template <typename T>
+int launch_pfft_z(cup_handle* H, const char* name, T* in, double* out, const int* skip) {
+  PFFT_DISPATCH(H->nz, (launch_pfft_z_M<M, T>(H, name, in, out, skip)));
+}
+
+// First x pass of the FP64 solve on the RHS formed from f (RHS never stored).
+template <int M, typename T>
+int launch_pfft_x_rhs_M(cup_handle* H, const char* name, void* const* f, double* out, DtArg dt) {
+  constexpr int WARPS = 4;
+  using Rw = PRows<M>;
+  const size_t smem = (size_t)WARPS * Rw::ELEMS * sizeof(double) + M * sizeof(double2) + 128;
+  auto kern = k_pfft_x_rhs<M, T, WARPS>;
+  int bpsm = 0;
+  int rc = prepare_kernel(H, kern, smem, 32 * WARPS, &bpsm);
+  if (rc) return rc;
+  const int ntiles = H->ny * H->nz / Rw::ROWS;
+  return launch_named(H, name, [&]() -> int {
+    klaunch(H, kern, (ntiles + WARPS - 1) / WARPS, 32 * WARPS, smem, (const T*)f[0], (const T*)f[1], (const T*)f[2], out,
+            dt, H->h, H->ny, H->nz, ntiles, (const double2*)H->ptw64[0]);
+    CKL();
+    return CUP_OK;
+  });
+}
+template <typename T>
+int launch_pfft_x_rhs(cup_handle* H, const char* name, void* const* f, double* out, DtArg dt) {
+  PFFT_DISPATCH(H->nx, (launch_pfft_x_rhs_M<M, T>(H, name, f, out, dt)));
+}
+
+// The passes of an FP64 solve after the first x pass, from `work` to `out`.
+int pfft_finish(cup_handle* H, const char* name_x, double* work, double* out, double* out2 = nullptr) {
   int rc;
-  if ((rc = launch_cols<R, 1, false>(H, work, work, skip))) return rc;
-  if ((rc = launch_cols<R, 2, true>(H, work, work, skip))) return rc;
-  if ((rc = launch_cols<R, 1, false>(H, work, work, skip))) return rc;
-  return CUP_OK;
+  if ((rc = launch_pfft_y<double, false>(H, "dht_y", work, 1, nullptr))) return rc;
+  if ((rc = launch_pfft_z<double>(H, "dht_z_solve", work, work, nullptr))) return rc;
+  if ((rc = launch_pfft_y<double, true>(H, "dht_y", work, 0, nullptr))) return rc;
+  return launch_pfft_x<double, PROW_INV>(H, name_x, work, out, out2, 1, nullptr);
+}
+
+// p = f . b over the three axes, FP64, the RHS in `work` (overwritten). A
+// handle whose z pass belongs to a pencil of a decomposed grid
+// (cup_set_spectral_window) runs the Hartley passes that the decomposed solve uses.
+int fft_poisson(cup_handle* H, double* work, double* out) {
+  int rc;
+  if (H->spec_ny != H->ny) {
+    if ((rc = launch_rows_pipe(H, "dht_x", work))) return rc;
+    if ((rc = launch_cols<1, false>(H, work))) return rc;
+    if ((rc = launch_cols<2, true>(H, work))) return rc;
+    if ((rc = launch_cols<1, false>(H, work))) return rc;
+    if ((rc = launch_rows_pipe(H, "dht_x", work))) return rc;
+    CK(cudaMemcpyAsync(out, work, H->n * sizeof(double), cudaMemcpyDeviceToDevice, H->stream));
+    return CUP_OK;
+  }
+  if ((rc = launch_pfft_x<double, PROW_FWD>(H, "dht_x", work, work, nullptr, 0, nullptr))) return rc;
+  return pfft_finish(H, "dht_x", work, out);
 }
 
 // Correction solve of the defect-correction loop, mixed precision: the x and y
 // forward transforms of the FP32 residual in FP32; the z pass widens to FP64
-// (forward, spectral divide, inverse); the y and x inverse transforms in FP64,
-// the last one adding the correction to p (minus the parity-class means of p
-// measured by the preceding residual pass). An FP32 inverse would leave white
-// rounding noise in the correction whose wide-Laplacian image is large next to
-// a smooth residual; with the inverse in FP64 one solve contracts the residual
-// by about 1e-7 whatever its spectrum.
+// between the spectral factor and the inverse; the y and x inverse transforms
+// in FP64, the last one adding the correction to p (minus the parity-class
+// means of p measured by the preceding residual pass). An FP32 inverse would
+// leave white rounding noise in the correction whose wide-Laplacian image is
+// large next to a smooth residual; with the inverse in FP64 one solve contracts
+// the residual by about 1e-7 whatever its spectrum.
 int dc_correction_solve(cup_handle* H, double* p, const int* skip) {
   int rc;
-  if ((rc = launch_rows_pipe<float>(H, "dht_x", H->work32, H->work32, skip))) return rc;
-  if ((rc = launch_cols<float, 1, false>(H, H->work32, H->work32, skip))) return rc;
-  if (H->nz == 256) {
-    if ((rc = launch_z_mixed<32, 1>(H, H->work32, H->work64, skip))) return rc;
-  } else if ((rc = launch_cols<double, 2, true, float>(H, H->work32, H->work64, skip))) {
-    return rc;
-  }
-  if ((rc = launch_cols<double, 1, false>(H, H->work64, H->work64, skip))) return rc;
-  return launch_rows_addp(H, "dht_x_update_p", H->work64, p, skip);
-}
-
-// p = H(f . H(work)) over the three axes, in place on `work`; the last x
-// pass writes to `out` (may equal work).
-template <typename R>
-int fft_poisson(cup_handle* H, R* work, R* out, const int* skip = nullptr) {
-  int rc;
-  if ((rc = launch_rows_pipe<R>(H, "dht_x", work, work, skip))) return rc;
-  if ((rc = fft_middle<R>(H, work, skip))) return rc;
-  return launch_rows_pipe<R>(H, "dht_x", work, out, skip);
+  if ((rc = launch_pfft_x<float, PROW_FWD>(H, "dht_x", H->work32, H->work32, nullptr, 0, skip))) return rc;
+  if ((rc = launch_pfft_y<F2, false>(H, "dht_y", H->work32, 0, skip))) return rc;
+  if ((rc = launch_pfft_z<float>(H, "dht_z_solve_mixed", H->work32, H->work64, skip))) return rc;
+  if ((rc = launch_pfft_y<double, true>(H, "dht_y_f64", H->work64, 0, skip))) return rc;
+  return launch_pfft_x<double, PROW_INV_ADDP>(H, "dht_x_update_p", H->work64, p, nullptr, 1, skip);
 }
 
 int box_grid(const Box& b) {
@@ -1716,19 +1733,22 @@ int do_poisson_dc(cup_handle* H) {
   return CUP_OK;
 }
 
-// FP64 solve with the RHS computed inside the first x pass (no RHS array).
+// FP64 solve with the RHS of the fields f computed inside the first x pass (no RHS array).
 template <typename T>
-int do_poisson_fused_fp64(cup_handle* H, DtArg dt) {
-  int rc;
-  RowsRhs<T> prod{(const T*)H->u, (const T*)H->v, (const T*)H->w, dt, H->h, H->nx, H->ny, H->nz};
-  if ((rc = launch_rows<double>(H, "rhs_dht_x", prod, RowsToArray<double>{H->rhs}, nullptr))) return rc;
-  if ((rc = fft_middle<double>(H, H->rhs, nullptr))) return rc;
-  return launch_rows_pipe<double>(H, "dht_x", H->rhs, H->p, nullptr);
+int do_solve_rhs_of(cup_handle* H, const char* name_rhs, const char* name_x, void* const* f, double* out, DtArg dt) {
+  if (H->spec_ny != H->ny) {
+    const void* cf[3] = {f[0], f[1], f[2]};
+    OpPressureRHS<T> op{H->rhs, dt, H->h, H->nx, H->ny};
+    int rc = launch_stream<T, 3, 1, 4, 4>(H, "pressure_rhs", cf, op);
+    return rc ? rc : fft_poisson(H, H->rhs, out);
+  }
+  int rc = launch_pfft_x_rhs<T>(H, name_rhs, f, H->rhs, dt);
+  return rc ? rc : pfft_finish(H, name_x, H->rhs, out);
 }
 
 // Poisson solve of the RHS array (operator-by-operator path, obstacles).
 int do_poisson(cup_handle* H) {
-  if (!H->fp32) return fft_poisson<double>(H, H->rhs, H->p);
+  if (!H->fp32) return fft_poisson(H, H->rhs, H->p);
   return do_poisson_dc(H);
 }
 
@@ -1963,9 +1983,9 @@ int do_spectral(cup_handle* H, bool filter, double raw[4], std::vector<double>& 
       return CUP_OK;
     });
     if (rc_) return rc_;
-    if ((rc_ = launch_rows_pipe<double>(H, "spectral_dht_x", H->spec[c], H->spec[c], nullptr))) return rc_;
-    if ((rc_ = launch_cols<double, 1, false>(H, H->spec[c], H->spec[c], nullptr))) return rc_;
-    if ((rc_ = launch_cols<double, 2, false>(H, H->spec[c], H->spec[c], nullptr))) return rc_;
+    if ((rc_ = launch_rows_pipe(H, "spectral_dht_x", H->spec[c]))) return rc_;
+    if ((rc_ = launch_cols<1, false>(H, H->spec[c]))) return rc_;
+    if ((rc_ = launch_cols<2, false>(H, H->spec[c]))) return rc_;
   }
   const int N = std::max(H->nx, std::max(H->ny, H->nz));
   const int nyquist = N / 2, nbin = nyquist - 1;
@@ -2042,9 +2062,9 @@ int do_spectral_forcing(cup_handle* H, double dt) {
     void* f[3] = {H->u, H->v, H->w};
     const int grid = std::min<size_t>(H->num_sms * 4, (H->n + 255) / 256);
     for (int c = 0; c < 3; ++c) {
-      if ((rc = launch_rows_pipe<double>(H, "spectral_dht_x", H->spec[c], H->spec[c], nullptr))) return rc;
-      if ((rc = launch_cols<double, 1, false>(H, H->spec[c], H->spec[c], nullptr))) return rc;
-      if ((rc = launch_cols<double, 2, false>(H, H->spec[c], H->spec[c], nullptr))) return rc;
+      if ((rc = launch_rows_pipe(H, "spectral_dht_x", H->spec[c]))) return rc;
+      if ((rc = launch_cols<1, false>(H, H->spec[c]))) return rc;
+      if ((rc = launch_cols<2, false>(H, H->spec[c]))) return rc;
       int rc_ = launch_named(H, "spectral_force", [&]() -> int {
         klaunch(H, k_add_scaled<T>, grid, 256, 0, (T*)f[c], H->spec[c], fac / NF, H->n);
         CKL();
@@ -2087,7 +2107,8 @@ int do_step(cup_handle* H, DtArg dt, const double* lambda_dev, int advance, int 
     // RHS, defect correction and gradient correction in z-queue passes
     if ((rc = do_pressure_dc_zq<T>(H, dt))) return rc;
   } else {
-    if ((rc = do_poisson_fused_fp64<T>(H, dt))) return rc;
+    void* us[3] = {H->u, H->v, H->w};
+    if ((rc = do_solve_rhs_of<T>(H, "rhs_dht_x", "dht_x", us, H->p, dt))) return rc;
   }
   if (!H->fp32) {
     if ((rc = do_grad<T>(H, dt))) return rc;
@@ -2144,20 +2165,6 @@ int launch_adjoint(cup_handle* H, const char* name, const void* const* f, const 
   });
 }
 
-// The projection P = I - G L^+ D of the pipeline (PressureRHS, the periodic
-// FFT solve in FP64, the gradient correction) applied to the fields `in`,
-// result in `out` (may equal `in`). D = -G^T on the periodic grid and L = D G
-// is the wide-stencil Laplacian the spectral factor inverts, so P is
-// symmetric: the adjoint of the projection is P itself.
-template <typename T>
-int do_solve_rhs_of(cup_handle* H, void* const* in, double* pbuf, DtArg dt) {
-  int rc;
-  RowsRhs<T> prod{(const T*)in[0], (const T*)in[1], (const T*)in[2], dt, H->h, H->nx, H->ny, H->nz};
-  if ((rc = launch_rows<double>(H, "adjoint_rhs_dht_x", prod, RowsToArray<double>{H->rhs}, nullptr))) return rc;
-  if ((rc = fft_middle<double>(H, H->rhs, nullptr))) return rc;
-  return launch_rows_pipe<double>(H, "adjoint_dht_x", H->rhs, pbuf, nullptr);
-}
-
 // out = in - dt/(2h) grad_c p (KernelGradP on given fields; out may equal in).
 template <typename T>
 int do_grad_fields(cup_handle* H, const char* name, void* const* in, void* const* out, const double* pbuf, DtArg dt) {
@@ -2168,10 +2175,15 @@ int do_grad_fields(cup_handle* H, const char* name, void* const* in, void* const
   return launch_stream<double, 1, 1, 4, 4>(H, name, pf, op, &ngp);
 }
 
+// The projection P = I - G L^+ D of the pipeline (PressureRHS, the periodic
+// FFT solve in FP64, the gradient correction) applied to the fields `in`,
+// result in `out` (may equal `in`). D = -G^T on the periodic grid and L = D G
+// is the wide-stencil Laplacian the spectral factor inverts, so P is
+// symmetric: the adjoint of the projection is P itself.
 template <typename T>
 int do_project_fields(cup_handle* H, void* const* in, void* const* out, double* pbuf, DtArg dt) {
   int rc;
-  if ((rc = do_solve_rhs_of<T>(H, in, pbuf, dt))) return rc;
+  if ((rc = do_solve_rhs_of<T>(H, "adjoint_rhs_dht_x", "adjoint_dht_x", in, pbuf, dt))) return rc;
   return do_grad_fields<T>(H, "adjoint_grad_p", in, out, pbuf, dt);
 }
 
@@ -2295,7 +2307,7 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
     if ((rc = launch_advect<T, 2, 2, 4, 1>(H, "adjoint_recompute_stage2", st1, un, us, dt))) return rc;
   }
   if ((rc = do_pressure_rhs<T>(H, dt, us, H->ab0))) return rc;
-  if ((rc = fft_poisson<double>(H, H->rhs, H->p_adj))) return rc;
+  if ((rc = fft_poisson(H, H->rhs, H->p_adj))) return rc;
   if ((rc = do_grad_fields<T>(H, "adjoint_recompute_grad_p", us, us, H->p_adj, dt))) return rc;
   // 2. penalization and force
   const int gb = box_grid(H->box);
@@ -2314,7 +2326,7 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
     if (rc_) return rc_;
   }
   // 3. projection with the transposed obstacle RHS terms
-  if ((rc = do_solve_rhs_of<T>(H, lam, H->p_adj, dt))) return rc;
+  if ((rc = do_solve_rhs_of<T>(H, "adjoint_rhs_dht_x", "adjoint_dht_x", lam, H->p_adj, dt))) return rc;
   const double kappa = dtv * dtv / (H->h * H->h * H->h);  // dJ/db2 = kappa q
   {
     int rc_ = launch_named(H, "adjoint_rhs_obstacle", [&]() -> int {
@@ -2612,31 +2624,38 @@ int cup_create(const cup_config* cfg, cup_handle** out) {
     CK(cudaMallocHost(&H->hstate, sizeof(DevState)));
     // FFT tables per axis, spectral cosines exactly as PoissonSolverPeriodic::_solve
     // computes them (source/poisson/PoissonSolverPeriodic.cpp:23-33).
+    // (one allocation and one copy for all of them)
+    double** cs[3] = {&H->cosx, &H->cosy, &H->cosz};
+    std::vector<unsigned char> blob;
+    std::vector<std::pair<void**, size_t>> at;
+    auto add = [&](auto** dst, const auto& v) {
+      const size_t bytes = v.size() * sizeof(v[0]), o = blob.size();
+      blob.resize(o + (bytes + 255) / 256 * 256);
+      memcpy(blob.data() + o, v.data(), bytes);
+      at.push_back({reinterpret_cast<void**>(dst), o});
+    };
     for (int d = 0; d < 3; ++d) {
       if (slab && d == 2) continue;  // no z transform on a z-slab handle
-      std::vector<double2> t64;
-      std::vector<float2> t32;
-      build_table(N[d], t64, t32);
-      CK(cudaMalloc(&H->tw64[d], t64.size() * sizeof(double2)));
-      CK(cudaMalloc(&H->tw32[d], t32.size() * sizeof(float2)));
-      CK(cudaMemcpy(H->tw64[d], t64.data(), t64.size() * sizeof(double2), cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(H->tw32[d], t32.data(), t32.size() * sizeof(float2), cudaMemcpyHostToDevice));
+      const long nK = N[d];
+      const double wFac = 4 * M_PI / nK;
+      std::vector<double> c(nK), pc;
+      for (long i = 0; i < nK; ++i) c[i] = std::cos(wFac * i);
+      std::vector<double2> t64, p64;
+      std::vector<float2> p32;
+      build_tables(N[d], c, d == 0, t64, p64, p32, pc);
+      add(cs[d], c);
+      add(&H->tw64[d], t64);
+      add(&H->ptw64[d], p64);
+      add(&H->ptw32[d], p32);
+      add(&H->pcos[d], pc);
     }
-    const size_t gsize[3] = {(size_t)N[0], (size_t)N[1], (size_t)N[2]};
-    const double h = H->h;
-    H->norm_factor = 4 / (gsize[0] * h * gsize[1] * gsize[2]);
+    CK(cudaMalloc(&H->tables, blob.size()));
+    CK(cudaMemcpy(H->tables, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+    for (auto& a : at) *a.first = static_cast<unsigned char*>(H->tables) + a.second;
+    H->norm_factor = 4 / ((size_t)N[0] * H->h * (size_t)N[1] * (size_t)N[2]);
+    H->pnorm = 8 * H->norm_factor;
     H->spec_ny = H->ny;
     H->spec_y0 = 0;
-    double** cs[3] = {&H->cosx, &H->cosy, &H->cosz};
-    for (int d = 0; d < 3; ++d) {
-      if (slab && d == 2) continue;
-      const long nK = (long)gsize[d];
-      const double wFac = 4 * M_PI / nK;
-      std::vector<double> c(nK);
-      for (long i = 0; i < nK; ++i) c[i] = std::cos(wFac * i);
-      CK(cudaMalloc(cs[d], nK * sizeof(double)));
-      CK(cudaMemcpy(*cs[d], c.data(), nK * sizeof(double), cudaMemcpyHostToDevice));
-    }
     H->hstate->lambda = H->lambda;
     CK(cudaMemcpyAsync(&H->dstate->lambda, &H->lambda, sizeof(double), cudaMemcpyHostToDevice, H->stream));
     CK(cudaStreamSynchronize(H->stream));
@@ -2661,13 +2680,9 @@ int cup_destroy(cup_handle* H) {
     if (f) cudaFree(f);
   for (void* f : {H->u, H->v, H->w, H->tu, H->tv, H->tw, H->u1, H->v1, H->w1, H->au, H->av, H->aw, (void*)H->p_adj,
                   H->chi, (void*)H->p, (void*)H->p_old, (void*)H->p_pred, (void*)H->rhs,
-                  (void*)H->work32, (void*)H->work64, (void*)H->partials, (void*)H->dstate, (void*)H->cosx,
-                  (void*)H->cosy, (void*)H->cosz, (void*)H->sp_dev, (void*)H->box_b, (void*)H->box_delta})
+                  (void*)H->work32, (void*)H->work64, (void*)H->partials, (void*)H->dstate, H->tables,
+                  (void*)H->cosy_win, (void*)H->sp_dev, (void*)H->box_b, (void*)H->box_delta})
     if (f) cudaFree(f);
-  for (int d = 0; d < 3; ++d) {
-    if (H->tw64[d]) cudaFree(H->tw64[d]);
-    if (H->tw32[d]) cudaFree(H->tw32[d]);
-  }
   prof_flush(H);
   for (cudaEvent_t e : H->ev_pool) cudaEventDestroy(e);
   if (H->hstate) cudaFreeHost(H->hstate);
@@ -3087,8 +3102,8 @@ int cup_set_spectral_window(cup_handle* H, int y0, int ny_global) {
   double* d = nullptr;
   CK(cudaMalloc(&d, ny_global * sizeof(double)));
   CK(cudaMemcpy(d, c.data(), ny_global * sizeof(double), cudaMemcpyHostToDevice));
-  cudaFree(H->cosy);
-  H->cosy = d;
+  cudaFree(H->cosy_win);
+  H->cosy = H->cosy_win = d;
   H->spec_ny = ny_global;
   H->spec_y0 = y0;
   H->norm_factor = 4 / ((double)H->nx * H->h * (double)ny_global * (double)H->nz);
@@ -3100,9 +3115,9 @@ int cup_poisson_pass(cup_handle* H, double* buf, int pass) {
   REQUIRE_H(H);
   if (!buf) return fail(H, CUP_ERR_ARG, "null buffer");
   switch (pass) {
-    case 0: return launch_rows_pipe<double>(H, "dht_x", buf, buf, nullptr);
-    case 1: return launch_cols<double, 1, false>(H, buf, buf, nullptr);
-    case 2: return launch_cols<double, 2, true>(H, buf, buf, nullptr);
+    case 0: return launch_rows_pipe(H, "dht_x", buf);
+    case 1: return launch_cols<1, false>(H, buf);
+    case 2: return launch_cols<2, true>(H, buf);
     default: return fail(H, CUP_ERR_ARG, "pass must be 0 (x), 1 (y) or 2 (z with the spectral divide)");
   }
 }

@@ -1,8 +1,12 @@
-// Shared-memory FFT passes of the periodic Poisson solve
-// (the device replacement of PoissonSolverPeriodic's FFTW r2c / _solve / c2r,
-// source/poisson/PoissonSolverPeriodic.cpp:15-146).
+// Shared-memory Hartley passes: the transforms of the z-slab decomposed
+// Poisson solve (cup_poisson_pass, the device replacement of
+// PoissonSolverPeriodic's FFTW-MPI r2c / _solve / c2r,
+// source/poisson/PoissonSolverPeriodic.cpp:15-146) and of the spectral analysis
+// and forcing, which need the coefficients themselves. (The solve of a whole
+// grid runs the packed transforms of pfft.cuh, whose bins mix the even and odd
+// cells and are of no use to a caller.)
 //
-// The solve is p = H(f . H(b)) with H the separable real Hartley transform
+// p = H(f . H(b)) with H the separable real Hartley transform
 // H[k] = Re X[k] - Im X[k] (X the unnormalised DFT) applied along x, y and z,
 // and f the reference's grid-consistent factor
 //   f = 4 / (Nx h Ny Nz) / (2 (cos(4 pi kx/Nx) + cos(4 pi ky/Ny) + cos(4 pi kz/Nz)) - 6)
@@ -278,9 +282,7 @@ struct NoScale {
 // M-k, M+k share one eigenvalue, so the spectral divide costs one factor per
 // four values.
 // The outputs go to `ao`; all inputs are read before a block barrier and the
-// outputs written after it, so `ao` may alias `a` even with a wider element
-// type (the z pass of the mixed-precision solve reads FP32 lines and writes
-// FP64 ones over the same bytes).
+// outputs written after it, so `ao` may alias `a`.
 // Split task k of one line: Z[k] = A, Z[M-k] = B -> H[k], H[N-k], H[M-k],
 // H[M+k] (task 0: H[0], H[M] from A = Z[0]), times scale(k).
 template <int M, typename R, typename R2, class AccO, class Scale>
@@ -321,8 +323,7 @@ __device__ __forceinline__ void split_task(const AccO& ao, int l, int k, R2 A, R
     }
     ao.str(l, k, hk);
     ao.str(l, N - k, hNk);
-    // k = M/2: M - k = k and M + k = N - k (same values); write each index
-    // once, so that an accumulating accessor adds it once
+    // k = M/2: M - k = k and M + k = N - k (same values)
     if (2 * k != M) {
       ao.str(l, M - k, hMk);
       ao.str(l, M + k, hMpk);
@@ -367,7 +368,7 @@ __device__ __forceinline__ void dht_post_to(const Acc& a, const AccO& ao, const 
 // owns butterflies t+1, 63-t (tasks t+1, 63-t) and t+17, 47-t (tasks t+17,
 // 47-t); thread 15 owns 16, 48 (tasks 16, 48), 0 (tasks 0 and 64) and 32
 // (task 32). All inputs are read before a block barrier, all outputs
-// written after it (`ao` may alias `a`, also with a wider element type).
+// written after it (`ao` may alias `a`).
 template <typename R, typename R2, class Acc, class AccO, class Scale>
 __device__ __forceinline__ void dht128_tail(const Acc& a, const AccO& ao, const R2* tw3, const R2* twp, int l, int t,
                                             bool active, const Scale& scale) {
@@ -450,14 +451,10 @@ __device__ __forceinline__ void fft_stages(const Acc& a, const P& pad, const typ
 //      owns butterflies t and 16 - t (t = 0: 0 and 8, each its own partner)
 //      and does their split tasks in registers.
 // Meant for column tiles (ColLines), where stage A's 16-strided writes fall in
-// different columns across a warp. `ao` may alias `a` (see dht_post_to).
-// Stage A writes to `pa` and stage B reads from it (column tiles: `a` itself).
-// PA_APART: `pa` shares no bytes with `a`, so stage A writes without waiting
-// for every thread's reads (one block barrier less).
-template <typename R, bool PA_APART = false, class Acc, class PAcc, class AccO, class Scale>
-__device__ __forceinline__ void dht128_t8_to(const Acc& a, const PAcc& pa, const AccO& ao,
-                                             const typename Cplx<R>::T* tw, int l, int t, bool active,
-                                             const Scale& scale) {
+// different columns across a warp. In place.
+template <typename R, class Acc, class Scale>
+__device__ __forceinline__ void dht128_t8(const Acc& a, const typename Cplx<R>::T* tw, int l, int t, bool active,
+                                          const Scale& scale) {
   using R2 = typename Cplx<R>::T;
   using Pl = FFTPlan<128>;
   constexpr int M = 128;
@@ -470,10 +467,10 @@ __device__ __forceinline__ void dht128_t8_to(const Acc& a, const PAcc& pa, const
     for (int r = 0; r < 16; ++r) v[r] = a.ld(l, t + 8 * r);
     DFT<16, R2>::run(v);
   }
-  if constexpr (!PA_APART) __syncthreads();
+  __syncthreads();
   if (active) {
 #pragma unroll
-    for (int r = 0; r < 16; ++r) pa.st(l, 16 * t + r, v[r]);
+    for (int r = 0; r < 16; ++r) a.st(l, 16 * t + r, v[r]);
   }
   __syncthreads();
   // stage B + split
@@ -482,8 +479,8 @@ __device__ __forceinline__ void dht128_t8_to(const Acc& a, const PAcc& pa, const
   if (active) {
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
-      z0[r] = pa.ld(l, j0 + 16 * r);
-      z1[r] = pa.ld(l, j1 + 16 * r);
+      z0[r] = a.ld(l, j0 + 16 * r);
+      z1[r] = a.ld(l, j1 + 16 * r);
       if (r > 0) {
         z0[r] = cmul(z0[r], twB[16 * r + j0]);
         z1[r] = cmul(z1[r], twB[16 * r + j1]);
@@ -496,17 +493,17 @@ __device__ __forceinline__ void dht128_t8_to(const Acc& a, const PAcc& pa, const
   if (active) {
     if (t == 0) {
       // butterfly 0: Z[16 r] pairs with Z[16 (8 - r)]; tasks 0, 16, 32, 48, 64
-      split_task<M, R, R2>(ao, l, 0, z0[0], z0[0], twp[0], scale);
+      split_task<M, R, R2>(a, l, 0, z0[0], z0[0], twp[0], scale);
 #pragma unroll
-      for (int r = 1; r <= 4; ++r) split_task<M, R, R2>(ao, l, 16 * r, z0[r], z0[8 - r], twp[16 * r], scale);
+      for (int r = 1; r <= 4; ++r) split_task<M, R, R2>(a, l, 16 * r, z0[r], z0[8 - r], twp[16 * r], scale);
       // butterfly 8: Z[8 + 16 r] pairs with Z[8 + 16 (7 - r)]; tasks 8, 24, 40, 56
 #pragma unroll
-      for (int r = 0; r < 4; ++r) split_task<M, R, R2>(ao, l, 8 + 16 * r, z1[r], z1[7 - r], twp[8 + 16 * r], scale);
+      for (int r = 0; r < 4; ++r) split_task<M, R, R2>(a, l, 8 + 16 * r, z1[r], z1[7 - r], twp[8 + 16 * r], scale);
     } else {
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        split_task<M, R, R2>(ao, l, j0 + 16 * r, z0[r], z1[7 - r], twp[j0 + 16 * r], scale);
-        split_task<M, R, R2>(ao, l, j1 + 16 * r, z1[r], z0[7 - r], twp[j1 + 16 * r], scale);
+        split_task<M, R, R2>(a, l, j0 + 16 * r, z0[r], z1[7 - r], twp[j0 + 16 * r], scale);
+        split_task<M, R, R2>(a, l, j1 + 16 * r, z1[r], z0[7 - r], twp[j1 + 16 * r], scale);
       }
     }
   }
@@ -539,72 +536,6 @@ __device__ __forceinline__ void dht_lines(const Acc& a, const P& pad, const type
 template <typename R2>
 __device__ __forceinline__ void load_table(R2* dst, const R2* src, int n) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
-}
-
-// ---------------------------------------------------------------------------
-// x pass: LPC consecutive rows of length N = 2M per CTA (rows are contiguous
-// in the [z][y][x] layout: row r is (y, z) = (r % ny, r / ny)). A producer
-// computes the rows in shared memory from other fields, the rows are
-// transformed, and a consumer stores them (one bulk store).
-
-// Consumer: rows stored to an array (one bulk store).
-template <typename R>
-struct RowsToArray {
-  R* out;
-  __device__ R* dst(int row0, int N) const { return out + (size_t)row0 * N; }
-};
-
-// Output accessor of the last step of a correction solve's last x pass
-// (k_dht_rows_addp_pipe): element n of line l is added to the shared-memory p
-// row, minus the parity-class mean of p measured by the preceding residual
-// pass (row r is (y, z) = (r & (ny-1), r >> log2ny); ny is a power of two).
-struct AddToPRows {
-  using elem = double;
-  double* prow;
-  const double* cm;  // the 8 class means (shared memory)
-  int N, row0, log2ny;
-  __device__ __forceinline__ void str(int l, int n, double v) const {
-    const int r = row0 + l;
-    const int cls = (n & 1) | ((r & 1) << 1) | (((r >> log2ny) & 1) << 2);
-    double* q = prow + l * N + n;
-    *q = *q + v - cm[cls];
-  }
-};
-
-template <int M, typename R, class Prod, class Cons>
-__global__ void __launch_bounds__(256) k_dht_rows(const Prod prod, const Cons cons, int nrows, int lpc,
-                                                  const typename Cplx<R>::T* tw_g, int* err, const int* skip) {
-  pdl_entry();
-  using R2 = typename Cplx<R>::T;
-  if (skip && *skip) return;
-  constexpr int N = 2 * M, TPL = M / 8;
-  constexpr int TL = FFTPlan<M>::rows_table_len();
-  constexpr bool PAD = FFTPlan<M>::nstages > 1;
-  constexpr int PPITCH = 2 * (M + M / 8);
-  extern __shared__ __align__(128) unsigned char smem_dyn[];
-  unsigned char* smem_raw = smem_align128(smem_dyn);
-  R* rows = reinterpret_cast<R*>(smem_raw);  // lpc * N
-  R* padb = rows + (size_t)lpc * N;          // lpc * PPITCH
-  R2* tw = reinterpret_cast<R2*>(padb + (PAD ? (size_t)lpc * PPITCH : 0));
-  const int row0 = blockIdx.x * lpc;
-  const int nr = min(lpc, nrows - row0);
-  if (nr <= 0) return;
-  const uint32_t bytes = (uint32_t)((size_t)nr * N * sizeof(R));
-  load_table(tw, tw_g, TL);
-  prod.fill(rows, row0, nr, N);
-  __syncthreads();
-  const int l = threadIdx.x / TPL, t = threadIdx.x % TPL;
-  const bool active = l < nr;
-  RowLines<R> A{rows, N};
-  RowLinesPad<R> P{padb, PPITCH};
-  dht_lines<M, PAD, R>(A, P, tw, l, t, active);
-  fence_proxy_async_smem();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    bulk_store(cons.dst(row0, N), rows, bytes);
-    bulk_commit();
-    bulk_wait_all();
-  }
 }
 
 // Pipelined x pass: persistent CTAs walk tiles of lpc consecutive rows
@@ -692,97 +623,6 @@ __global__ void __launch_bounds__(256, 2) k_dht_rows_pipe(const R* __restrict__ 
   }
 }
 
-// Pipelined last x pass of a correction solve (FP64): persistent CTAs walk
-// tiles of lpc rows through NB buffer pairs, each pair holding the tile's
-// transform rows and its p rows, both filled by 1-D bulk copies on one
-// barrier. The inverse transform's last step adds into the p rows (AddToPRows:
-// p += rows - class means of p) and one bulk store writes them back. The loads
-// of the next NB-1 tiles and the store of the previous one overlap the
-// transform of the current tile; the twiddle table and the class means are
-// loaded once per CTA.
-template <int M, int NB>
-__global__ void __launch_bounds__(256, 1) k_dht_rows_addp_pipe(const double* __restrict__ in, double* p,
-                                                               const double* cmean, int log2ny, int nrows, int lpc,
-                                                               const double2* tw_g, int* err, const int* skip) {
-  pdl_entry();
-  static_assert(NB >= 2, "need at least two buffer pairs");
-  if (skip && *skip) return;
-  constexpr int N = 2 * M, TPL = M / 8;
-  constexpr int TL = FFTPlan<M>::rows_table_len();
-  constexpr bool PAD = FFTPlan<M>::nstages > 1;
-  constexpr int PPITCH = 2 * (M + M / 8);
-  extern __shared__ __align__(128) unsigned char smem_dyn[];
-  unsigned char* smem_raw = smem_align128(smem_dyn);
-  double* bufs = reinterpret_cast<double*>(smem_raw);  // NB * lpc * N transform rows
-  double* pbufs = bufs + (size_t)NB * lpc * N;         // NB * lpc * N p rows
-  double* padb = pbufs + (size_t)NB * lpc * N;         // lpc * PPITCH
-  double2* tw = reinterpret_cast<double2*>(padb + (PAD ? (size_t)lpc * PPITCH : 0));
-  uint64_t* bar = reinterpret_cast<uint64_t*>(tw + TL);
-  double* cms = reinterpret_cast<double*>(bar + NB);   // the 8 class means
-  const int tid = threadIdx.x;
-  const int ntiles = (nrows + lpc - 1) / lpc;
-  const int my = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  if (tid == 0) {
-    for (int b = 0; b < NB; ++b) mbar_init(&bar[b], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  auto rows_of = [&](int i, int& row0, int& nr) {
-    row0 = (blockIdx.x + i * gridDim.x) * lpc;
-    nr = min(lpc, nrows - row0);
-  };
-  auto issue = [&](int i) {
-    int row0, nr;
-    rows_of(i, row0, nr);
-    const int b = i % NB;
-    const uint32_t bytes = (uint32_t)((size_t)nr * N * sizeof(double));
-    mbar_arrive_expect_tx(&bar[b], 2 * bytes);
-    bulk_load(bufs + (size_t)b * lpc * N, in + (size_t)row0 * N, bytes, &bar[b]);
-    bulk_load(pbufs + (size_t)b * lpc * N, p + (size_t)row0 * N, bytes, &bar[b]);
-  };
-  int issued = 0;
-  if (tid == 0)
-    for (; issued < min(NB - 1, my); ++issued) issue(issued);
-  load_table(tw, tw_g, TL);
-  if (tid < 8) cms[tid] = cmean[tid];
-  __syncthreads();
-  const int l = tid / TPL, t = tid % TPL;
-  RowLinesPad<double> P{padb, PPITCH};
-  bool ok = true;
-  int done = 0;
-  for (int i = 0; i < my; ++i) {
-    // refill: tile i + NB - 1 goes into the buffer pair of tile i - 1, once
-    // the store of its p rows has read them
-    if (tid == 0 && ok && issued < my) {
-      bulk_wait_read<0>();
-      issue(issued++);
-    }
-    int row0, nr;
-    rows_of(i, row0, nr);
-    const int b = i % NB;
-    ok = __syncthreads_and(ok && mbar_wait(&bar[b], (i / NB) & 1, err));
-    if (!ok) break;
-    RowLines<double> A{bufs + (size_t)b * lpc * N, N};
-    double* prow = pbufs + (size_t)b * lpc * N;
-    const bool active = l < nr;
-    fft_stages<M, PAD, double>(A, P, tw, l, t, active);
-    dht_tail_to<M, double>(A, AddToPRows{prow, cms, N, row0, log2ny}, tw, l, t, active, NoScale());
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      bulk_store(p + (size_t)row0 * N, prow, (uint32_t)((size_t)nr * N * sizeof(double)));
-      bulk_commit();
-    }
-    done = i + 1;
-  }
-  if (tid == 0) {
-    bulk_wait_all();
-    // after a timed-out wait: bounded drain of the loads still in flight
-    if (!ok)
-      for (int r = done; r < issued; ++r) mbar_wait(&bar[r % NB], (r / NB) & 1, nullptr);
-  }
-}
-
 // Spectral factor of PoissonSolverPeriodic::_solve (grid-consistent branch,
 // source/poisson/PoissonSolverPeriodic.cpp:23-61): cx/cy/cz hold
 // cos(4 pi k / N) evaluated on the host exactly as the reference does.
@@ -799,33 +639,21 @@ struct SpectralParams {
 // nf / (2 (cos_x + cos_y + cos_z) - 6), zero on the 8 null modes (kx in
 // {0, Nx/2}, ky in {0, Ny/2}, kz in {0, Nz/2}); the z indices 0 and Nz/2 are
 // both handled by task k = 0. cz: cos_z[0..Nz/4] (the tasks' k range), staged
-// in shared memory by the pass. SF = double divides exactly (the direct FP64
-// solve). SF = float is the correction solve of the defect-correction loop:
-// the denominator is still formed in FP64 (it cancels to 2 (1 - cos(4 pi/N))
-// at the lowest modes), then the FP32 quotient scales the FP32 forward
-// transform's output. A factor with relative error e changes each mode of the
-// correction by the factor 1 + e, which leaves a residual of relative size e:
-// the same order as the FP32 forward transform's own rounding.
-template <typename SF>
+// in shared memory by the pass.
 struct ZColumnFactor {
-  using type = SF;
+  using type = double;
   double cxy;  // cos_x[kx] + cos_y[ky]
   const double* cz;
   double nf;
   bool null_col;
   static constexpr bool kOn = true;
-  __device__ __forceinline__ SF operator()(int k) const {
-    if (k == 0 && null_col) return (SF)0;
-    const double den = 2 * (cxy + cz[k]) - 6;
-    if constexpr (sizeof(SF) == 4) return __fdividef((float)nf, (float)den);
-    else return nf / den;
+  __device__ __forceinline__ double operator()(int k) const {
+    return k == 0 && null_col ? 0.0 : nf / (2 * (cxy + cz[k]) - 6);
   }
 };
 
-template <typename SF>
-__device__ __forceinline__ ZColumnFactor<SF> z_column_factor(const SpectralParams& sp, const double* cz, int kx,
-                                                             int ky) {
-  ZColumnFactor<SF> f;
+__device__ __forceinline__ ZColumnFactor z_column_factor(const SpectralParams& sp, const double* cz, int kx, int ky) {
+  ZColumnFactor f;
   const int gy = sp.y0 + ky;
   f.cxy = __ldg(sp.cx + kx) + __ldg(sp.cy + gy);
   f.cz = cz;
@@ -839,36 +667,23 @@ __device__ __forceinline__ ZColumnFactor<SF> z_column_factor(const SpectralParam
 // coordinate t / ntiles_x) through NB shared-memory tile buffers. The TMA
 // loads of the next NB-1 tiles and the store of the previous tile overlap the
 // transform of the current one; the twiddle table is loaded once per CTA.
-//
-// RIN = float with R = double (z pass of the mixed-precision correction
-// solve): the FP32 tile lands in the upper half of its FP64 buffer; the
-// forward transform runs in FP32 on it (like the x and y forward passes) and
-// its even/odd split writes the divided spectrum in FP64 over the whole
-// buffer (all reads before a barrier, all writes after it); the inverse runs
-// in FP64 and the tile is stored in FP64. tw_in_g: the FP32 table.
-template <int M, typename R, int AXIS, bool DIVIDE, int W, int NB, typename RIN = R, bool T8 = false>
-__global__ void __launch_bounds__(W * (T8 ? 8 : M / 8)) k_dht_cols_pipe(const __grid_constant__ CUtensorMap map_in,
-                                                       const __grid_constant__ CUtensorMap map_out, int ntiles_x,
-                                                       int ntiles, const typename Cplx<R>::T* tw_g,
-                                                       const typename Cplx<RIN>::T* tw_in_g, SpectralParams sp,
-                                                       int* err, const int* skip) {
+template <int M, typename R, int AXIS, bool DIVIDE, int W, int NB, bool T8 = false>
+__global__ void __launch_bounds__(W * (T8 ? 8 : M / 8)) k_dht_cols_pipe(const __grid_constant__ CUtensorMap map,
+                                                       int ntiles_x, int ntiles, const typename Cplx<R>::T* tw_g,
+                                                       SpectralParams sp, int* err, const int* skip) {
   pdl_entry();
   using R2 = typename Cplx<R>::T;
-  using RI2 = typename Cplx<RIN>::T;
   static_assert(NB >= 2, "need at least two tile buffers");
-  static_assert(sizeof(RIN) <= sizeof(R), "input may only be narrower than the transform type");
   static_assert(!T8 || M == 128, "the 8-thread plan is for 256-long lines");
   if (skip && *skip) return;
   constexpr int N = 2 * M, TPL = T8 ? 8 : M / 8;
   constexpr int TL = FFTPlan<M>::table_len();
-  constexpr bool WIDEN = sizeof(RIN) < sizeof(R);
-  constexpr uint32_t TILE_BYTES = (uint32_t)(N * W * sizeof(RIN));
+  constexpr uint32_t TILE_BYTES = (uint32_t)(N * W * sizeof(R));
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   unsigned char* smem_raw = smem_align128(smem_dyn);
   R* tiles = reinterpret_cast<R*>(smem_raw);  // [NB][N][W]
   R2* tw = reinterpret_cast<R2*>(tiles + (size_t)NB * N * W);
-  RI2* tw_in = reinterpret_cast<RI2*>(tw + TL);  // (WIDEN only)
-  uint64_t* bar = reinterpret_cast<uint64_t*>(tw_in + (WIDEN ? TL : 0));
+  uint64_t* bar = reinterpret_cast<uint64_t*>(tw + TL);
   double* czs = reinterpret_cast<double*>(bar + NB);  // cos_z[0..M/2] (DIVIDE)
   const int tid = threadIdx.x;
   const int my = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
@@ -887,16 +702,12 @@ __global__ void __launch_bounds__(W * (T8 ? 8 : M / 8)) k_dht_cols_pipe(const __
     coords(i, x0, other);
     const int b = i % NB;
     mbar_arrive_expect_tx(&bar[b], TILE_BYTES);
-    // widening: the narrow tile occupies the upper half of the buffer
-    unsigned char* dst = reinterpret_cast<unsigned char*>(tiles + (size_t)b * N * W) +
-                         (WIDEN ? (size_t)N * W * (sizeof(R) - sizeof(RIN)) : 0);
-    tma_load_3d(dst, &map_in, x0, AXIS == 1 ? 0 : other, AXIS == 1 ? other : 0, &bar[b]);
+    tma_load_3d(tiles + (size_t)b * N * W, &map, x0, AXIS == 1 ? 0 : other, AXIS == 1 ? other : 0, &bar[b]);
   };
   int issued = 0;
   if (tid == 0)
     for (; issued < min(NB - 1, my); ++issued) issue(issued);
   load_table(tw, tw_g, TL);
-  if constexpr (WIDEN) load_table(tw_in, tw_in_g, TL);
   if constexpr (DIVIDE)
     for (int i = tid; i <= M / 2; i += blockDim.x) czs[i] = sp.cz[i];
   __syncthreads();
@@ -918,48 +729,25 @@ __global__ void __launch_bounds__(W * (T8 ? 8 : M / 8)) k_dht_cols_pipe(const __
     coords(i, x0, other);
     R* tile = tiles + (size_t)b * N * W;
     ColLines<R> A{tile, W};
-    if constexpr (T8) {
-      if constexpr (WIDEN) {
-        ColLines<RIN> An{reinterpret_cast<RIN*>(reinterpret_cast<unsigned char*>(tile) +
-                                                (size_t)N * W * (sizeof(R) - sizeof(RIN))),
-                         W};
-        // the lower part of the buffer is free until the widened output:
-        // stage A of the narrow transform writes there
-        ColLines<RIN> Lo{reinterpret_cast<RIN*>(tile), W};
-        if constexpr (DIVIDE) {
-          dht128_t8_to<RIN, true>(An, Lo, A, tw_in, l, t, active, z_column_factor<RIN>(sp, czs, x0 + l, other));
-          dht128_t8_to<R>(A, A, A, tw, l, t, active, NoScale());
-        } else {
-          dht128_t8_to<RIN, true>(An, Lo, A, tw_in, l, t, active, NoScale());
-        }
-      } else if constexpr (DIVIDE) {
-        dht128_t8_to<R>(A, A, A, tw, l, t, active, z_column_factor<double>(sp, czs, x0 + l, other));
-        dht128_t8_to<R>(A, A, A, tw, l, t, active, NoScale());
-      } else {
-        dht128_t8_to<R>(A, A, A, tw, l, t, active, NoScale());
-      }
-    } else if constexpr (WIDEN) {
-      ColLines<RIN> An{reinterpret_cast<RIN*>(reinterpret_cast<unsigned char*>(tile) +
-                                              (size_t)N * W * (sizeof(R) - sizeof(RIN))),
-                       W};
-      fft_stages<M, false, RIN>(An, An, tw_in, l, t, active);
-      if constexpr (DIVIDE) {
-        dht_tail_to<M, RIN>(An, A, tw_in, l, t, active, z_column_factor<RIN>(sp, czs, x0 + l, other));
-        dht_lines<M, false, R>(A, A, tw, l, t, active);
-      } else {
-        dht_tail_to<M, RIN>(An, A, tw_in, l, t, active, NoScale());
-      }
-    } else if constexpr (DIVIDE) {
+    if constexpr (DIVIDE) {
       // forward, spectral divide fused into the even/odd split, inverse
-      dht_lines<M, false, R>(A, A, tw, l, t, active, z_column_factor<double>(sp, czs, x0 + l, other));
-      dht_lines<M, false, R>(A, A, tw, l, t, active);
+      const ZColumnFactor f = z_column_factor(sp, czs, x0 + l, other);
+      if constexpr (T8) {
+        dht128_t8<R>(A, tw, l, t, active, f);
+        dht128_t8<R>(A, tw, l, t, active, NoScale());
+      } else {
+        dht_lines<M, false, R>(A, A, tw, l, t, active, f);
+        dht_lines<M, false, R>(A, A, tw, l, t, active);
+      }
+    } else if constexpr (T8) {
+      dht128_t8<R>(A, tw, l, t, active, NoScale());
     } else {
       dht_lines<M, false, R>(A, A, tw, l, t, active);
     }
     fence_proxy_async_smem();
     __syncthreads();
     if (tid == 0) {
-      tma_store_3d(&map_out, x0, AXIS == 1 ? 0 : other, AXIS == 1 ? other : 0, tile);
+      tma_store_3d(&map, x0, AXIS == 1 ? 0 : other, AXIS == 1 ? other : 0, tile);
       bulk_commit();
     }
     done = i + 1;
@@ -969,101 +757,6 @@ __global__ void __launch_bounds__(W * (T8 ? 8 : M / 8)) k_dht_cols_pipe(const __
     // after a timed-out wait: bounded drain of the loads still in flight
     if (!ok)
       for (int r = done; r < issued; ++r) mbar_wait(&bar[r % NB], (r / NB) & 1, nullptr);
-  }
-}
-
-// Mixed-precision z pass of the correction solve (256-long lines, the 8-thread
-// plan) with a narrow input ring: the FP32 input tiles (W columns by the whole
-// z line) arrive by TMA in NBN narrow buffers and each tile is transformed in
-// one FP64 buffer. Stage A of the FP32 forward transform reads the narrow tile
-// and writes into the lower half of the FP64 buffer, so once the forward
-// transform is done the narrow buffer takes the load of tile i + NBN while the
-// FP64 inverse runs; the FP64 buffer is reused once the store of the previous
-// tile has read it. Only the post-split and radix-16 twiddles of the 8-thread
-// plan are staged. At W = 32, NBN = 1 a CTA needs 101 KB of shared memory
-// (two CTAs per SM) and its tile rows are 128 B in FP32 and 256 B in FP64;
-// the ring of two FP64 buffers at W = 16 needed 70 KB (three CTAs per SM) for
-// 64-B and 128-B rows. Same arithmetic, in the same order, as
-// k_dht_cols_pipe<128, double, 2, true, W, NB, float, true>.
-template <int W, int NBN>
-__global__ void __launch_bounds__(W * 8) k_dht_z_mixed(const __grid_constant__ CUtensorMap map_in,
-                                                      const __grid_constant__ CUtensorMap map_out, int ntiles_x,
-                                                      int ntiles, const double2* tw_g, const float2* tw_in_g,
-                                                      SpectralParams sp, int* err, const int* skip) {
-  pdl_entry();
-  if (skip && *skip) return;
-  using Pl = FFTPlan<128>;
-  constexpr int M = 128, N = 2 * M;
-  constexpr int T0 = Pl::post_off(), TN = Pl::table_len() - Pl::post_off();  // staged part of the tables
-  constexpr uint32_t IN_BYTES = (uint32_t)(N * W * sizeof(float));
-  extern __shared__ __align__(128) unsigned char smem_dyn[];
-  unsigned char* smem_raw = smem_align128(smem_dyn);
-  double* wide = reinterpret_cast<double*>(smem_raw);         // [N][W]
-  float* narrow = reinterpret_cast<float*>(wide + N * W);      // [NBN][N][W]
-  double2* tws = reinterpret_cast<double2*>(narrow + NBN * N * W);
-  float2* tws_in = reinterpret_cast<float2*>(tws + TN);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(tws_in + TN);
-  double* czs = reinterpret_cast<double*>(bar + NBN);  // cos_z[0..M/2]
-  // the transforms index the tables from their start; entries below T0 are never read
-  const double2* tw = tws - T0;
-  const float2* tw_in = tws_in - T0;
-  const int tid = threadIdx.x;
-  const int my = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  if (tid == 0) {
-    for (int b = 0; b < NBN; ++b) mbar_init(&bar[b], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  auto coords = [&](int i, int& x0, int& y) {
-    const int t = blockIdx.x + i * gridDim.x;
-    x0 = (t % ntiles_x) * W;
-    y = t / ntiles_x;
-  };
-  auto issue = [&](int i) {
-    int x0, y;
-    coords(i, x0, y);
-    const int b = i % NBN;
-    mbar_arrive_expect_tx(&bar[b], IN_BYTES);
-    tma_load_3d(narrow + (size_t)b * N * W, &map_in, x0, y, 0, &bar[b]);
-  };
-  int issued = 0;
-  if (tid == 0)
-    for (; issued < min(NBN, my); ++issued) issue(issued);
-  load_table(tws, tw_g + T0, TN);
-  load_table(tws_in, tw_in_g + T0, TN);
-  for (int i = tid; i <= M / 2; i += blockDim.x) czs[i] = sp.cz[i];
-  __syncthreads();
-  const int l = tid % W, t = tid / W;
-  bool ok = true;
-  int done = 0;
-  for (int i = 0; i < my; ++i) {
-    // the store of tile i - 1 must have read the FP64 buffer before stage A writes it
-    if (tid == 0 && i > 0) bulk_wait_read<0>();
-    const int b = i % NBN;
-    ok = __syncthreads_and(ok && mbar_wait(&bar[b], (i / NBN) & 1, err));
-    if (!ok) break;
-    int x0, y;
-    coords(i, x0, y);
-    ColLines<float> An{narrow + (size_t)b * N * W, W};
-    ColLines<float> Lo{reinterpret_cast<float*>(wide), W};
-    ColLines<double> A{wide, W};
-    dht128_t8_to<float, true>(An, Lo, A, tw_in, l, t, true, z_column_factor<float>(sp, czs, x0 + l, y));
-    // every read of the narrow tile came before the barriers of the forward transform
-    if (tid == 0 && issued < my) issue(issued++);
-    dht128_t8_to<double>(A, A, A, tw, l, t, true, NoScale());
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      tma_store_3d(&map_out, x0, y, 0, wide);
-      bulk_commit();
-    }
-    done = i + 1;
-  }
-  if (tid == 0) {
-    bulk_wait_all();
-    // after a timed-out wait: bounded drain of the loads still in flight
-    if (!ok)
-      for (int r = done; r < issued; ++r) mbar_wait(&bar[r % NBN], (r / NBN) & 1, nullptr);
   }
 }
 

@@ -186,30 +186,6 @@ struct OpResidual {
   }
 };
 
-// ---- producers / consumers of the fused x pass (k_dht_rows) ---------------
-
-// Rows of the pressure RHS computed from u* (KernelPressureRHS,
-// source/operators/PressureRHS.cpp:51-76): fused into the first x pass so the
-// RHS never goes to HBM.
-template <typename T>
-struct RowsRhs {
-  const T *u, *v, *w;
-  DtArg dt;
-  double h;
-  int nx, ny, nz;
-  __device__ void fill(double* rows, int row0, int nr, int N) const {
-    const double fac = 0.5 * h * h / dt.get();
-    for (int i = threadIdx.x; i < nr * N; i += blockDim.x) {
-      const int l = i / N, x = i - l * N;
-      const int r = row0 + l, y = r % ny, z = r / ny;
-      const double uE = u[gidx(wrapi(x + 1, nx), y, z, nx, ny)], uW = u[gidx(wrapi(x - 1, nx), y, z, nx, ny)];
-      const double vN = v[gidx(x, wrapi(y + 1, ny), z, nx, ny)], vS = v[gidx(x, wrapi(y - 1, ny), z, nx, ny)];
-      const double wB = w[gidx(x, y, wrapi(z + 1, nz), nx, ny)], wF = w[gidx(x, y, wrapi(z - 1, nz), nx, ny)];
-      rows[i] = fac * (uE - uW + vN - vS + wB - wF);
-    }
-  }
-};
-
 // Active box of the obstacle: cells [lo, lo+n) per dimension (global indices,
 // wrapped periodically). Outside it chi == 0 and the obstacle terms vanish.
 struct Box {
