@@ -871,6 +871,8 @@ struct cup_handle {
     long long launches;
   };
   std::vector<StepGraph> graphs;
+  cudaStream_t cap_stream = nullptr;  // captures run here: the default streams cannot be captured
+  long long steps_run = 0;            // steps since creation
   // launch accounting and optional per-kernel CUDA-event profiling
   long long launches = 0;
   bool prof_on = false;
@@ -2439,12 +2441,18 @@ void drop_graph(cup_handle* H) {
   H->graphs.clear();
 }
 
-// Steps may replay a captured graph: no per-kernel profiling, a stream that
-// can be captured, nothing that needs the host between steps (a moving
-// obstacle, spectral forcing), and the FP32-DC pressure history in its steady
-// state (warm start ready), so that every step issues the same launches.
+// Steps may replay a captured graph: no per-kernel profiling, a stream that is
+// not itself being captured by the caller, nothing that needs the host between
+// steps (a moving obstacle, spectral forcing), and the FP32-DC pressure history
+// in its steady state (warm start ready), so that every step issues the same
+// launches.
 bool graph_ok(const cup_handle* H) {
   if (!H->use_graphs || H->prof_on || !H->stream || H->forcing) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(H->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
   if (H->has_sphere && H->sphere_moves) return false;
   if (H->fp32 && !(H->pred_ready && H->p_valid >= 1)) return false;
   return true;
@@ -2454,7 +2462,9 @@ bool graph_ok(const cup_handle* H) {
 // (dt from the device state; next_dt: each step computes the next step's dt)
 // unless it is cached; *out = the cached graph, or nullptr when the capture
 // failed (graphs are then off for the handle). The host state is left as it
-// was: the captured steps only move it forward when the graph is replayed.
+// was: the captured steps only move it forward when the graph is replayed. The
+// capture runs on a stream of its own, so that a handle bound to a default
+// stream (torch's, unless its caller opened another) replays graphs too.
 int capture_graph(cup_handle* H, int nsteps, int next_dt, cup_handle::StepGraph** out) {
   *out = nullptr;
   const cup_handle::StepState in = step_state(H);
@@ -2465,16 +2475,20 @@ int capture_graph(cup_handle* H, int nsteps, int next_dt, cup_handle::StepGraph*
     }
   if (H->graphs.size() >= 32) drop_graph(H);
   const long long l0 = H->launches;
-  if (cudaStreamBeginCapture(H->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
+  if ((!H->cap_stream && cudaStreamCreateWithFlags(&H->cap_stream, cudaStreamNonBlocking) != cudaSuccess) ||
+      cudaStreamBeginCapture(H->cap_stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
     cudaGetLastError();
     H->use_graphs = false;
     return CUP_OK;
   }
+  const cudaStream_t run_stream = H->stream;
+  H->stream = H->cap_stream;
   int rc = CUP_OK;
   for (int s = 0; s < nsteps && rc == CUP_OK; ++s)
     rc = DISPATCH_T(H, do_step, DtArg{0.0, &H->dstate->dt}, (const double*)&H->dstate->lambda, 1, next_dt);
   cudaGraph_t g = nullptr;
-  const cudaError_t e = cudaStreamEndCapture(H->stream, &g);
+  const cudaError_t e = cudaStreamEndCapture(H->cap_stream, &g);
+  H->stream = run_stream;
   cudaGraphExec_t ex = nullptr;
   const cup_handle::StepState after = step_state(H);
   set_step_state(H, in);
@@ -2497,14 +2511,26 @@ int capture_graph(cup_handle* H, int nsteps, int next_dt, cup_handle::StepGraph*
 // swap and the three FP32-DC pressure levels) and replayed with the host
 // state set to what the captured steps left. *ran = false: the capture
 // failed, nothing ran, the host state is as before and graphs are off for
-// the handle.
+// the handle, or the handle has not run long enough to capture.
+// A handle captures for itself once it has run kGraphAfter steps: a 6-step
+// graph and the one-step graphs of a tail take about 1.5 ms of host time with
+// the GPU idle, and replaying saves 20-60 us a step, so a run that ends earlier
+// would not win it back. cup_prepare_run captures at any time.
+constexpr int kGraphAfter = 24;
 int run_graph(cup_handle* H, int nsteps, int next_dt, bool* ran) {
   *ran = false;
   cup_handle::StepGraph* hit = nullptr;
+  if (H->steps_run < kGraphAfter) {
+    const cup_handle::StepState in = step_state(H);
+    bool cached = false;
+    for (const auto& g : H->graphs) cached = cached || (g.nsteps == nsteps && g.next_dt == next_dt && same_state(g.in, in));
+    if (!cached) return CUP_OK;
+  }
   int rc = capture_graph(H, nsteps, next_dt, &hit);
   if (rc || !hit) return rc;
   CK(cudaGraphLaunch(hit->exec, H->stream));
   H->launches += hit->launches;
+  H->steps_run += nsteps;
   set_step_state(H, hit->out);
   *ran = true;
   return CUP_OK;
@@ -2686,6 +2712,7 @@ int cup_destroy(cup_handle* H) {
   prof_flush(H);
   for (cudaEvent_t e : H->ev_pool) cudaEventDestroy(e);
   if (H->hstate) cudaFreeHost(H->hstate);
+  if (H->cap_stream) cudaStreamDestroy(H->cap_stream);
   if (H->own_stream && H->stream) cudaStreamDestroy(H->stream);
   delete H;
   return CUP_OK;
@@ -3238,7 +3265,10 @@ int cup_step(cup_handle* H, double dt, cup_step_stats* stats) {
   bool ran = false;
   int rc = graph_ok(H) ? run_graph(H, 1, 1, &ran) : CUP_OK;
   if (rc) return rc;
-  if (!ran) rc = DISPATCH_T(H, do_step, DtArg{dt, nullptr}, (const double*)&H->dstate->lambda, 1, 1);
+  if (!ran) {
+    rc = DISPATCH_T(H, do_step, DtArg{dt, nullptr}, (const double*)&H->dstate->lambda, 1, 1);
+    H->steps_run += 1;
+  }
   if (rc) return rc;
   if (H->has_sphere && H->sphere_free && (rc = read_sphere_motion(H))) return rc;
   H->step += 1;
@@ -3414,6 +3444,7 @@ int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
     rc = DISPATCH_T(H, do_step, DtArg{0.0, &H->dstate->dt}, (const double*)&H->dstate->lambda, 1,
                     i + 1 < nsteps ? 1 : 0);
     if (rc) return rc;
+    H->steps_run += 1;
     ++i;
   }
   if ((rc = read_state(H))) return rc;

@@ -257,8 +257,9 @@ int cup_step(struct cup_handle* h, double dt, cup_step_stats* stats);
  * with dt computed on the device (no host round trip per step). */
 int cup_run(struct cup_handle* h, int nsteps, cup_step_stats* stats);
 /* cup_run replays its steady-state steps from CUDA graphs of 6 steps and its
- * tail from one-step graphs (captured on first use; same kernels, same
- * results); off: every step is launched. */
+ * tail from one-step graphs (captured once the handle has run 24 steps, or by
+ * cup_prepare_run; same kernels, same results), on any stream; off: every step
+ * is launched. */
 int cup_set_graphs(struct cup_handle* h, int on);
 /* Captures, without running anything, the CUDA graphs that cup_run(nsteps)
  * replays from the handle's current state (6-step graphs, then one-step graphs

@@ -38,3 +38,27 @@ def test_packed_transforms_every_line_length(oracle, cells, precision):
     tol = 1e-12 if precision == "fp64" else 1e-10 * kappa
     assert rel_l2(p, oracle.poisson_solve(rhs, sim.h)) < tol
     sim.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_dc"])
+def test_graph_replay_on_the_default_stream(precision):
+    """A handle bound to torch's default stream (which cannot be captured)
+    replays graphs, with the results of launching every step; inside a capture
+    of the caller's it launches."""
+    import torch
+    from cubismup_3d_b200 import initial_conditions as ic
+    cells = (64, 32, 32)
+    u = ic.random_solenoidal(cells, 3, lambda k: k ** 4 * np.exp(-2 * (k / 4) ** 2), rms=1.0)
+    out = []
+    for graphs in (True, False):
+        sim = make_sim(cells, 2 * np.pi, nu=1e-3, precision=precision, scheme="upwind3_rk2")
+        sim.use_graphs(graphs)
+        sim.set_velocity(*u)
+        sim.bind_torch_stream()
+        sim.run_steps(26)
+        assert (sim.prepare_run(13) > 0) == graphs
+        sim.run_steps(13)
+        sim.timestep(sim.calcMaxTimestep())
+        out.append(sim.velocity_raw())
+        sim.close()
+    assert torch.equal(out[0], out[1])
