@@ -15,9 +15,8 @@
 // and the kernel writes out = alpha lam + beta S'(f)^T g (lam point-wise).
 //
 // Structure as k_advect_zq: TMA ring of planes (base f and g with G halo
-// rows, lam's output rows riding with the completing load), register queues
-// of the last 2G+1 planes of f and g, x/y partials on arrival, z terms at
-// output, one block barrier per plane.
+// rows), register queues of the last 2G+1 planes of f and g, one x/y partial,
+// z terms at output; lam is loaded at the end of the plane before its use.
 #pragma once
 
 #include "advect.cuh"
@@ -25,15 +24,13 @@
 namespace cup {
 
 struct AdjointMaps {
-  CUtensorMap main[6];  // f (3) then g (3), box {nx, TY, 1}
-  CUtensorMap halo[6];  // box {nx, G, 1}
-  CUtensorMap lam[3];   // point-wise lam, box {nx, TY, 1}
+  RowMaps f[6];         // f (3) then g (3)
 };
 
-template <typename T, int SCHEME, bool LAM, int TY, int NS, int CPT>
+template <typename T, int SCHEME, int TY, int NS>
 constexpr size_t adjoint_smem_bytes(int nx) {
   constexpr int G = SCHEME == 0 ? 1 : 2;
-  return (size_t)NS * (6 * (TY + 2 * G) + (LAM ? 3 * TY : 0)) * nx * sizeof(T) + NS * sizeof(uint64_t);
+  return (size_t)NS * 6 * (TY + 2 * G) * nx * sizeof(T) + PlaneRing<NS, G - 1, 6>::kBytes;
 }
 
 // transpose of the transport stencil at one point from the 5 products
@@ -62,69 +59,32 @@ __device__ __forceinline__ T tr_up3(T hm2, T hm1, T hp1, T hp2, T km2, T km1, T 
 
 template <typename T, int SCHEME, bool LAM, int TY, int NS, int CPT>
 __global__ void __launch_bounds__(512) k_adjoint_zq(const __grid_constant__ AdjointMaps maps, const StreamGeom g,
-                                                   T* __restrict__ ou, T* __restrict__ ov, T* __restrict__ ow,
+                                                   const T* lu, const T* lv, const T* lw, T* ou, T* ov, T* ow,
                                                    T alpha, T beta, DtArg dt, double h, double nu, double ux,
                                                    double uy, double uz, int* err) {
   pdl_entry();
   constexpr int G = SCHEME == 0 ? 1 : 2;
   constexpr int ROWS = TY + 2 * G;
   constexpr int Q = 2 * G + 1;
-  constexpr int U = (G == 1) ? 3 : 10;
   // a G-row halo box starting at y0 - G (wrapped) stays inside [0, ny) only if y0 is a multiple of TY >= G
   static_assert(TY >= G, "tile height must cover the halo depth");
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   unsigned char* smem_raw = smem_align128(smem_dyn);
-  const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const size_t field_elems = (size_t)ROWS * nx;
-  const size_t stencil_elems = 6 * field_elems;
-  const size_t slot_elems = stencil_elems + (LAM ? (size_t)3 * TY * nx : 0);
+  const int nx = g.nx, ny = g.ny, nz = g.nz, zc = g.zc;
+  static_assert(NS > G, "the ring must hold the planes in use and one in flight");
+  const int field_elems = ROWS * nx;
+  const int slot_elems = 6 * field_elems;
   T* slots = reinterpret_cast<T*>(smem_raw);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + NS * slot_elems * sizeof(T));
+  PlaneRing<NS, G - 1, 6> ring(smem_raw + (size_t)NS * slot_elems * sizeof(T), err);
   const int tid = threadIdx.x;
-  const int PL = g.zc + 2 * G;
-  const int my_items = blockIdx.x < g.n_items ? (g.n_items - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const int L = my_items * PL;
-  const uint32_t stencil_bytes = (uint32_t)(stencil_elems * sizeof(T));
-  const uint32_t lam_bytes = (uint32_t)(3 * TY * nx * sizeof(T));
-
-  if (tid == 0) {
-    for (int s = 0; s < NS; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-
-  auto issue = [&](int q) {
-    const int it = q / PL, j = q - it * PL;
-    const int item = blockIdx.x + it * gridDim.x;
-    const int ty = item % g.items_y, zi = item / g.items_y;
-    const int y0 = ty * TY, z0 = zi * g.zc;
-    int z = z0 - G + j;
+  const int PL = zc + 2 * G;
+  auto issue = [&](int f, int s, int j, const ItemPos& p) {
+    int z = p.z0 - G + j;
     z = z < 0 ? z + nz : (z >= nz ? z - nz : z);
-    const int s = q % NS;
-    T* dst = slots + s * slot_elems;
-    int ylo = y0 - G;
-    if (ylo < 0) ylo += ny;
-    int yhi = y0 + TY;
-    if (yhi >= ny) yhi -= ny;
-    const bool with_lam = LAM && j >= 2 * G;
-    mbar_arrive_expect_tx(&full[s], stencil_bytes + (with_lam ? lam_bytes : 0u));
-#pragma unroll
-    for (int f = 0; f < 6; ++f) {
-      T* fd = dst + f * field_elems;
-      tma_load_3d(fd, &maps.halo[f], 0, ylo, z, &full[s]);
-      tma_load_3d(fd + G * nx, &maps.main[f], 0, y0, z, &full[s]);
-      tma_load_3d(fd + (G + TY) * nx, &maps.halo[f], 0, yhi, z, &full[s]);
-    }
-    if (with_lam) {
-      const int zk = z0 + (j - 2 * G);
-#pragma unroll
-      for (int f = 0; f < 3; ++f) tma_load_3d(dst + stencil_elems + f * TY * nx, &maps.lam[f], 0, y0, zk, &full[s]);
-    }
+    mbar_arrive_expect_tx(&ring.full[s], (uint32_t)(field_elems * sizeof(T)));
+    tma_load_rows<G, TY>(slots + s * slot_elems + f * field_elems, maps.f[f], nx, ny, p.y0, z, &ring.full[s]);
   };
-
-  int q_issued = 0;
-  if (tid == 0)
-    for (; q_issued < min(L, NS); ++q_issued) issue(q_issued);
+  ring.start(item_pos(g, blockIdx.x, TY, zc), issue);
 
   const int mask = nx - 1;
   int cx[CPT], cy[CPT];
@@ -141,7 +101,9 @@ __global__ void __launch_bounds__(512) k_adjoint_zq(const __grid_constant__ Adjo
 
   T qf[3][Q][CPT];  // base field centre values, plane j in slot j % Q
   T qg[3][Q][CPT];  // adjoint input centre values
-  T part[3][G][CPT];
+  T part[3][CPT];
+  T lam[LAM ? 3 : 1][CPT];  // point-wise lam of the next output plane
+  const T* lsrc[3] = {lu, lv, lw};
 #pragma unroll
   for (int f = 0; f < 3; ++f)
 #pragma unroll
@@ -154,25 +116,25 @@ __global__ void __launch_bounds__(512) k_adjoint_zq(const __grid_constant__ Adjo
 #pragma unroll
   for (int f = 0; f < 3; ++f)
 #pragma unroll
-    for (int d = 0; d < G; ++d)
-#pragma unroll
-      for (int i = 0; i < CPT; ++i) part[f][d][i] = (T)0;
+    for (int i = 0; i < CPT; ++i) part[f][i] = (T)0;
 
   bool ok = true;
-  int q = 0;
-  for (int it = 0; it < my_items; ++it) {
-    const int item = blockIdx.x + it * gridDim.x;
-    const int ty = item % g.items_y, zi = item / g.items_y;
-    const int y0 = ty * TY, z0 = zi * g.zc;
-    for (int j0 = 0; j0 < PL; j0 += U) {
+  ItemPos pos = item_pos(g, blockIdx.x, TY, zc);
+  for (int item = blockIdx.x; item < g.n_items; item += gridDim.x) {
+    const bool more = item + gridDim.x < g.n_items;
+    const ItemPos nextp = item_pos(g, item + gridDim.x, TY, zc);
+    size_t o[CPT];  // output index of the next plane
 #pragma unroll
-      for (int jj = 0; jj < U; ++jj) {
+    for (int i = 0; i < CPT; ++i) o[i] = gidx(cx[i], pos.y0 + cy[i], pos.z0, nx, ny);
+    for (int j0 = 0; j0 < PL; j0 += Q) {
+#pragma unroll
+      for (int jj = 0; jj < Q; ++jj) {
         const int j = j0 + jj;
-        const int s = q % NS;
-        if (ok) ok = mbar_wait(&full[s], (q / NS) & 1, err);
+        if (j >= PL) break;
+        if (ok) ok = ring.wait();
         if (ok) {
-          const T* sl = slots + s * slot_elems;
-          const int QN = jj % Q;
+          const T* sl = slots + ring.slot * slot_elems;
+          const int QN = jj;
 #pragma unroll
           for (int f = 0; f < 3; ++f)
 #pragma unroll
@@ -183,14 +145,11 @@ __global__ void __launch_bounds__(512) k_adjoint_zq(const __grid_constant__ Adjo
             }
           // z terms and output of plane k = j - 2G
           if (j >= 2 * G) {
-            const int k = j - 2 * G;
             const int QC = (jj + 3 * Q - G) % Q;
             const int QM1 = (jj + 3 * Q - G - 1) % Q, QP1 = (jj + 3 * Q - G + 1) % Q;
             const int QM2 = (jj + 3 * Q - G - 2) % Q, QP2 = (jj + 3 * Q - G + 2) % Q;
-            const int PS = jj % G;
 #pragma unroll
             for (int i = 0; i < CPT; ++i) {
-              const size_t o = gidx(cx[i], y0 + cy[i], z0 + k, nx, ny);
               const T azc = qf[2][QC][i] + uinf[2];
               // adjoint of a_z at the cell: sum_q' g_q' D_z(f_q')
               T advz = (T)0;
@@ -215,38 +174,40 @@ __global__ void __launch_bounds__(512) k_adjoint_zq(const __grid_constant__ Adjo
                               tabs(am2) * qg[f][QM2][i], tabs(am1) * qg[f][QM1][i], tabs(azc) * g0,
                               tabs(ap1) * qg[f][QP1][i], tabs(ap2) * qg[f][QP2][i]);
                 }
-                T v = part[f][PS][i] + facD * (qg[f][QM1][i] + qg[f][QP1][i] - g0 * 6) + facA * tz;
+                T v = part[f][i] + facD * (qg[f][QM1][i] + qg[f][QP1][i] - g0 * 6) + facA * tz;
                 if (f == 2) v += facA * advz;
                 outv[f] = v;
               }
               if constexpr (LAM) {
-                const T* ls = sl + stencil_elems + cy[i] * nx + cx[i];
-                ou[o] = alpha * ls[0] + beta * outv[0];
-                ov[o] = alpha * ls[TY * nx] + beta * outv[1];
-                ow[o] = alpha * ls[2 * TY * nx] + beta * outv[2];
+#pragma unroll
+                for (int f = 0; f < 3; ++f) outv[f] = alpha * lam[f][i] + beta * outv[f];
               } else {
-                ou[o] = beta * outv[0];
-                ov[o] = beta * outv[1];
-                ow[o] = beta * outv[2];
+#pragma unroll
+                for (int f = 0; f < 3; ++f) outv[f] = beta * outv[f];
               }
+              ou[o[i]] = outv[0];
+              ov[o[i]] = outv[1];
+              ow[o[i]] = outv[2];
+              o[i] += (size_t)nx * ny;
             }
           }
-          // x/y partial of plane j
-          if (j >= G && j < G + g.zc) {
-            const int PS = jj % G;
+          // x/y partial of plane j - G + 1 (output plane j - 2G + 1)
+          if (j >= 2 * G - 1 && j < PL - 1) {
+            const T* sp = slots + ring.slot_back(G - 1) * slot_elems;
+            const int QX = (jj + Q - G + 1) % Q;
 #pragma unroll
             for (int i = 0; i < CPT; ++i) {
               const int x = cx[i], r = G + cy[i];
               const int xm1 = (x - 1) & mask, xp1 = (x + 1) & mask, xm2 = (x - 2) & mask, xp2 = (x + 2) & mask;
-              const T* Fx = sl;                    // base u (advects in x)
-              const T* Fy = sl + field_elems;      // base v (advects in y)
-              const T ax0 = qf[0][QN][i] + uinf[0], ay0 = qf[1][QN][i] + uinf[1];
+              const T* Fx = sp;                    // base u (advects in x)
+              const T* Fy = sp + field_elems;      // base v (advects in y)
+              const T ax0 = qf[0][QX][i] + uinf[0], ay0 = qf[1][QX][i] + uinf[1];
               // adjoints of a_x, a_y at the cell: sum_q' g_q' D(f_q')
               T advx = (T)0, advy = (T)0;
 #pragma unroll
               for (int f = 0; f < 3; ++f) {
-                const T* F = sl + f * field_elems;
-                const T f0 = qf[f][QN][i], gq = qg[f][QN][i];
+                const T* F = sp + f * field_elems;
+                const T f0 = qf[f][QX][i], gq = qg[f][QX][i];
                 T dx, dy;
                 if constexpr (SCHEME == 0) {
                   dx = F[r * nx + xp1] - F[r * nx + xm1];
@@ -260,8 +221,8 @@ __global__ void __launch_bounds__(512) k_adjoint_zq(const __grid_constant__ Adjo
               }
 #pragma unroll
               for (int f = 0; f < 3; ++f) {
-                const T* Gf = sl + (3 + f) * field_elems;
-                const T g0 = qg[f][QN][i];
+                const T* Gf = sp + (3 + f) * field_elems;
+                const T g0 = qg[f][QX][i];
                 const T gxm1 = Gf[r * nx + xm1], gxp1 = Gf[r * nx + xp1];
                 const T gym1 = Gf[(r - 1) * nx + x], gyp1 = Gf[(r + 1) * nx + x];
                 T tx, ty;
@@ -283,20 +244,24 @@ __global__ void __launch_bounds__(512) k_adjoint_zq(const __grid_constant__ Adjo
                 T v = g0 + facD * (gyp1 + gym1 + gxp1 + gxm1) + facA * (tx + ty);
                 if (f == 0) v += facA * advx;
                 if (f == 1) v += facA * advy;
-                part[f][PS][i] = v;
+                part[f][i] = v;
               }
+            }
+            if constexpr (LAM) {
+              // of output plane j - 2G + 1, finished by the next plane
+#pragma unroll
+              for (int i = 0; i < CPT; ++i)
+#pragma unroll
+                for (int f = 0; f < 3; ++f) lam[f][i] = lsrc[f][o[i]];
             }
           }
         }
-        __syncthreads();
-        if (tid == 0 && ok && q_issued < L && q_issued == q + NS) issue(q_issued++);
-        ++q;
+        ring.step(ok, ring.n & 1, j, PL, pos, nextp, more, issue);
       }
     }
+    pos = nextp;
   }
-  if (!ok && tid == 0) {
-    for (int r = q - NS < 0 ? 0 : q - NS; r < q_issued; ++r) mbar_wait(&full[r % NS], (r / NS) & 1, nullptr);
-  }
+  ring.drain(ok);
 }
 
 }  // namespace cup

@@ -14,9 +14,8 @@
 // up3_da). The 1/2 is folded into facA. A thread owns PPT pairs (x, x+1) of a
 // TY x nx tile and marches down z: TMA ring of planes of the six fields (base
 // f, adjoint input g; G = 2 halo rows), register queues of the last 5 planes
-// of both, the x/y part of each plane on arrival and the z part two planes
-// later; LAM: out = alpha lam + beta (...), the lam rows riding with the
-// completing load. In x, the pairs at x -+ 2 come in whole and the values at
+// of both, one x/y partial and the z part a plane later; LAM: out = alpha lam +
+// beta (...), lam loaded at the end of the plane before its use. In x, the pairs at x -+ 2 come in whole and the values at
 // x -+ 1 straddle two pairs, so the terms at -+1 go in as scalar FMAs.
 #pragma once
 
@@ -51,79 +50,39 @@ __device__ __forceinline__ void sq_pairs(float2 fm2, float2 fm1, float2 f0, floa
   Qs = fma2(splat2(6.f), f0, fma2(splat2(-4.f), add2(fm1, fp1), add2(fm2, fp2)));
 }
 
-template <bool LAM, int TY, int NS, int PPT, int NXC = 0, int ZCC = 0>
+template <int TY, int NS>
 constexpr size_t adjoint_f2_smem_bytes(int nx) {
-  return (size_t)NS * (6 * (TY + 4) + (LAM ? 3 * TY : 0)) * nx * sizeof(float) + NS * sizeof(uint64_t);
+  return (size_t)NS * 6 * (TY + 4) * nx * sizeof(float) + PlaneRing<NS, 1, 6>::kBytes;
 }
 
-// blockDim.x * PPT * 2 == TY * nx (<= 512 threads). NXC, ZCC: nx and the
-// planes per work item fixed at compile time (0: read from g).
-template <bool LAM, int TY, int NS, int PPT, int NXC = 0, int ZCC = 0>
+// blockDim.x * PPT * 2 == TY * nx (<= 512 threads). NXC: nx fixed at compile
+// time (0: read from g).
+template <bool LAM, int TY, int NS, int PPT, int NXC = 0>
 __global__ void __launch_bounds__(512) k_adjoint_zq_f2(const __grid_constant__ AdjointMaps maps, const StreamGeom g,
-                                                      float* __restrict__ ou, float* __restrict__ ov,
-                                                      float* __restrict__ ow, float alpha, float beta, DtArg dt,
+                                                      const float* lu, const float* lv, const float* lw, float* ou,
+                                                      float* ov, float* ow, float alpha, float beta, DtArg dt,
                                                       double h, double nu, double ux, double uy, double uz, int* err) {
   pdl_entry();
   constexpr int G = 2;
   constexpr int ROWS = TY + 2 * G;
   constexpr int Q = 2 * G + 1;
-  constexpr int U = ZCC ? ZCC + 2 * G : 10;  // planes per unrolled chunk: a whole item, or lcm(Q, G)
-  static_assert(ZCC == 0 || ZCC % 2 == 0, "items of an even plane count");
   static_assert(TY >= G, "tile height must cover the halo depth");
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   unsigned char* smem_raw = smem_align128(smem_dyn);
-  const int nx = NXC ? NXC : g.nx, ny = g.ny, nz = g.nz;
-  const int zc = ZCC ? ZCC : g.zc;
-  const size_t field_elems = (size_t)ROWS * nx;
-  const size_t stencil_elems = 6 * field_elems;
-  const size_t slot_elems = stencil_elems + (LAM ? (size_t)3 * TY * nx : 0);
+  const int nx = NXC ? NXC : g.nx, ny = g.ny, nz = g.nz, zc = g.zc;
+  const int field_elems = ROWS * nx;
+  const int slot_elems = 6 * field_elems;
   float* slots = reinterpret_cast<float*>(smem_raw);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + NS * slot_elems * sizeof(float));
+  PlaneRing<NS, 1, 6> ring(smem_raw + (size_t)NS * slot_elems * sizeof(float), err);
   const int tid = threadIdx.x;
   const int PL = zc + 2 * G;
-  const int my_items = blockIdx.x < g.n_items ? (g.n_items - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const int L = my_items * PL;
-  const uint32_t stencil_bytes = (uint32_t)(stencil_elems * sizeof(float));
-  const uint32_t lam_bytes = (uint32_t)(3 * TY * nx * sizeof(float));
-
-  if (tid == 0) {
-    for (int s = 0; s < NS; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-
-  auto issue = [&](int q) {
-    const int it = q / PL, j = q - it * PL;
-    const int item = blockIdx.x + it * gridDim.x;
-    const int ty = item % g.items_y, zi = item / g.items_y;
-    const int y0 = ty * TY, z0 = zi * zc;
-    int z = z0 - G + j;
+  auto issue = [&](int f, int s, int j, const ItemPos& p) {
+    int z = p.z0 - G + j;
     z = z < 0 ? z + nz : (z >= nz ? z - nz : z);
-    const int s = q % NS;
-    float* dst = slots + s * slot_elems;
-    int ylo = y0 - G;
-    if (ylo < 0) ylo += ny;
-    int yhi = y0 + TY;
-    if (yhi >= ny) yhi -= ny;
-    const bool with_lam = LAM && j >= 2 * G;
-    mbar_arrive_expect_tx(&full[s], stencil_bytes + (with_lam ? lam_bytes : 0u));
-#pragma unroll
-    for (int f = 0; f < 6; ++f) {
-      float* fd = dst + f * field_elems;
-      tma_load_3d(fd, &maps.halo[f], 0, ylo, z, &full[s]);
-      tma_load_3d(fd + G * nx, &maps.main[f], 0, y0, z, &full[s]);
-      tma_load_3d(fd + (G + TY) * nx, &maps.halo[f], 0, yhi, z, &full[s]);
-    }
-    if (with_lam) {
-      const int zk = z0 + (j - 2 * G);
-#pragma unroll
-      for (int f = 0; f < 3; ++f) tma_load_3d(dst + stencil_elems + f * TY * nx, &maps.lam[f], 0, y0, zk, &full[s]);
-    }
+    mbar_arrive_expect_tx(&ring.full[s], (uint32_t)(field_elems * sizeof(float)));
+    tma_load_rows<G, TY>(slots + s * slot_elems + f * field_elems, maps.f[f], nx, ny, p.y0, z, &ring.full[s]);
   };
-
-  int q_issued = 0;
-  if (tid == 0)
-    for (; q_issued < min(L, NS); ++q_issued) issue(q_issued);
+  ring.start(item_pos(g, blockIdx.x, TY, zc), issue);
 
   const int mask = nx - 1;
   const int half = nx >> 1;
@@ -147,7 +106,9 @@ __global__ void __launch_bounds__(512) k_adjoint_zq_f2(const __grid_constant__ A
 
   float2 qf[3][Q][PPT];  // base field pairs, plane j in slot j % Q
   float2 qg[3][Q][PPT];  // adjoint input pairs
-  float2 part[3][G][PPT];
+  float2 part[3][PPT];
+  float2 lam[LAM ? 3 : 1][PPT];  // point-wise lam of the next output plane
+  const float* lsrc[3] = {lu, lv, lw};
 #pragma unroll
   for (int f = 0; f < 3; ++f)
 #pragma unroll
@@ -160,29 +121,25 @@ __global__ void __launch_bounds__(512) k_adjoint_zq_f2(const __grid_constant__ A
 #pragma unroll
   for (int f = 0; f < 3; ++f)
 #pragma unroll
-    for (int d = 0; d < G; ++d)
-#pragma unroll
-      for (int i = 0; i < PPT; ++i) part[f][d][i] = splat2(0.f);
+    for (int i = 0; i < PPT; ++i) part[f][i] = splat2(0.f);
 
   bool ok = true;
-  int q = 0;
-  for (int it = 0; it < my_items; ++it) {
-    const int item = blockIdx.x + it * gridDim.x;
-    const int ty = item % g.items_y, zi = item / g.items_y;
-    const int y0 = ty * TY, z0 = zi * zc;
-    size_t obase[PPT];
+  ItemPos pos = item_pos(g, blockIdx.x, TY, zc);
+  for (int item = blockIdx.x; item < g.n_items; item += gridDim.x) {
+    const bool more = item + gridDim.x < g.n_items;
+    const ItemPos nextp = item_pos(g, item + gridDim.x, TY, zc);
+    size_t o[PPT];  // output index of the next plane
 #pragma unroll
-    for (int i = 0; i < PPT; ++i) obase[i] = gidx(px[i], y0 + cy[i], z0, nx, ny);
-    for (int j0 = 0; j0 < PL; j0 += U) {
+    for (int i = 0; i < PPT; ++i) o[i] = gidx(px[i], pos.y0 + cy[i], pos.z0, nx, ny);
+    for (int j0 = 0; j0 < PL; j0 += Q) {
 #pragma unroll
-      for (int jj = 0; jj < U; ++jj) {
+      for (int jj = 0; jj < Q; ++jj) {
         const int j = j0 + jj;
         if (j >= PL) break;
-        const int s = q % NS;
-        if (ok) ok = mbar_wait(&full[s], (q / NS) & 1, err);
+        if (ok) ok = ring.wait();
         if (ok) {
-          const float* sl = slots + s * slot_elems;
-          const int QN = jj % Q;
+          const float* sl = slots + ring.slot * slot_elems;
+          const int QN = jj;
 #pragma unroll
           for (int f = 0; f < 3; ++f)
 #pragma unroll
@@ -192,14 +149,11 @@ __global__ void __launch_bounds__(512) k_adjoint_zq_f2(const __grid_constant__ A
             }
           // z terms and output of plane k = j - 2G
           if (j >= 2 * G) {
-            const int k = j - 2 * G;
             const int QC = (jj + 3 * Q - G) % Q;
             const int QM1 = (jj + 3 * Q - G - 1) % Q, QP1 = (jj + 3 * Q - G + 1) % Q;
             const int QM2 = (jj + 3 * Q - G - 2) % Q, QP2 = (jj + 3 * Q - G + 2) % Q;
-            const int PS = jj % G;
 #pragma unroll
             for (int i = 0; i < PPT; ++i) {
-              const size_t o = obase[i] + (size_t)k * plane;
               const float2 am2 = add2(qf[2][QM2][i], uinf[2]), am1 = add2(qf[2][QM1][i], uinf[2]);
               const float2 a0 = add2(qf[2][QC][i], uinf[2]);
               const float2 ap1 = add2(qf[2][QP1][i], uinf[2]), ap2 = add2(qf[2][QP2][i], uinf[2]);
@@ -221,39 +175,39 @@ __global__ void __launch_bounds__(512) k_adjoint_zq_f2(const __grid_constant__ A
                                             qg[f][QP1][i], qg[f][QP2][i]);
                 // Lap_z with the centre's -6 g0
                 const float2 lz = fma2(splat2(-6.f), g0, add2(qg[f][QM1][i], qg[f][QP1][i]));
-                float2 v = fma2(facD, lz, fma2(facA, tz, part[f][PS][i]));
+                float2 v = fma2(facD, lz, fma2(facA, tz, part[f][i]));
                 if (f == 2) v = fma2(facA, advz, v);
                 outv[f] = v;
               }
               if constexpr (LAM) {
-                const float* ls = sl + stencil_elems + cy[i] * nx + px[i];
 #pragma unroll
-                for (int f = 0; f < 3; ++f)
-                  outv[f] = fma2(alpha2, *reinterpret_cast<const float2*>(ls + f * TY * nx), mul2(beta2, outv[f]));
+                for (int f = 0; f < 3; ++f) outv[f] = fma2(alpha2, lam[f][i], mul2(beta2, outv[f]));
               } else {
 #pragma unroll
                 for (int f = 0; f < 3; ++f) outv[f] = mul2(beta2, outv[f]);
               }
-              *reinterpret_cast<float2*>(ou + o) = outv[0];
-              *reinterpret_cast<float2*>(ov + o) = outv[1];
-              *reinterpret_cast<float2*>(ow + o) = outv[2];
+              *reinterpret_cast<float2*>(ou + o[i]) = outv[0];
+              *reinterpret_cast<float2*>(ov + o[i]) = outv[1];
+              *reinterpret_cast<float2*>(ow + o[i]) = outv[2];
+              o[i] += plane;
             }
           }
-          // x/y part of plane j
-          if (j >= G && j < G + zc) {
-            const int PS = jj % G;
+          // x/y partial of plane j - 1 (output plane j - 2G + 1)
+          if (j >= 2 * G - 1 && j < PL - 1) {
+            const float* sp = slots + ring.slot_back(1) * slot_elems;
+            const int QX = (jj + Q - 1) % Q;
 #pragma unroll
             for (int i = 0; i < PPT; ++i) {
-              const float* Fx = sl;                // base u (advects in x)
-              const float* Fy = sl + field_elems;  // base v (advects in y)
+              const float* Fx = sp;                // base u (advects in x)
+              const float* Fy = sp + field_elems;  // base v (advects in y)
               const int c = ctr[i];
               // advecting velocities: x at x-2..x+3 (pairs A, C, B), y at rows -2..2
               const float2 axA = add2(*reinterpret_cast<const float2*>(Fx + xl[i]), uinf[0]);
-              const float2 axC = add2(qf[0][QN][i], uinf[0]);
+              const float2 axC = add2(qf[0][QX][i], uinf[0]);
               const float2 axB = add2(*reinterpret_cast<const float2*>(Fx + xr[i]), uinf[0]);
               const float2 aym2 = add2(*reinterpret_cast<const float2*>(Fy + c - 2 * nx), uinf[1]);
               const float2 aym1 = add2(*reinterpret_cast<const float2*>(Fy + c - nx), uinf[1]);
-              const float2 ay0 = add2(qf[1][QN][i], uinf[1]);
+              const float2 ay0 = add2(qf[1][QX][i], uinf[1]);
               const float2 ayp1 = add2(*reinterpret_cast<const float2*>(Fy + c + nx), uinf[1]);
               const float2 ayp2 = add2(*reinterpret_cast<const float2*>(Fy + c + 2 * nx), uinf[1]);
               const float2 kxA = abs2(axA), kxC = abs2(axC), kxB = abs2(axB);
@@ -261,11 +215,11 @@ __global__ void __launch_bounds__(512) k_adjoint_zq_f2(const __grid_constant__ A
               float2 sSx = splat2(0.f), sQx = splat2(0.f), sSy = splat2(0.f), sQy = splat2(0.f);
 #pragma unroll
               for (int f = 0; f < 3; ++f) {
-                const float* F = sl + f * field_elems;
+                const float* F = sp + f * field_elems;
                 const float2 fA = *reinterpret_cast<const float2*>(F + xl[i]);
-                const float2 fC = qf[f][QN][i];
+                const float2 fC = qf[f][QX][i];
                 const float2 fB = *reinterpret_cast<const float2*>(F + xr[i]);
-                const float2 gq = qg[f][QN][i];
+                const float2 gq = qg[f][QX][i];
                 // x: S = f-2 - 8 f-1 + 8 f+1 - f+2, Q = f-2 - 4 f-1 + 6 f0 - 4 f+1 + f+2
                 float2 Sx = sub2(fA, fB);  // the -+2 terms of each lane
                 Sx.x = fmaf(8.f, fC.y - fA.y, Sx.x);
@@ -286,9 +240,9 @@ __global__ void __launch_bounds__(512) k_adjoint_zq_f2(const __grid_constant__ A
               const float2 advy = fma2(sgn2(ay0), sQy, sSy);
 #pragma unroll
               for (int f = 0; f < 3; ++f) {
-                const float* Gf = sl + (3 + f) * field_elems;
+                const float* Gf = sp + (3 + f) * field_elems;
                 const float2 gA = *reinterpret_cast<const float2*>(Gf + xl[i]);
-                const float2 g0 = qg[f][QN][i];
+                const float2 g0 = qg[f][QX][i];
                 const float2 gB = *reinterpret_cast<const float2*>(Gf + xr[i]);
                 const float2 gym2 = *reinterpret_cast<const float2*>(Gf + c - 2 * nx);
                 const float2 gym1 = *reinterpret_cast<const float2*>(Gf + c - nx);
@@ -308,22 +262,24 @@ __global__ void __launch_bounds__(512) k_adjoint_zq_f2(const __grid_constant__ A
                 float2 v = fma2(facD, lxy, fma2(facA, add2(tx, ty), g0));
                 if (f == 0) v = fma2(facA, advx, v);
                 if (f == 1) v = fma2(facA, advy, v);
-                part[f][PS][i] = v;
+                part[f][i] = v;
               }
+            }
+            if constexpr (LAM) {
+              // of output plane j - 2G + 1, finished by the next plane
+#pragma unroll
+              for (int i = 0; i < PPT; ++i)
+#pragma unroll
+                for (int f = 0; f < 3; ++f) lam[f][i] = *reinterpret_cast<const float2*>(lsrc[f] + o[i]);
             }
           }
         }
-        __syncthreads();  // slot s fully consumed
-        if (tid == 0 && ok && q_issued < L && q_issued == q + NS) issue(q_issued++);
-        ++q;
+        ring.step(ok, ring.n & 1, j, PL, pos, nextp, more, issue);
       }
     }
+    pos = nextp;
   }
-  // after a timed-out wait: bounded drain of the loads that may be in flight
-  if (!ok && tid == 0) {
-    for (int r = q_issued - NS < 0 ? 0 : q_issued - NS; r < q_issued; ++r)
-      mbar_wait(&full[r % NS], (r / NS) & 1, nullptr);
-  }
+  ring.drain(ok);
 }
 
 }  // namespace cup

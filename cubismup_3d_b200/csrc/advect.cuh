@@ -6,18 +6,29 @@
 // Each thread owns CPT fixed (x, y) columns of a TY x nx row tile and marches
 // down z. Planes arrive by TMA into a ring of NS shared-memory slots (TY main
 // rows plus G periodic halo rows per field; the x halo is the row's periodic
-// wrap). When plane j lands, a thread
+// wrap; PlaneRing). When plane j lands, a thread
 //   1. pushes its columns' centre values into a register queue of the last
 //      2G+1 planes (the z stencil),
-//   2. finishes output plane j-2G: adds the z terms (from the queue) to the
-//      x/y partial it computed G planes earlier, and stores it,
-//   3. computes the x/y partial of plane j (x/y neighbours from shared memory,
-//      advecting velocity from the queue),
-// and the slot is released at once: only planes in flight occupy shared
-// memory, so NS-1 planes of loads are always outstanding. For RK2 stage 2 the
-// point-wise base rows u^n of the output plane ride in the same slot as the
-// load that completes it. Work items (TY rows x ZC planes) of a CTA form one
-// flat load stream, so the pipeline never drains between items.
+//   2. finishes output plane j-2G: adds the z terms (from the queue) to that
+//      plane's x/y partial, and stores it,
+//   3. computes the x/y partial of output plane j-2G+1, plane j-G+1 of the
+//      stream (x/y neighbours from its slot, advecting velocity from the
+//      queue), and releases the slot of that plane,
+// so one partial per column is alive and only G planes are held in shared
+// memory. For RK2 stage 2 the point-wise base values u^n are loaded at the end
+// of the plane before their use. Work items (TY rows x ZC planes) of a CTA form
+// one flat load stream, so the pipeline never drains between items.
+//
+// The upwind3 stages were bound by the FP64 pipe (about 130 FP64 instructions
+// per cell with both one-sided stencils evaluated) and by shared-memory reads.
+// Their update is written with four taps per direction whose weights depend on
+// the advecting velocity a only, with B = dt |a| / 6h and D = nu dt / h^2:
+//   upwind neighbour 6 B + D, downwind neighbour D - 2 B, second upwind cell -B,
+//   centre -3 B - 2 D,
+// so the three components share them and a tap costs one FMA (about 50 FP64
+// instructions per cell); the neighbours swap weights with the sign of a, the
+// second upwind cell is one select (x: of its address). A thread's two columns
+// are two rows of one x (six row loads serve both).
 #pragma once
 
 #include "common.cuh"
@@ -27,152 +38,125 @@
 namespace cup {
 
 struct AdvectMaps {
-  CUtensorMap main[3];  // stencil fields, box {nx, TY, 1}
-  CUtensorMap halo[3];  // stencil fields, box {nx, G, 1}
-  CUtensorMap base[3];  // stage-2 point-wise fields, box {nx, TY, 1}
+  RowMaps f[3];         // stencil fields
+  CUtensorMap base[3];  // (k_advect_zq_f2, stage 2) point-wise fields, box {nx, TY, 1}
 };
 
 // SCHEME 0: central2 (reference) Euler; 1: upwind3 stage 1; 2: upwind3 stage 2.
 template <int SCHEME>
 struct AdvectTraits {
   static constexpr int G = SCHEME == 0 ? 1 : 2;
-  static constexpr bool BASE = SCHEME == 2;
 };
 
-template <typename T, int SCHEME, int TY, int NS, int CPT>
+template <typename T, int SCHEME, int TY, int NS>
 constexpr size_t advect_smem_bytes(int nx) {
-  constexpr int G = AdvectTraits<SCHEME>::G;
-  return (size_t)NS * (3 * (TY + 2 * G) + (AdvectTraits<SCHEME>::BASE ? 3 * TY : 0)) * nx * sizeof(T) +
-         NS * sizeof(uint64_t);
+  return (size_t)NS * 3 * (TY + 2 * AdvectTraits<SCHEME>::G) * nx * sizeof(T) +
+         PlaneRing<NS, AdvectTraits<SCHEME>::G - 1, 3>::kBytes;
+}
+
+// The weights of one direction of an upwind3 update (see the head of the file):
+// m1, p1 of the neighbours at -1 and +1, far = -B of the second upwind cell.
+template <typename T>
+struct UpW {
+  T m1, p1, far;
+  bool pos;
+};
+template <typename T>
+__device__ __forceinline__ UpW<T> up_weights(T a, T absA, T facD) {
+  const T B = absA * fabs(a);
+  const T wu = (T)6 * B + facD, wd = facD - (T)2 * B;
+  UpW<T> w;
+  w.pos = a > (T)0;
+  w.m1 = w.pos ? wu : wd;
+  w.p1 = w.pos ? wd : wu;
+  w.far = -B;
+  return w;
 }
 
 // blockDim.x * CPT must equal TY * nx (<= 512 threads).
-// NXC, ZCC: nx and the planes per work item fixed at compile time (0: read
-// from g); fixed, the stencil's shared-memory offsets are immediates and the
-// ring slot of each plane is known when NS divides the item's plane count.
-template <typename T, int SCHEME, int TY, int NS, int CPT, int NXC = 0, int ZCC = 0>
+// NXC: nx fixed at compile time (0: read from g); fixed, the stencil's
+// shared-memory offsets are immediates.
+// Columns of a thread: SCHEME 0, tid + i blockDim.x; upwind3, rows CPT (tid / nx) + i of x = tid % nx.
+// bu, bv, bw: u^n of stage 2 (else unused).
+template <typename T, int SCHEME, int TY, int NS, int CPT, int NXC = 0>
 __global__ void __launch_bounds__(512) k_advect_zq(const __grid_constant__ AdvectMaps maps, const StreamGeom g,
-                                                  T* __restrict__ ou, T* __restrict__ ov, T* __restrict__ ow, DtArg dt,
-                                                  double h, double nu, double ux, double uy, double uz, int* err) {
+                                                  const T* __restrict__ bu, const T* __restrict__ bv,
+                                                  const T* __restrict__ bw, T* __restrict__ ou, T* __restrict__ ov,
+                                                  T* __restrict__ ow, DtArg dt, double h, double nu, double ux,
+                                                  double uy, double uz, int* err) {
   pdl_entry();
   constexpr int G = AdvectTraits<SCHEME>::G;
-  constexpr bool BASE = AdvectTraits<SCHEME>::BASE;
+  constexpr bool UP = SCHEME != 0, BASE = SCHEME == 2;
   constexpr int ROWS = TY + 2 * G;
   constexpr int Q = 2 * G + 1;
   // a G-row halo box starting at y0 - G (wrapped) stays inside [0, ny) only if y0 is a multiple of TY >= G
   static_assert(TY >= G, "tile height must cover the halo depth");
+  static_assert(NS > G, "the ring must hold the planes in use and one in flight");
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   unsigned char* smem_raw = smem_align128(smem_dyn);
-  const int nx = NXC ? NXC : g.nx, ny = g.ny, nz = g.nz;
-  const int zc = ZCC ? ZCC : g.zc;
-  const size_t field_elems = (size_t)ROWS * nx;
-  const size_t stencil_elems = 3 * field_elems;
-  const size_t slot_elems = stencil_elems + (BASE ? (size_t)3 * TY * nx : 0);
+  const int nx = NXC ? NXC : g.nx, ny = g.ny, nz = g.nz, zc = g.zc;
+  const int field_elems = ROWS * nx;
+  const int slot_elems = 3 * field_elems;
   T* slots = reinterpret_cast<T*>(smem_raw);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + NS * slot_elems * sizeof(T));
+  PlaneRing<NS, G - 1, 3> ring(smem_raw + (size_t)NS * slot_elems * sizeof(T), err);
   const int tid = threadIdx.x;
   const int PL = zc + 2 * G;
-  const int my_items = blockIdx.x < g.n_items ? (g.n_items - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const int L = my_items * PL;
-  const uint32_t stencil_bytes = (uint32_t)(stencil_elems * sizeof(T));
-  const uint32_t base_bytes = (uint32_t)(3 * TY * nx * sizeof(T));
-
-  if (tid == 0) {
-    for (int s = 0; s < NS; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-
-  auto issue = [&](int q) {
-    const int it = q / PL, j = q - it * PL;
-    const int item = blockIdx.x + it * gridDim.x;
-    const int ty = item % g.items_y, zi = item / g.items_y;
-    const int y0 = ty * TY, z0 = zi * zc;
-    int z = z0 - G + j;
+  auto issue = [&](int f, int s, int j, const ItemPos& p) {
+    int z = p.z0 - G + j;
     z = z < 0 ? z + nz : (z >= nz ? z - nz : z);
-    const int s = q % NS;
-    T* dst = slots + s * slot_elems;
-    int ylo = y0 - G;
-    if (ylo < 0) ylo += ny;
-    int yhi = y0 + TY;
-    if (yhi >= ny) yhi -= ny;
-    const bool with_base = BASE && j >= 2 * G;
-    mbar_arrive_expect_tx(&full[s], stencil_bytes + (with_base ? base_bytes : 0u));
-#pragma unroll
-    for (int f = 0; f < 3; ++f) {
-      T* fd = dst + f * field_elems;
-      tma_load_3d(fd, &maps.halo[f], 0, ylo, z, &full[s]);
-      tma_load_3d(fd + G * nx, &maps.main[f], 0, y0, z, &full[s]);
-      tma_load_3d(fd + (G + TY) * nx, &maps.halo[f], 0, yhi, z, &full[s]);
-    }
-    if (with_base) {
-      const int zk = z0 + (j - 2 * G);  // output plane completed by this load (< nz)
-#pragma unroll
-      for (int f = 0; f < 3; ++f) tma_load_3d(dst + stencil_elems + f * TY * nx, &maps.base[f], 0, y0, zk, &full[s]);
-    }
+    mbar_arrive_expect_tx(&ring.full[s], (uint32_t)(field_elems * sizeof(T)));
+    tma_load_rows<G, TY>(slots + s * slot_elems + f * field_elems, maps.f[f], nx, ny, p.y0, z, &ring.full[s]);
   };
-
-  int q_issued = 0;
-  if (tid == 0)
-    for (; q_issued < min(L, NS); ++q_issued) issue(q_issued);
+  ring.start(item_pos(g, blockIdx.x, TY, zc), issue);
 
   const int mask = nx - 1;
   int cx[CPT], cy[CPT];
 #pragma unroll
   for (int i = 0; i < CPT; ++i) {
-    const int c = tid + i * blockDim.x;
+    const int c = UP ? tid : tid + i * blockDim.x;
     cx[i] = c & mask;
     cy[i] = NXC ? c / NXC : c >> g.log2nx;
+    if constexpr (UP) cy[i] = CPT * cy[i] + i;
   }
   const double dtv = dt.get();
-  const T facA = (T)(SCHEME == 0 ? -dtv / (2 * h) : -dtv / (6 * h));
+  const T facA = (T)(SCHEME == 0 ? -dtv / (2 * h) : dtv / (6 * h));  // upwind3: the B of the weights over |a|
   const T facD = (T)((nu / h) * (dtv / h));
   const T uinf[3] = {(T)ux, (T)uy, (T)uz};
 
-  // Register rings: qv holds the centre values of the last Q = 2G+1 planes
-  // (plane j in slot j % Q), part the x/y partials awaiting their z terms
-  // (the partial of load j in slot j % G). The plane loop is unrolled by
-  // U = lcm(Q, G) and every item's PL = ZC + 2G planes is a multiple of U, so
-  // all ring indices fold to constants: no register shuffling.
-  constexpr int U = ZCC ? ZCC + 2 * G : ((G == 1) ? 3 : 10);
-  constexpr bool SLOT_CT = ZCC != 0 && (ZCC + 2 * G) % NS == 0;  // ring slot of plane j is j % NS
-  static_assert(ZCC % 2 == 0, "paired barriers need an even plane count");
+  // qv: the centre values of the last Q planes (plane j in slot j % Q); the
+  // plane loop is unrolled by Q, so the ring indices fold to constants.
   T qv[3][Q][CPT];
-  T part[3][G][CPT];
+  T part[3][CPT];
+  T base[BASE ? 3 : 1][CPT];  // u^n of the next output plane
+  const T* bsrc[3] = {bu, bv, bw};
 #pragma unroll
   for (int f = 0; f < 3; ++f)
 #pragma unroll
-    for (int d = 0; d < Q; ++d)
+    for (int i = 0; i < CPT; ++i) {
+      part[f][i] = (T)0;
 #pragma unroll
-      for (int i = 0; i < CPT; ++i) qv[f][d][i] = (T)0;
-#pragma unroll
-  for (int f = 0; f < 3; ++f)
-#pragma unroll
-    for (int d = 0; d < G; ++d)
-#pragma unroll
-      for (int i = 0; i < CPT; ++i) part[f][d][i] = (T)0;
+      for (int d = 0; d < Q; ++d) qv[f][d][i] = (T)0;
+    }
 
-  // One block barrier per plane (slot release). Each thread waits on the
-  // slot's mbarrier itself; a thread whose wait timed out stops waiting and
-  // computing but keeps taking the barrier, so the block never deadlocks and
-  // the error word tells the host.
+  // A thread whose wait timed out stops waiting and computing but keeps
+  // releasing slots, so the block never deadlocks and the error word tells the host.
   bool ok = true;
-  int q = 0;
-  for (int it = 0; it < my_items; ++it) {
-    const int item = blockIdx.x + it * gridDim.x;
-    const int ty = item % g.items_y, zi = item / g.items_y;
-    const int y0 = ty * TY, z0 = zi * zc;
-    const int q0 = q;  // first load of the item (a multiple of NS when SLOT_CT)
-    for (int j0 = 0; j0 < PL; j0 += U) {
+  ItemPos pos = item_pos(g, blockIdx.x, TY, zc);
+  for (int item = blockIdx.x; item < g.n_items; item += gridDim.x) {
+    const bool more = item + gridDim.x < g.n_items;
+    const ItemPos nextp = item_pos(g, item + gridDim.x, TY, zc);
+    size_t o[CPT];  // output index of the next plane
 #pragma unroll
-      for (int jj = 0; jj < U; ++jj) {
+    for (int i = 0; i < CPT; ++i) o[i] = gidx(cx[i], pos.y0 + cy[i], pos.z0, nx, ny);
+    for (int j0 = 0; j0 < PL; j0 += Q) {
+#pragma unroll
+      for (int jj = 0; jj < Q; ++jj) {
         const int j = j0 + jj;
-        const int s = SLOT_CT ? jj % NS : q % NS;
-        const uint32_t phase = SLOT_CT ? ((q0 / NS + jj / NS) & 1) : ((q / NS) & 1);
-        if (ok) ok = mbar_wait(&full[s], phase, err);
+        if (j >= PL) break;
+        if (ok) ok = ring.wait();
         if (ok) {
-          const T* sl = slots + s * slot_elems;
-          const int QN = jj % Q;  // slot of the newest plane
+          const T* sl = slots + ring.slot * slot_elems;
+          const int QN = jj;  // queue slot of the newest plane
           // 1. centre values of plane j
 #pragma unroll
           for (int f = 0; f < 3; ++f)
@@ -180,93 +164,113 @@ __global__ void __launch_bounds__(512) k_advect_zq(const __grid_constant__ Advec
             for (int i = 0; i < CPT; ++i) qv[f][QN][i] = sl[f * field_elems + (G + cy[i]) * nx + cx[i]];
           // 2. finish output plane k = j - 2G (queue slot of plane k + d - G: (jj - 2G + d) mod Q)
           if (j >= 2 * G) {
-            const int k = j - 2 * G;
             const int QC = (jj + 3 * Q - G) % Q;       // centre (load j - G)
             const int QM1 = (jj + 3 * Q - G - 1) % Q;  // plane k - 1
             const int QP1 = (jj + 3 * Q - G + 1) % Q;  // plane k + 1
             const int QM2 = (jj + 3 * Q - G - 2) % Q;  // plane k - 2 (G = 2)
             const int QP2 = (jj + 3 * Q - G + 2) % Q;  // plane k + 2 (G = 2)
-            const int PS = jj % G;                      // partial of load j - G
 #pragma unroll
             for (int i = 0; i < CPT; ++i) {
-              const size_t o = gidx(cx[i], y0 + cy[i], z0 + k, nx, ny);
               const T ww = qv[2][QC][i] + uinf[2];
               T outv[3];
+              if constexpr (UP) {
+                const UpW<T> wz = up_weights(ww, facA, facD);
+                const T cz = (T)3 * wz.far - (T)2 * facD;
 #pragma unroll
-              for (int f = 0; f < 3; ++f) {
-                const T f0 = qv[f][QC][i];
-                T dz;
-                if constexpr (SCHEME == 0) {
-                  dz = qv[f][QP1][i] - qv[f][QM1][i];
-                } else {
-                  dz = up3(ww, qv[f][QM2][i], qv[f][QM1][i], f0, qv[f][QP1][i], qv[f][QP2][i]);
+                for (int f = 0; f < 3; ++f) {
+                  const T f0 = qv[f][QC][i];
+                  const T far = wz.pos ? qv[f][QM2][i] : qv[f][QP2][i];
+                  T acc = part[f][i] + wz.far * far;
+                  acc += wz.m1 * qv[f][QM1][i];
+                  acc += wz.p1 * qv[f][QP1][i];
+                  acc += cz * f0;
+                  outv[f] = f0 + acc;
                 }
-                const T lz = qv[f][QM1][i] + qv[f][QP1][i];
-                outv[f] = f0 + part[f][PS][i] + facA * (ww * dz) + facD * (lz - f0 * 6);
+              } else {
+#pragma unroll
+                for (int f = 0; f < 3; ++f) {
+                  const T f0 = qv[f][QC][i];
+                  const T dz = qv[f][QP1][i] - qv[f][QM1][i];
+                  const T lz = qv[f][QM1][i] + qv[f][QP1][i];
+                  outv[f] = f0 + part[f][i] + facA * (ww * dz) + facD * (lz - f0 * 6);
+                }
               }
               if constexpr (BASE) {
-                const T* bs = sl + stencil_elems + cy[i] * nx + cx[i];
-                ou[o] = (T)0.5 * (bs[0] + outv[0]);
-                ov[o] = (T)0.5 * (bs[TY * nx] + outv[1]);
-                ow[o] = (T)0.5 * (bs[2 * TY * nx] + outv[2]);
-              } else {
-                ou[o] = outv[0];
-                ov[o] = outv[1];
-                ow[o] = outv[2];
+#pragma unroll
+                for (int f = 0; f < 3; ++f) outv[f] = (T)0.5 * (base[f][i] + outv[f]);
               }
+              ou[o[i]] = outv[0];
+              ov[o[i]] = outv[1];
+              ow[o[i]] = outv[2];
+              o[i] += (size_t)nx * ny;
             }
           }
-          // 3. x/y partial of plane j (output plane j - G), into slot j % G
-          if (j >= G && j < G + zc) {
-            const int PS = jj % G;
+          // 3. x/y partial of plane j - G + 1 (output plane j - 2G + 1)
+          if (j >= 2 * G - 1 && j < PL - 1) {
+            const T* sp = slots + ring.slot_back(G - 1) * slot_elems;
+            const int QX = (jj + 3 * Q - G + 1) % Q;
+            if constexpr (UP) {
+              const int x = cx[0], r = G + cy[0];
+              const int xm1 = (x - 1) & mask, xp1 = (x + 1) & mask, xm2 = (x - 2) & mask, xp2 = (x + 2) & mask;
+              UpW<T> wx[CPT], wy[CPT];
+              T cxy[CPT];
+              int xfar[CPT];
 #pragma unroll
-            for (int i = 0; i < CPT; ++i) {
-              const T uu = qv[0][QN][i] + uinf[0], vv = qv[1][QN][i] + uinf[1];
-              const int x = cx[i], r = G + cy[i];
+              for (int i = 0; i < CPT; ++i) {
+                wx[i] = up_weights(qv[0][QX][i] + uinf[0], facA, facD);
+                wy[i] = up_weights(qv[1][QX][i] + uinf[1], facA, facD);
+                cxy[i] = (T)3 * (wx[i].far + wy[i].far) - (T)4 * facD;
+                xfar[i] = wx[i].pos ? xm2 : xp2;
+              }
 #pragma unroll
               for (int f = 0; f < 3; ++f) {
-                const T* F = sl + f * field_elems;
-                const T f0 = qv[f][QN][i];
-                const T xm1 = F[r * nx + ((x - 1) & mask)], xp1 = F[r * nx + ((x + 1) & mask)];
-                const T ym1 = F[(r - 1) * nx + x], yp1 = F[(r + 1) * nx + x];
-                T dx, dy;
-                if constexpr (SCHEME == 0) {
-                  dx = xp1 - xm1;
-                  dy = yp1 - ym1;
-                } else {
-                  const T xm2 = F[r * nx + ((x - 2) & mask)], xp2 = F[r * nx + ((x + 2) & mask)];
-                  const T ym2 = F[(r - 2) * nx + x], yp2 = F[(r + 2) * nx + x];
-                  dx = up3(uu, xm2, xm1, f0, xp1, xp2);
-                  dy = up3(vv, ym2, ym1, f0, yp1, yp2);
+                const T* F = sp + f * field_elems + r * nx;
+                // rows r - 2 .. r + CPT + 1 of this x (the thread's own rows from the queue)
+                T row[CPT + 2 * G];
+#pragma unroll
+                for (int d = 0; d < CPT + 2 * G; ++d)
+                  row[d] = d >= G && d < G + CPT ? qv[f][QX][d - G] : F[(d - G) * nx + x];
+#pragma unroll
+                for (int i = 0; i < CPT; ++i) {
+                  const T* Fx = F + i * nx;
+                  T acc = cxy[i] * row[G + i] + wx[i].far * Fx[xfar[i]];
+                  acc += wx[i].m1 * Fx[xm1];
+                  acc += wx[i].p1 * Fx[xp1];
+                  acc += wy[i].far * (wy[i].pos ? row[i] : row[i + 4]);
+                  acc += wy[i].m1 * row[i + 1];
+                  acc += wy[i].p1 * row[i + 3];
+                  part[f][i] = acc;
                 }
-                part[f][PS][i] = facA * (uu * dx + vv * dy) + facD * (yp1 + ym1 + xp1 + xm1);
               }
+            } else {
+#pragma unroll
+              for (int i = 0; i < CPT; ++i) {
+                const T uu = qv[0][QX][i] + uinf[0], vv = qv[1][QX][i] + uinf[1];
+                const int x = cx[i], r = G + cy[i];
+#pragma unroll
+                for (int f = 0; f < 3; ++f) {
+                  const T* F = sp + f * field_elems;
+                  const T xm1 = F[r * nx + ((x - 1) & mask)], xp1 = F[r * nx + ((x + 1) & mask)];
+                  const T ym1 = F[(r - 1) * nx + x], yp1 = F[(r + 1) * nx + x];
+                  part[f][i] = facA * (uu * (xp1 - xm1) + vv * (yp1 - ym1)) + facD * (yp1 + ym1 + xp1 + xm1);
+                }
+              }
+            }
+            if constexpr (BASE) {
+              // u^n of output plane j - 2G + 1, finished by the next plane
+#pragma unroll
+              for (int i = 0; i < CPT; ++i)
+#pragma unroll
+                for (int f = 0; f < 3; ++f) base[f][i] = __ldg(bsrc[f] + o[i]);
             }
           }
         }
-        // rings of 4+ slots: one block barrier per two planes (slots of loads
-        // q-1 and q fully consumed, refill both; PL is even, so a pair never
-        // straddles items); shallower rings keep one barrier per plane
-        if constexpr (NS >= 4) {
-          if (q & 1) {
-            __syncthreads();
-            if (tid == 0 && ok)
-              for (int r = q - 1 + NS; r <= q + NS && r < L; ++r)
-                if (r == q_issued) issue(q_issued++);
-          }
-        } else {
-          __syncthreads();  // slot s fully consumed
-          if (tid == 0 && ok && q_issued < L && q_issued == q + NS) issue(q_issued++);
-        }
-        ++q;
+        ring.step(ok, ring.n & 1, j, PL, pos, nextp, more, issue);
       }
     }
+    pos = nextp;
   }
-  if (!ok && tid == 0) {
-    // bounded drain of this CTA's loads still in flight (at most the last NS issued)
-    for (int r = q_issued - NS < 0 ? 0 : q_issued - NS; r < q_issued; ++r)
-      mbar_wait(&full[r % NS], (r / NS) & 1, nullptr);
-  }
+  ring.drain(ok);
 }
 
 }  // namespace cup

@@ -971,6 +971,15 @@ int make_map(cup_handle* H, CUtensorMap* m, const void* base, CUtensorMapDataTyp
   return CUP_OK;
 }
 
+// The boxes of a field's TY tile rows with G halo rows (RowMaps).
+template <typename T>
+int make_row_maps(cup_handle* H, RowMaps* m, const void* base, int TY, int G) {
+  int rc = make_map(H, &m->all, base, tma_dtype<T>(), sizeof(T), H->nx, TY + 2 * G, 1);
+  if (!rc) rc = make_map(H, &m->main, base, tma_dtype<T>(), sizeof(T), H->nx, TY, 1);
+  if (!rc) rc = make_map(H, &m->halo, base, tma_dtype<T>(), sizeof(T), H->nx, G, 1);
+  return rc;
+}
+
 template <class K>
 int prepare_kernel(cup_handle* H, K kern, size_t smem, int threads, int* blocks_per_sm) {
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1000,25 +1009,11 @@ void klaunch(cup_handle* H, void (*kern)(KArgs...), dim3 grid, dim3 block, size_
   cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
-// Launches k_stencil_stream over `fields` (device arrays of T). Returns the
-// grid size through *grid_out (the number of per-CTA partials written).
-template <typename T, int NF, int G, int TY, int NS, class Op>
-int launch_stream(cup_handle* H, const char* name, const void* const* fields, const Op& op, int* grid_out = nullptr,
-                  const int* skip = nullptr) {
-  FieldMaps<NF> maps;
-  for (int f = 0; f < NF; ++f) {
-    int rc = make_map(H, &maps.main[f], fields[f], tma_dtype<T>(), sizeof(T), H->nx, TY, 1);
-    if (rc) return rc;
-    rc = make_map(H, &maps.halo[f], fields[f], tma_dtype<T>(), sizeof(T), H->nx, G, 1);
-    if (rc) return rc;
-  }
-  const size_t smem = stream_smem_bytes<T, NF, G, TY, NS>(H->nx) + 128;
-  auto kern = k_stencil_stream<T, NF, G, TY, NS, Op>;
-  int bpsm = 0;
-  int rc = prepare_kernel(H, kern, smem, 256, &bpsm);
-  if (rc) return rc;
-  // planes per work item (16, 8 or 4): the fewest plane loads on the busiest
-  // CTA, waves of items times the planes an item loads (its 2G halo planes too)
+// Planes per work item (16, 8 or 4): the fewest plane loads on the busiest CTA,
+// waves of items times the planes an item loads (its 2G halo planes too), so
+// that a small grid spreads over the SMs. (At 64^3 the FP64 upwind3 stages had
+// run 64 items of 20 planes on 148 SMs.)
+int planes_per_item(const cup_handle* H, int TY, int G, int bpsm) {
   int zc = std::min(16, H->nz);
   long long best = -1;
   for (int c = std::min(16, H->nz); c >= 4; c /= 2) {
@@ -1027,6 +1022,25 @@ int launch_stream(cup_handle* H, const char* name, const void* const* fields, co
     const long long cost = (items + resident - 1) / resident * (c + 2 * G);
     if (best < 0 || cost < best) best = cost, zc = c;
   }
+  return zc;
+}
+
+// Launches k_stencil_stream over `fields` (device arrays of T). Returns the
+// grid size through *grid_out (the number of per-CTA partials written).
+template <typename T, int NF, int G, int TY, int NS, class Op>
+int launch_stream(cup_handle* H, const char* name, const void* const* fields, const Op& op, int* grid_out = nullptr,
+                  const int* skip = nullptr) {
+  FieldMaps<NF> maps;
+  for (int f = 0; f < NF; ++f) {
+    int rc = make_row_maps<T>(H, &maps.f[f], fields[f], TY, G);
+    if (rc) return rc;
+  }
+  const size_t smem = stream_smem_bytes<T, NF, G, TY, NS>(H->nx) + 128;
+  auto kern = k_stencil_stream<T, NF, G, TY, NS, Op>;
+  int bpsm = 0;
+  int rc = prepare_kernel(H, kern, smem, 256, &bpsm);
+  if (rc) return rc;
+  const int zc = planes_per_item(H, TY, G, bpsm);
   StreamGeom g{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
   const int grid = std::min(g.n_items, bpsm * H->num_sms);
   if (grid > kPartialCap / 16) return fail(H, CUP_ERR_ARG, "too many CTAs for the partial buffers");
@@ -1329,8 +1343,11 @@ int read_state(cup_handle* H) {
 
 // ---- typed pipeline pieces -------------------------------------------------
 // Launches one k_advect_zq pass: fields `in` (stencil), `base` (stage-2
-// point-wise u^n, else unused), output `out`.
-template <typename T, int SCHEME, int TY, int NS, int CPT, int NXC, int ZCC>
+// point-wise u^n, else unused), output `out`. Grids of nx 64, 128 or 256 take
+// the compile-time-nx kernels; other shapes the same kernel with runtime sizes.
+// (The planes per item stay a runtime count: unrolling a whole 20-plane item
+// measured slower for the FP64 stages than the 10-plane loop.)
+template <typename T, int SCHEME, int TY, int NS, int CPT, int NXC>
 int launch_advect_sized(cup_handle* H, const char* name, void* const* in, void* const* base, void* const* out,
                         DtArg dt) {
   constexpr int G = AdvectTraits<SCHEME>::G;
@@ -1339,74 +1356,63 @@ int launch_advect_sized(cup_handle* H, const char* name, void* const* in, void* 
     return fail(H, CUP_ERR_ARG, "advection tile does not fit the grid");
   AdvectMaps maps;
   for (int f = 0; f < 3; ++f) {
-    int rc = make_map(H, &maps.main[f], in[f], tma_dtype<T>(), sizeof(T), H->nx, TY, 1);
-    if (!rc) rc = make_map(H, &maps.halo[f], in[f], tma_dtype<T>(), sizeof(T), H->nx, G, 1);
-    if (!rc) rc = make_map(H, &maps.base[f], AdvectTraits<SCHEME>::BASE ? base[f] : in[f], tma_dtype<T>(), sizeof(T),
-                           H->nx, TY, 1);
+    int rc = make_row_maps<T>(H, &maps.f[f], in[f], TY, G);
     if (rc) return rc;
+    maps.base[f] = maps.f[f].main;
   }
-  const int zc = std::min(16, H->nz);
-  if ((NXC && NXC != H->nx) || (ZCC && ZCC != zc)) return fail(H, CUP_ERR_ARG, "advection specialisation mismatch");
-  StreamGeom g{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
-  const size_t smem = advect_smem_bytes<T, SCHEME, TY, NS, CPT>(H->nx) + 128;
-  auto kern = k_advect_zq<T, SCHEME, TY, NS, CPT, NXC, ZCC>;
+  if (NXC && NXC != H->nx) return fail(H, CUP_ERR_ARG, "advection specialisation mismatch");
+  const size_t smem = advect_smem_bytes<T, SCHEME, TY, NS>(H->nx) + 128;
+  auto kern = k_advect_zq<T, SCHEME, TY, NS, CPT, NXC>;
   const int threads = cells / CPT;
   int bpsm = 0;
   int rc = prepare_kernel(H, kern, smem, threads, &bpsm);
   if (rc) return rc;
+  const int zc = planes_per_item(H, TY, G, bpsm);
+  StreamGeom g{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
   const int grid = std::min(g.n_items, bpsm * H->num_sms);
   return launch_named(H, name, [&]() -> int {
-    klaunch(H, kern, grid, threads, smem, maps, g, (T*)out[0], (T*)out[1], (T*)out[2], dt, H->h, H->cfg.nu,
-                                             H->uinf[0], H->uinf[1], H->uinf[2], H->derr);
+    klaunch(H, kern, grid, threads, smem, maps, g, (const T*)base[0], (const T*)base[1], (const T*)base[2], (T*)out[0],
+            (T*)out[1], (T*)out[2], dt, H->h, H->cfg.nu, H->uinf[0], H->uinf[1], H->uinf[2], H->derr);
     CKL();
     return CUP_OK;
   });
 }
 
-// Grids of nx 64, 128 or 256 take the compile-time-nx kernels; other
-// shapes the same kernel with runtime sizes. (The planes per item stay a
-// runtime count here: unrolling a whole 20-plane item measured slower for
-// the FP64 stages than the 10-plane loop.)
 template <typename T, int SCHEME, int TY, int NS, int CPT>
 int launch_advect(cup_handle* H, const char* name, void* const* in, void* const* base, void* const* out, DtArg dt) {
   switch (H->nx) {
-    case 64: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 64, 0>(H, name, in, base, out, dt);
-    case 128: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 128, 0>(H, name, in, base, out, dt);
-    case 256: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 256, 0>(H, name, in, base, out, dt);
+    case 64: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 64>(H, name, in, base, out, dt);
+    case 128: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 128>(H, name, in, base, out, dt);
+    case 256: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 256>(H, name, in, base, out, dt);
     default: break;
   }
-  return launch_advect_sized<T, SCHEME, TY, NS, CPT, 0, 0>(H, name, in, base, out, dt);
+  return launch_advect_sized<T, SCHEME, TY, NS, CPT, 0>(H, name, in, base, out, dt);
 }
 
 // Launches one packed-FP32 upwind3 stage (k_advect_zq_f2): `in` stencil
 // fields, `base` the stage-2 point-wise u^n, `out` the result.
-// zmax: z planes per work item (at most; nz when smaller): a tall tile (TY 8)
-// uses 8 so that the items spread evenly over the SMs.
-// NXC, ZCC: compile-time nx and planes per item (0: runtime); the caller
-// picks them only when they equal H->nx and min(zmax, nz).
-template <bool STAGE2, int TY, int NS, int PPT, int NXC = 0, int ZCC = 0>
-int launch_advect_f2(cup_handle* H, const char* name, void* const* in, void* const* base, void* const* out, DtArg dt,
-                     int zmax = 16) {
+// NXC: compile-time nx (0: runtime).
+template <bool STAGE2, int TY, int NS, int PPT, int NXC = 0>
+int launch_advect_f2(cup_handle* H, const char* name, void* const* in, void* const* base, void* const* out, DtArg dt) {
   constexpr int G = 2;
   const int pairs = TY * H->nx / 2;
   if (pairs % PPT || pairs / PPT > 512 || H->ny % TY) return fail(H, CUP_ERR_ARG, "advection tile does not fit the grid");
   AdvectMaps maps;
   for (int f = 0; f < 3; ++f) {
-    int rc = make_map(H, &maps.main[f], in[f], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), H->nx, TY, 1);
-    if (!rc) rc = make_map(H, &maps.halo[f], in[f], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), H->nx, G, 1);
+    int rc = make_row_maps<float>(H, &maps.f[f], in[f], TY, G);
     if (!rc) rc = make_map(H, &maps.base[f], STAGE2 ? base[f] : in[f], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float),
                            H->nx, TY, 1);
     if (rc) return rc;
   }
-  const int zc = std::min(zmax, H->nz);
-  if ((NXC && NXC != H->nx) || (ZCC && ZCC != zc)) return fail(H, CUP_ERR_ARG, "advection specialisation mismatch");
-  StreamGeom g{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
-  const size_t smem = advect_smem_bytes<float, STAGE2 ? 2 : 1, TY, NS, 1>(H->nx) + 128;
-  auto kern = k_advect_zq_f2<STAGE2, TY, NS, PPT, NXC, ZCC>;
+  if (NXC && NXC != H->nx) return fail(H, CUP_ERR_ARG, "advection specialisation mismatch");
+  const size_t smem = advect_f2_smem_bytes<STAGE2, TY, NS>(H->nx) + 128;
+  auto kern = k_advect_zq_f2<STAGE2, TY, NS, PPT, NXC>;
   const int threads = pairs / PPT;
   int bpsm = 0;
   int rc = prepare_kernel(H, kern, smem, threads, &bpsm);
   if (rc) return rc;
+  const int zc = planes_per_item(H, TY, G, bpsm);
+  StreamGeom g{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
   const int grid = std::min(g.n_items, bpsm * H->num_sms);
   return launch_named(H, name, [&]() -> int {
     klaunch(H, kern, grid, threads, smem, maps, g, (float*)out[0], (float*)out[1], (float*)out[2], dt, H->h,
@@ -1417,32 +1423,26 @@ int launch_advect_f2(cup_handle* H, const char* name, void* const* in, void* con
 }
 
 // FP32 upwind3 stages: packed FP32x2 kernels (shared by the forward step and
-// the adjoint's stage recompute, so both see the same u1). Tile height, ring
-// depth and pairs per thread as measured best at 256^3: stage 1 (TY 8, NS 4,
-// 2 pairs, 8-plane items) about 100 us, stage 2 (TY 4, NS 4, 1 pair, 16-plane
-// items) about 129 us; rings of 6 and 5 slots measured the same.
-// Grids of nx 64, 128 or 256 with nz >= ZC take the compile-time-size
-// kernels; other shapes the same kernel with runtime sizes.
-template <bool STAGE2, int TY, int NS, int PPT, int ZC>
+// the adjoint's stage recompute, so both see the same u1). Grids of nx 64, 128
+// or 256 take the compile-time-nx kernels; other shapes the same kernel with
+// runtime sizes.
+template <bool STAGE2, int TY, int NS, int PPT>
 int launch_advect_f2_sized(cup_handle* H, const char* name, void* const* in, void* const* base, void* const* out,
                            DtArg dt) {
-  if (H->nz >= ZC) {
-    switch (H->nx) {
-      case 64: return launch_advect_f2<STAGE2, TY, NS, PPT, 64, ZC>(H, name, in, base, out, dt, ZC);
-      case 128: return launch_advect_f2<STAGE2, TY, NS, PPT, 128, ZC>(H, name, in, base, out, dt, ZC);
-      case 256: return launch_advect_f2<STAGE2, TY, NS, PPT, 256, ZC>(H, name, in, base, out, dt, ZC);
-      default: break;
-    }
+  switch (H->nx) {
+    case 64: return launch_advect_f2<STAGE2, TY, NS, PPT, 64>(H, name, in, base, out, dt);
+    case 128: return launch_advect_f2<STAGE2, TY, NS, PPT, 128>(H, name, in, base, out, dt);
+    case 256: return launch_advect_f2<STAGE2, TY, NS, PPT, 256>(H, name, in, base, out, dt);
+    default: break;
   }
-  return launch_advect_f2<STAGE2, TY, NS, PPT>(H, name, in, base, out, dt, ZC);
+  return launch_advect_f2<STAGE2, TY, NS, PPT>(H, name, in, base, out, dt);
 }
 int upwind_stage1_f32(cup_handle* H, const char* name, void* const* in, void* const* out, DtArg dt) {
-  if (H->ny % 8 == 0 && 4 * H->nx <= 512 * 2) return launch_advect_f2_sized<false, 8, 4, 2, 8>(H, name, in, in, out, dt);
-  return launch_advect_f2<false, 4, 4, 1>(H, name, in, in, out, dt);
+  return launch_advect_f2_sized<false, 8, 6, 2>(H, name, in, in, out, dt);
 }
 int upwind_stage2_f32(cup_handle* H, const char* name, void* const* in, void* const* base, void* const* out,
                       DtArg dt) {
-  return launch_advect_f2_sized<true, 4, 4, 1, 16>(H, name, in, base, out, dt);
+  return launch_advect_f2_sized<true, 4, 6, 1>(H, name, in, base, out, dt);
 }
 
 template <typename T>
@@ -1463,8 +1463,8 @@ int do_advect_diffuse(cup_handle* H, DtArg dt) {
       if ((rc = upwind_stage1_f32(H, "upwind3_stage1", uvw, st1, dt))) return rc;
       rc = upwind_stage2_f32(H, "upwind3_stage2", st1, uvw, tmp, dt);
     } else {
-      if ((rc = launch_advect<T, 1, 4, 3, 2>(H, "upwind3_stage1", uvw, uvw, st1, dt))) return rc;
-      rc = launch_advect<T, 2, 2, 4, 1>(H, "upwind3_stage2", st1, uvw, tmp, dt);
+      if ((rc = launch_advect<T, 1, 4, 4, 2>(H, "upwind3_stage1", uvw, uvw, st1, dt))) return rc;
+      rc = launch_advect<T, 2, 4, 4, 2>(H, "upwind3_stage2", st1, uvw, tmp, dt);
     }
   }
   if (rc) return rc;
@@ -1554,29 +1554,28 @@ int dc_min_iter(const cup_handle* H) {
 }
 
 // Launches one k_pres_zq pass; returns the grid size (number of partials).
-template <typename T, int MODE, int TY, int NS, int CPT, int NXC, int ZCC, bool BD>
+template <typename T, int MODE, int TY, int NS, int CPT, int NXC, bool BD>
 int launch_pzq_sized(cup_handle* H, const char* name, double* pw, double* partials, const double* rmean, DtArg dt,
                      int* grid_out, const int* skip, int pred_order, double* pred_out, void* const* out) {
   const int cells = TY * H->nx;
   if (cells % CPT || cells / CPT > 512 || H->ny % TY)
     return fail(H, CUP_ERR_ARG, "pressure tile does not fit the grid");
   PzqMaps maps;
-  int rc = make_map(H, &maps.p_main, pw, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, sizeof(double), H->nx, TY, 1);
-  if (!rc) rc = make_map(H, &maps.p_halo, pw, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, sizeof(double), H->nx, 2, 1);
+  int rc = make_row_maps<double>(H, &maps.p, pw, TY, 2);
   if (!rc) rc = make_map(H, &maps.h_main, pred_order >= 1 ? H->p : pw, CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
                          sizeof(double), H->nx, TY, 1);
   const void* f[3] = {H->u, H->v, H->w};
   for (int q = 0; q < 3 && !rc; ++q) rc = make_map(H, &maps.f_main[q], f[q], tma_dtype<T>(), sizeof(T), H->nx, TY, 1);
-  if (!rc) rc = make_map(H, &maps.v_halo, H->v, tma_dtype<T>(), sizeof(T), H->nx, 1, 1);
+  if (!rc) rc = make_row_maps<T>(H, &maps.v, H->v, TY, 1);
   if (rc) return rc;
-  const int zc = ZCC ? ZCC : std::min(16, H->nz);
-  if ((NXC && NXC != H->nx) || (ZCC && ZCC != zc)) return fail(H, CUP_ERR_ARG, "pressure specialisation mismatch");
-  StreamGeom geo{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
+  if (NXC && NXC != H->nx) return fail(H, CUP_ERR_ARG, "pressure specialisation mismatch");
   const size_t smem = pzq_smem_bytes_host<T, MODE, TY, NS>(H->nx) + 128;
-  auto kern = k_pres_zq<T, MODE, TY, NS, CPT, NXC, ZCC, BD>;
+  auto kern = k_pres_zq<T, MODE, TY, NS, CPT, NXC, BD>;
   const int threads = cells / CPT;
   int bpsm = 0;
   if ((rc = prepare_kernel(H, kern, smem, threads, &bpsm))) return rc;
+  const int zc = planes_per_item(H, TY, 2, bpsm);
+  StreamGeom geo{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
   const int grid = std::min(geo.n_items, bpsm * H->num_sms);
   if (grid > kPartialCap / pzq_partials_per_cta<MODE>())
     return fail(H, CUP_ERR_ARG, "too many CTAs for the partial buffers");
@@ -1596,29 +1595,27 @@ int launch_pzq_sized(cup_handle* H, const char* name, double* pw, double* partia
   return CUP_OK;
 }
 
-// Grids of nx 64, 128 or 256 with nz >= ZC take the compile-time-size
-// kernels; other shapes the same kernel with runtime sizes. BD: b carries the
-// obstacle terms on the box (H->box_delta).
-template <typename T, int MODE, int TY, int NS, int CPT, int ZC = 16, bool BD = false>
+// Grids of nx 64, 128 or 256 take the compile-time-nx kernels; other shapes the
+// same kernel with runtime sizes. BD: b carries the obstacle terms on the box
+// (H->box_delta).
+template <typename T, int MODE, int TY, int NS, int CPT, bool BD = false>
 int launch_pzq(cup_handle* H, const char* name, double* pw, double* partials, const double* rmean, DtArg dt,
                int* grid_out, const int* skip, int pred_order = -1, double* pred_out = nullptr,
                void* const* out = nullptr) {
-  if (H->nz >= ZC) {
-    switch (H->nx) {
-      case 64:
-        return launch_pzq_sized<T, MODE, TY, NS, CPT, 64, ZC, BD>(H, name, pw, partials, rmean, dt, grid_out, skip,
-                                                              pred_order, pred_out, out);
-      case 128:
-        return launch_pzq_sized<T, MODE, TY, NS, CPT, 128, ZC, BD>(H, name, pw, partials, rmean, dt, grid_out, skip,
-                                                               pred_order, pred_out, out);
-      case 256:
-        return launch_pzq_sized<T, MODE, TY, NS, CPT, 256, ZC, BD>(H, name, pw, partials, rmean, dt, grid_out, skip,
-                                                               pred_order, pred_out, out);
-      default: break;
-    }
+  switch (H->nx) {
+    case 64:
+      return launch_pzq_sized<T, MODE, TY, NS, CPT, 64, BD>(H, name, pw, partials, rmean, dt, grid_out, skip, pred_order,
+                                                            pred_out, out);
+    case 128:
+      return launch_pzq_sized<T, MODE, TY, NS, CPT, 128, BD>(H, name, pw, partials, rmean, dt, grid_out, skip,
+                                                             pred_order, pred_out, out);
+    case 256:
+      return launch_pzq_sized<T, MODE, TY, NS, CPT, 256, BD>(H, name, pw, partials, rmean, dt, grid_out, skip,
+                                                             pred_order, pred_out, out);
+    default: break;
   }
-  return launch_pzq_sized<T, MODE, TY, NS, CPT, 0, 0, BD>(H, name, pw, partials, rmean, dt, grid_out, skip, pred_order,
-                                                      pred_out, out);
+  return launch_pzq_sized<T, MODE, TY, NS, CPT, 0, BD>(H, name, pw, partials, rmean, dt, grid_out, skip, pred_order,
+                                                       pred_out, out);
 }
 
 int launch_finalize_residual(cup_handle* H, const double* partials, int stride, int grid, int k) {
@@ -1654,10 +1651,10 @@ int do_pressure_dc_zq(cup_handle* H, DtArg dt) {
   if (!H->pred_ready) CK(cudaMemcpyAsync(W, H->p, H->n * sizeof(double), cudaMemcpyDeviceToDevice, H->stream));
   int rc, grid = 0;
   if (box)
-    rc = launch_pzq<T, PZQ_RHS_RES, 4, 4, 2, 16, true>(H, "rhs_residual", W, partial(H, P_RES), nullptr, dt,
+    rc = launch_pzq<T, PZQ_RHS_RES, 4, 6, 2, true>(H, "rhs_residual", W, partial(H, P_RES), nullptr, dt,
                                                              &grid, nullptr);
   else
-    rc = launch_pzq<T, PZQ_RHS_RES, 4, 4, 2>(H, "rhs_residual", W, partial(H, P_RES), nullptr, dt, &grid,
+    rc = launch_pzq<T, PZQ_RHS_RES, 4, 6, 2>(H, "rhs_residual", W, partial(H, P_RES), nullptr, dt, &grid,
                                                    nullptr);
   if (rc) return rc;
   if ((rc = launch_finalize_residual(H, partial(H, P_RES), 18, grid, 0))) return rc;
@@ -1667,10 +1664,10 @@ int do_pressure_dc_zq(cup_handle* H, DtArg dt) {
   for (int k = 1; k <= max_iter; ++k) {
     if (k > 1) {
       if (box)
-        rc = launch_pzq<T, PZQ_RES, 4, 4, 2, 16, true>(H, "dc_residual", W, partial(H, P_RES),
+        rc = launch_pzq<T, PZQ_RES, 4, 6, 2, true>(H, "dc_residual", W, partial(H, P_RES),
                                                              H->dstate->rmean, dt, &grid, conv);
       else
-        rc = launch_pzq<T, PZQ_RES, 4, 4, 2>(H, "dc_residual", W, partial(H, P_RES), H->dstate->rmean, dt, &grid,
+        rc = launch_pzq<T, PZQ_RES, 4, 6, 2>(H, "dc_residual", W, partial(H, P_RES), H->dstate->rmean, dt, &grid,
                                                    conv);
       if (rc) return rc;
     }
@@ -1678,11 +1675,11 @@ int do_pressure_dc_zq(cup_handle* H, DtArg dt) {
     const int* skip = k > 1 ? conv : nullptr;
     const int pred = k == 1 ? order : -1;
     if (box)
-      rc = launch_pzq<T, PZQ_GRAD_CHECK_BOX, 4, 4, 2, 8, true>(H, "grad_p_check", W, partial(H, P_GRAD),
+      rc = launch_pzq<T, PZQ_GRAD_CHECK_BOX, 4, 4, 2, true>(H, "grad_p_check", W, partial(H, P_GRAD),
                                                                      H->dstate->rmean, dt, &H->n_grad_partials, skip,
                                                                      pred, H->p_old, unew);
     else
-      rc = launch_pzq<T, PZQ_GRAD_CHECK, 4, 4, 2, 8>(H, "grad_p_check", W, partial(H, P_GRAD), H->dstate->rmean, dt,
+      rc = launch_pzq<T, PZQ_GRAD_CHECK, 4, 4, 2>(H, "grad_p_check", W, partial(H, P_GRAD), H->dstate->rmean, dt,
                                                         &H->n_grad_partials, skip, pred, H->p_old, unew);
     if (rc) return rc;
     if ((rc = launch_finalize_residual(H, partial(H, P_GRAD), kGradStride, H->n_grad_partials, k))) return rc;
@@ -2096,23 +2093,20 @@ int do_step(cup_handle* H, DtArg dt, const double* lambda_dev, int advance, int 
     if (dt.dev) return fail(H, CUP_ERR_STATE, "spectral forcing needs the step's dt on the host");
     if ((rc = do_spectral_forcing<T>(H, dt.host))) return rc;
   }
-  if (H->has_sphere && H->fp32) {
-    // the obstacle terms need global sums over the RHS first: they are formed
-    // on the sphere's box and added back by the z-queue defect correction's
-    // passes, which recompute the rest of b from u*
-    if ((rc = do_box_rhs_terms<T>(H, dt))) return rc;
-    if ((rc = do_pressure_dc_zq<T>(H, dt))) return rc;
-  } else if (H->has_sphere) {
-    if ((rc = do_pressure_rhs<T>(H, dt))) return rc;
-    if ((rc = do_poisson(H))) return rc;
-  } else if (H->fp32) {
-    // RHS, defect correction and gradient correction in z-queue passes
+  if constexpr (std::is_same<T, float>::value) {
+    // RHS, defect correction and gradient correction in z-queue passes. The
+    // sphere's RHS terms need global sums over the RHS first: they are formed on
+    // its box and added back by the passes, which recompute the rest of b from u*
+    if (H->has_sphere && (rc = do_box_rhs_terms<T>(H, dt))) return rc;
     if ((rc = do_pressure_dc_zq<T>(H, dt))) return rc;
   } else {
-    void* us[3] = {H->u, H->v, H->w};
-    if ((rc = do_solve_rhs_of<T>(H, "rhs_dht_x", "dht_x", us, H->p, dt))) return rc;
-  }
-  if (!H->fp32) {
+    if (H->has_sphere) {
+      if ((rc = do_pressure_rhs<T>(H, dt))) return rc;
+      if ((rc = do_poisson(H))) return rc;
+    } else {
+      void* us[3] = {H->u, H->v, H->w};
+      if ((rc = do_solve_rhs_of<T>(H, "rhs_dht_x", "dht_x", us, H->p, dt))) return rc;
+    }
     if ((rc = do_grad<T>(H, dt))) return rc;
   }
   // UpdateObstacles: the free dofs' velocities from the pre-penalization flow
@@ -2143,24 +2137,23 @@ int launch_adjoint(cup_handle* H, const char* name, const void* const* f, const 
     return fail(H, CUP_ERR_ARG, "adjoint tile does not fit the grid");
   AdjointMaps maps;
   for (int q = 0; q < 3; ++q) {
-    int rc = make_map(H, &maps.main[q], f[q], tma_dtype<T>(), sizeof(T), H->nx, TY, 1);
-    if (!rc) rc = make_map(H, &maps.halo[q], f[q], tma_dtype<T>(), sizeof(T), H->nx, G, 1);
-    if (!rc) rc = make_map(H, &maps.main[3 + q], g[q], tma_dtype<T>(), sizeof(T), H->nx, TY, 1);
-    if (!rc) rc = make_map(H, &maps.halo[3 + q], g[q], tma_dtype<T>(), sizeof(T), H->nx, G, 1);
-    if (!rc) rc = make_map(H, &maps.lam[q], LAM ? lam[q] : g[q], tma_dtype<T>(), sizeof(T), H->nx, TY, 1);
+    int rc = make_row_maps<T>(H, &maps.f[q], f[q], TY, G);
+    if (!rc) rc = make_row_maps<T>(H, &maps.f[3 + q], g[q], TY, G);
     if (rc) return rc;
   }
-  const int zc = std::min(16, H->nz);
-  StreamGeom geo{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
-  const size_t smem = adjoint_smem_bytes<T, SCHEME, LAM, TY, NS, CPT>(H->nx) + 128;
+  const size_t smem = adjoint_smem_bytes<T, SCHEME, TY, NS>(H->nx) + 128;
   auto kern = k_adjoint_zq<T, SCHEME, LAM, TY, NS, CPT>;
   const int threads = cells / CPT;
   int bpsm = 0;
   int rc = prepare_kernel(H, kern, smem, threads, &bpsm);
   if (rc) return rc;
+  const int zc = planes_per_item(H, TY, G, bpsm);
+  StreamGeom geo{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
   const int grid = std::min(geo.n_items, bpsm * H->num_sms);
+  const void* lm[3] = {LAM ? lam[0] : nullptr, LAM ? lam[1] : nullptr, LAM ? lam[2] : nullptr};
   return launch_named(H, name, [&]() -> int {
-    klaunch(H, kern, grid, threads, smem, maps, geo, (T*)out[0], (T*)out[1], (T*)out[2], (T)alpha, (T)beta, dt, H->h,
+    klaunch(H, kern, grid, threads, smem, maps, geo, (const T*)lm[0], (const T*)lm[1], (const T*)lm[2], (T*)out[0],
+            (T*)out[1], (T*)out[2], (T)alpha, (T)beta, dt, H->h,
                                              H->cfg.nu, H->uinf[0], H->uinf[1], H->uinf[2], H->derr);
     CKL();
     return CUP_OK;
@@ -2195,54 +2188,50 @@ int do_project_fields(cup_handle* H, void* const* in, void* const* out, double* 
 //                   mu = 1/2 S'(u1)^T lam*,  lam = 1/2 lam* + S'(un)^T mu
 //   central + Euler: lam = S'(un)^T (P lam)
 // FP32 upwind3 stage transposes on x-pairs (k_adjoint_zq_f2); grids of nx 64,
-// 128 or 256 with nz >= ZC take the compile-time-size kernels.
-template <bool LAM, int TY, int NS, int PPT, int NXC = 0, int ZCC = 0>
+// 128 or 256 take the compile-time-nx kernels.
+template <bool LAM, int TY, int NS, int PPT, int NXC = 0>
 int launch_adjoint_f2(cup_handle* H, const char* name, const void* const* f, const void* const* g,
-                      const void* const* lam, void* const* out, double alpha, double beta, DtArg dt, int zmax) {
+                      const void* const* lam, void* const* out, double alpha, double beta, DtArg dt) {
   constexpr int G = 2;
   const int pairs = TY * H->nx / 2;
   if (pairs % PPT || pairs / PPT > 512 || H->ny % TY)
     return fail(H, CUP_ERR_ARG, "adjoint tile does not fit the grid");
   AdjointMaps maps;
   for (int q = 0; q < 3; ++q) {
-    int rc = make_map(H, &maps.main[q], f[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), H->nx, TY, 1);
-    if (!rc) rc = make_map(H, &maps.halo[q], f[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), H->nx, G, 1);
-    if (!rc) rc = make_map(H, &maps.main[3 + q], g[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), H->nx, TY, 1);
-    if (!rc) rc = make_map(H, &maps.halo[3 + q], g[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), H->nx, G, 1);
-    if (!rc)
-      rc = make_map(H, &maps.lam[q], LAM ? lam[q] : g[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float), H->nx, TY, 1);
+    int rc = make_row_maps<float>(H, &maps.f[q], f[q], TY, G);
+    if (!rc) rc = make_row_maps<float>(H, &maps.f[3 + q], g[q], TY, G);
     if (rc) return rc;
   }
-  const int zc = std::min(zmax, H->nz);
-  if ((NXC && NXC != H->nx) || (ZCC && ZCC != zc)) return fail(H, CUP_ERR_ARG, "adjoint specialisation mismatch");
-  StreamGeom geo{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
-  const size_t smem = adjoint_f2_smem_bytes<LAM, TY, NS, PPT>(H->nx) + 128;
-  auto kern = k_adjoint_zq_f2<LAM, TY, NS, PPT, NXC, ZCC>;
+  if (NXC && NXC != H->nx) return fail(H, CUP_ERR_ARG, "adjoint specialisation mismatch");
+  const size_t smem = adjoint_f2_smem_bytes<TY, NS>(H->nx) + 128;
+  auto kern = k_adjoint_zq_f2<LAM, TY, NS, PPT, NXC>;
   const int threads = pairs / PPT;
   int bpsm = 0;
   int rc = prepare_kernel(H, kern, smem, threads, &bpsm);
   if (rc) return rc;
+  const int zc = planes_per_item(H, TY, G, bpsm);
+  StreamGeom geo{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
   const int grid = std::min(geo.n_items, bpsm * H->num_sms);
+  const void* lm[3] = {LAM ? lam[0] : nullptr, LAM ? lam[1] : nullptr, LAM ? lam[2] : nullptr};
   return launch_named(H, name, [&]() -> int {
-    klaunch(H, kern, grid, threads, smem, maps, geo, (float*)out[0], (float*)out[1], (float*)out[2], (float)alpha,
+    klaunch(H, kern, grid, threads, smem, maps, geo, (const float*)lm[0], (const float*)lm[1], (const float*)lm[2],
+            (float*)out[0], (float*)out[1], (float*)out[2], (float)alpha,
             (float)beta, dt, H->h, H->cfg.nu, H->uinf[0], H->uinf[1], H->uinf[2], H->derr);
     CKL();
     return CUP_OK;
   });
 }
 
-template <bool LAM, int TY, int NS, int PPT, int ZC>
+template <bool LAM, int TY, int NS, int PPT>
 int launch_adjoint_f2_sized(cup_handle* H, const char* name, const void* const* f, const void* const* g,
                             const void* const* lam, void* const* out, double alpha, double beta, DtArg dt) {
-  if (H->nz >= ZC) {
-    switch (H->nx) {
-      case 64: return launch_adjoint_f2<LAM, TY, NS, PPT, 64, ZC>(H, name, f, g, lam, out, alpha, beta, dt, ZC);
-      case 128: return launch_adjoint_f2<LAM, TY, NS, PPT, 128, ZC>(H, name, f, g, lam, out, alpha, beta, dt, ZC);
-      case 256: return launch_adjoint_f2<LAM, TY, NS, PPT, 256, ZC>(H, name, f, g, lam, out, alpha, beta, dt, ZC);
-      default: break;
-    }
+  switch (H->nx) {
+    case 64: return launch_adjoint_f2<LAM, TY, NS, PPT, 64>(H, name, f, g, lam, out, alpha, beta, dt);
+    case 128: return launch_adjoint_f2<LAM, TY, NS, PPT, 128>(H, name, f, g, lam, out, alpha, beta, dt);
+    case 256: return launch_adjoint_f2<LAM, TY, NS, PPT, 256>(H, name, f, g, lam, out, alpha, beta, dt);
+    default: break;
   }
-  return launch_adjoint_f2<LAM, TY, NS, PPT>(H, name, f, g, lam, out, alpha, beta, dt, ZC);
+  return launch_adjoint_f2<LAM, TY, NS, PPT>(H, name, f, g, lam, out, alpha, beta, dt);
 }
 
 // The two transposed upwind3 stages of an FP32 adjoint step: mu = 1/2 S'(u1)^T
@@ -2252,9 +2241,9 @@ int launch_adjoint_f2_sized(cup_handle* H, const char* name, const void* const* 
 // and a 4-deep ring, and 2.17 ms for the scalar kernels (k_adjoint_zq).
 int adjoint_upwind_f32(cup_handle* H, void* const* un, void* const* st1, void* const* lam, void* const* mu, DtArg dt) {
   int rc;
-  if ((rc = launch_adjoint_f2_sized<false, 4, 3, 1, 8>(H, "adjoint_stage2", st1, lam, nullptr, mu, 0.0, 0.5, dt)))
+  if ((rc = launch_adjoint_f2_sized<false, 4, 4, 1>(H, "adjoint_stage2", st1, lam, nullptr, mu, 0.0, 0.5, dt)))
     return rc;
-  return launch_adjoint_f2_sized<true, 4, 3, 1, 8>(H, "adjoint_stage1", un, mu, lam, lam, 0.5, 1.0, dt);
+  return launch_adjoint_f2_sized<true, 4, 4, 1>(H, "adjoint_stage1", un, mu, lam, lam, 0.5, 1.0, dt);
 }
 
 template <typename T>
@@ -2273,9 +2262,9 @@ int do_adjoint_step(cup_handle* H, void* const* un, void* const* lam, DtArg dt) 
     if ((rc = upwind_stage1_f32(H, "adjoint_recompute_stage1", un, st1, dt))) return rc;
     return adjoint_upwind_f32(H, un, st1, lam, mu, dt);
   } else {
-    if ((rc = launch_advect<T, 1, 4, 3, 2>(H, "adjoint_recompute_stage1", un, un, st1, dt))) return rc;
-    if ((rc = launch_adjoint<T, 1, false, 2, 2, 1>(H, "adjoint_stage2", st1, lam, nullptr, mu, 0.0, 0.5, dt))) return rc;
-    return launch_adjoint<T, 1, true, 2, 2, 1>(H, "adjoint_stage1", un, mu, lam, lam, 0.5, 1.0, dt);
+    if ((rc = launch_advect<T, 1, 4, 4, 2>(H, "adjoint_recompute_stage1", un, un, st1, dt))) return rc;
+    if ((rc = launch_adjoint<T, 1, false, 2, 3, 1>(H, "adjoint_stage2", st1, lam, nullptr, mu, 0.0, 0.5, dt))) return rc;
+    return launch_adjoint<T, 1, true, 2, 3, 1>(H, "adjoint_stage1", un, mu, lam, lam, 0.5, 1.0, dt);
   }
 }
 
@@ -2305,8 +2294,8 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
     if ((rc = upwind_stage1_f32(H, "adjoint_recompute_stage1", un, st1, dt))) return rc;
     if ((rc = upwind_stage2_f32(H, "adjoint_recompute_stage2", st1, un, us, dt))) return rc;
   } else {
-    if ((rc = launch_advect<T, 1, 4, 3, 2>(H, "adjoint_recompute_stage1", un, un, st1, dt))) return rc;
-    if ((rc = launch_advect<T, 2, 2, 4, 1>(H, "adjoint_recompute_stage2", st1, un, us, dt))) return rc;
+    if ((rc = launch_advect<T, 1, 4, 4, 2>(H, "adjoint_recompute_stage1", un, un, st1, dt))) return rc;
+    if ((rc = launch_advect<T, 2, 4, 4, 2>(H, "adjoint_recompute_stage2", st1, un, us, dt))) return rc;
   }
   if ((rc = do_pressure_rhs<T>(H, dt, us, H->ab0))) return rc;
   if ((rc = fft_poisson(H, H->rhs, H->p_adj))) return rc;
@@ -2357,8 +2346,8 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
   if constexpr (F32) {
     return adjoint_upwind_f32(H, un, st1, lam, mu, dt);
   } else {
-    if ((rc = launch_adjoint<T, 1, false, 2, 2, 1>(H, "adjoint_stage2", st1, lam, nullptr, mu, 0.0, 0.5, dt))) return rc;
-    return launch_adjoint<T, 1, true, 2, 2, 1>(H, "adjoint_stage1", un, mu, lam, lam, 0.5, 1.0, dt);
+    if ((rc = launch_adjoint<T, 1, false, 2, 3, 1>(H, "adjoint_stage2", st1, lam, nullptr, mu, 0.0, 0.5, dt))) return rc;
+    return launch_adjoint<T, 1, true, 2, 3, 1>(H, "adjoint_stage1", un, mu, lam, lam, 0.5, 1.0, dt);
   }
 }
 

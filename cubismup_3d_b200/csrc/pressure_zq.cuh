@@ -50,9 +50,8 @@ constexpr bool pzq_grad() {
 }
 
 struct PzqMaps {
-  CUtensorMap p_main, p_halo;  // FP64 p: box {nx, TY, 1} and {nx, 2, 1}
+  RowMaps p, v;                // FP64 p with 2 halo rows, v* (storage type) with 1
   CUtensorMap f_main[3];       // u*, v*, w* (storage type): box {nx, TY, 1}
-  CUtensorMap v_halo;          // v*: box {nx, 1, 1}
   CUtensorMap h_main;          // FP64 pressure of the previous step p_n: box {nx, TY, 1} (GRAD_CHECK)
 };
 
@@ -99,15 +98,14 @@ struct PzqSlot {
 
 template <typename T, int MODE, int TY, int NS>
 constexpr size_t pzq_smem_bytes_host(int nx) {
-  return (size_t)NS * PzqSlot<T, MODE, TY>::bytes(nx) + NS * sizeof(uint64_t) + 18 * 32 * sizeof(double);
+  return (size_t)NS * PzqSlot<T, MODE, TY>::bytes(nx) + PlaneRing<NS, 0, 8>::kBytes + 18 * 32 * sizeof(double);
 }
 
 // blockDim.x * CPT == TY * nx (<= 512 threads), TY even.
-// NXC, ZCC: nx and the planes per work item fixed at compile time (0: read
-// from g); fixed, the stencil's shared-memory offsets are immediates and the
-// ring slot of each plane is known.
+// NXC: nx fixed at compile time (0: read from g): the stencil's shared-memory
+// offsets are then immediates. Items of an even number of planes.
 // BD: the obstacle terms of b added back on the box (prm.bdelta).
-template <typename T, int MODE, int TY, int NS, int CPT, int NXC = 0, int ZCC = 0, bool BD = false>
+template <typename T, int MODE, int TY, int NS, int CPT, int NXC = 0, bool BD = false>
 __global__ void __launch_bounds__(512) k_pres_zq(const __grid_constant__ PzqMaps maps, const StreamGeom g,
                                                 T* __restrict__ ou, T* __restrict__ ov, T* __restrict__ ow,
                                                 float* __restrict__ rout,
@@ -116,82 +114,53 @@ __global__ void __launch_bounds__(512) k_pres_zq(const __grid_constant__ PzqMaps
   pdl_entry();
   constexpr int G = 2;
   constexpr int Q = 2 * G + 1;
-  constexpr int U = ZCC ? ZCC + 2 * G : 10;  // planes per unrolled chunk: a whole item, or lcm(Q, G)
-  constexpr bool SLOT_CT = ZCC != 0 && (ZCC + 2 * G) % NS == 0;  // ring slot of plane j is j % NS
+  constexpr int U = 10;  // planes per unrolled chunk: lcm(Q, G)
   static_assert(TY >= G && TY % 2 == 0, "tile height must cover the halo depth and keep the row parity");
-  static_assert(ZCC % 2 == 0, "paired barriers and the z parity need an even plane count");
   using Slot = PzqSlot<T, MODE, TY>;
+  constexpr int NL = pzq_grad<MODE>() ? 8 : 4;  // loads of a plane
   static_assert(BD || MODE != PZQ_GRAD_CHECK_BOX, "with the obstacle, b needs its terms");
   if (skip && *skip) return;  // converged defect correction: nothing to check
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   unsigned char* smem_raw = smem_align128(smem_dyn);
   const int nx = NXC ? NXC : g.nx, ny = g.ny, nz = g.nz;
-  const int zc = ZCC ? ZCC : g.zc;
+  const int zc = g.zc;
   const size_t slot_bytes = Slot::bytes(nx);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + NS * slot_bytes);
-  double* scratch = reinterpret_cast<double*>(full + NS);
+  PlaneRing<NS, 0, NL> ring(smem_raw + NS * slot_bytes, err);
+  double* scratch = reinterpret_cast<double*>(smem_raw + NS * slot_bytes + PlaneRing<NS, 0, NL>::kBytes);
   const int tid = threadIdx.x;
   const int PL = zc + 2 * G;
-  const int my_items = blockIdx.x < g.n_items ? (g.n_items - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  const int L = my_items * PL;
-  const uint32_t p_bytes = (uint32_t)Slot::p_bytes(nx);
   const uint32_t rowsT = (uint32_t)(TY * nx * sizeof(T));
-  const uint32_t rowsD = (uint32_t)(TY * nx * sizeof(double));
-
-  if (tid == 0) {
-    for (int s = 0; s < NS; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-
-  auto issue = [&](int q) {
-    const int it = q / PL, j = q - it * PL;
-    const int item = blockIdx.x + it * gridDim.x;
-    const int ty = item % g.items_y, zi = item / g.items_y;
-    const int y0 = ty * TY, z0 = zi * zc;
+  // loads 0: p with its halo rows, 1-3: u*, v* (with its halo rows), w* of the
+  // plane, 4-7 (GRAD_CHECK): u*, v*, w* and the previous p of the output plane
+  auto issue = [&](int l, int s, int j, const ItemPos& p) {
+    const int y0 = p.y0, z0 = p.z0;
     int z = z0 - G + j;
     z = z < 0 ? z + nz : (z >= nz ? z - nz : z);
-    const int s = q % NS;
     unsigned char* dst = smem_raw + s * slot_bytes;
-    int ylo = y0 - G;
-    if (ylo < 0) ylo += ny;
-    int yhi = y0 + TY;
-    if (yhi >= ny) yhi -= ny;
-    uint32_t bytes = p_bytes;
+    uint64_t* bar = &ring.full[s];
     const bool xy_plane = j >= G && j < G + zc;    // planes whose x/y part is computed
-    const bool w_plane = j >= 1 && j < PL - 1;        // planes at z0-1 .. z0+zc (w at z +- 1)
-    const bool out_plane = j >= 2 * G;                // completes output plane j - 2G
-    if (xy_plane) bytes += rowsT + (uint32_t)((TY + 2) * nx * sizeof(T));
-    if (w_plane) bytes += rowsT;
-    if constexpr (pzq_grad<MODE>()) {
-      if (out_plane) bytes += 3 * rowsT + (prm.pred_order >= 1 ? rowsD : 0u);
-    }
-    mbar_arrive_expect_tx(&full[s], bytes);
-    double* P = reinterpret_cast<double*>(dst);
-    tma_load_3d(P, &maps.p_halo, 0, ylo, z, &full[s]);
-    tma_load_3d(P + G * nx, &maps.p_main, 0, y0, z, &full[s]);
-    tma_load_3d(P + (G + TY) * nx, &maps.p_halo, 0, yhi, z, &full[s]);
-    if (xy_plane) {
-      tma_load_3d(dst + Slot::u_off(nx), &maps.f_main[0], 0, y0, z, &full[s]);
-      T* V = reinterpret_cast<T*>(dst + Slot::v_off(nx));
-      tma_load_3d(V, &maps.v_halo, 0, y0 == 0 ? ny - 1 : y0 - 1, z, &full[s]);
-      tma_load_3d(V + nx, &maps.f_main[1], 0, y0, z, &full[s]);
-      tma_load_3d(V + (TY + 1) * nx, &maps.v_halo, 0, yhi, z, &full[s]);
-    }
-    if (w_plane) tma_load_3d(dst + Slot::w_off(nx), &maps.f_main[2], 0, y0, z, &full[s]);
-    if (out_plane) {
-      const int zk = z0 + (j - 2 * G);  // output plane completed by this load (< nz)
-      if constexpr (pzq_grad<MODE>()) {
-#pragma unroll
-        for (int f = 0; f < 3; ++f) tma_load_3d(dst + Slot::f_off(nx, f), &maps.f_main[f], 0, y0, zk, &full[s]);
-        if (prm.pred_order >= 1) tma_load_3d(dst + Slot::h_off(nx), &maps.h_main, 0, y0, zk, &full[s]);
-      }
+    const bool w_plane = j >= 1 && j < PL - 1;     // planes at z0-1 .. z0+zc (w at z +- 1)
+    const bool out_plane = j >= 2 * G;             // completes output plane j - 2G (< nz)
+    if (l == 0) {
+      mbar_arrive_expect_tx(bar, (uint32_t)Slot::p_bytes(nx));
+      tma_load_rows<G, TY>(reinterpret_cast<double*>(dst), maps.p, nx, ny, y0, z, bar);
+    } else if (l == 2 && xy_plane) {
+      mbar_arrive_expect_tx(bar, (uint32_t)((TY + 2) * nx * sizeof(T)));
+      tma_load_rows<1, TY>(reinterpret_cast<T*>(dst + Slot::v_off(nx)), maps.v, nx, ny, y0, z, bar);
+    } else if ((l == 1 && xy_plane) || (l == 3 && w_plane)) {
+      mbar_arrive_expect_tx(bar, rowsT);
+      tma_load_3d(dst + (l == 1 ? Slot::u_off(nx) : Slot::w_off(nx)), &maps.f_main[l - 1], 0, y0, z, bar);
+    } else if (l >= 4 && l < 7 && out_plane) {
+      mbar_arrive_expect_tx(bar, rowsT);
+      tma_load_3d(dst + Slot::f_off(nx, l - 4), &maps.f_main[l - 4], 0, y0, z0 + j - 2 * G, bar);
+    } else if (l == 7 && out_plane && prm.pred_order >= 1) {
+      mbar_arrive_expect_tx(bar, (uint32_t)(TY * nx * sizeof(double)));
+      tma_load_3d(dst + Slot::h_off(nx), &maps.h_main, 0, y0, z0 + j - 2 * G, bar);
+    } else {
+      mbar_arrive(bar);
     }
   };
-
-  int q_issued = 0;
-  if (tid == 0)
-    for (; q_issued < min(L, NS); ++q_issued) issue(q_issued);
+  ring.start(item_pos(g, blockIdx.x, TY, zc), issue);
 
   const int mask = nx - 1;
   // per column: its cell, the shared-memory offsets of its x/y neighbours in
@@ -222,7 +191,7 @@ __global__ void __launch_bounds__(512) k_pres_zq(const __grid_constant__ PzqMaps
   double pq[Q][CPT];
   T wq[Q][CPT];
   // x/y parts of the planes in flight (G of them): Laplacian, divergence and
-  // (GRAD_CHECK) the gradient of p and the u*, v* centre values
+  // (GRAD_CHECK) the gradient of p
   double partL[G][CPT];
   T partD[G][CPT];               // x/y part of the divergence (b from u*: div_xy, div_b)
   double partB[BD ? G : 1][CPT];  // BD: the obstacle terms of the output cell, loaded two planes ahead
@@ -257,25 +226,22 @@ __global__ void __launch_bounds__(512) k_pres_zq(const __grid_constant__ PzqMaps
   for (int i = 0; i < CPT; ++i) pc[i][0] = pc[i][1] = rc[i][0] = rc[i][1] = 0.0;
 
   bool ok = true;
-  int q = 0;
-  for (int it = 0; it < my_items; ++it) {
-    const int item = blockIdx.x + it * gridDim.x;
-    const int ty = item % g.items_y, zi = item / g.items_y;
-    const int y0 = ty * TY, z0 = zi * zc;
-    size_t obase[CPT];  // output index of plane z0
+  ItemPos pos = item_pos(g, blockIdx.x, TY, zc);
+  for (int item = blockIdx.x; item < g.n_items; item += gridDim.x) {
+    const bool more = item + gridDim.x < g.n_items;
+    const ItemPos nextp = item_pos(g, item + gridDim.x, TY, zc);
+    const int y0 = pos.y0, z0 = pos.z0;
+    size_t ob[CPT];  // output index of the next plane
 #pragma unroll
-    for (int i = 0; i < CPT; ++i) obase[i] = gidx(cx[i], y0 + cy[i], z0, nx, ny);
-    const int q0 = q;  // first load of the item (a multiple of NS when SLOT_CT)
+    for (int i = 0; i < CPT; ++i) ob[i] = gidx(cx[i], y0 + cy[i], z0, nx, ny);
     for (int j0 = 0; j0 < PL; j0 += U) {
 #pragma unroll
       for (int jj = 0; jj < U; ++jj) {
         const int j = j0 + jj;
         if (j >= PL) break;  // items of PL planes, PL not a multiple of U
-        const int s = SLOT_CT ? jj % NS : q % NS;
-        const uint32_t phase = SLOT_CT ? ((q0 / NS + jj / NS) & 1) : ((q / NS) & 1);
-        if (ok) ok = mbar_wait(&full[s], phase, err);
+        if (ok) ok = ring.wait();
         if (ok) {
-          const unsigned char* sl = smem_raw + s * slot_bytes;
+          const unsigned char* sl = smem_raw + ring.slot * slot_bytes;
           const double* P = reinterpret_cast<const double*>(sl);
           const int QN = jj % Q;
 #pragma unroll
@@ -295,7 +261,8 @@ __global__ void __launch_bounds__(512) k_pres_zq(const __grid_constant__ PzqMaps
             const int zp = jj & 1;
 #pragma unroll
             for (int i = 0; i < CPT; ++i) {
-              const size_t o = obase[i] + (size_t)k * plane;
+              const size_t o = ob[i];
+              ob[i] += plane;
               const int c = cy[i] * nx + cx[i];
               const double p0 = pq[QC][i];
               const double lap = partL[PS][i] + (pq[QP2][i] + pq[QM2][i] - 2 * p0);
@@ -369,30 +336,13 @@ __global__ void __launch_bounds__(512) k_pres_zq(const __grid_constant__ PzqMaps
             }
           }
         }
-        // rings of 4+ slots: one block barrier per two planes (slots of loads
-        // q-1 and q fully consumed, refill both; q is odd here: PL and U are
-        // even); shallower rings keep one barrier per plane for lookahead
-        if constexpr (NS >= 4) {
-          if (jj & 1) {
-            __syncthreads();
-            if (tid == 0 && ok)
-              for (int r = q - 1 + NS; r <= q + NS && r < L; ++r)
-                if (r == q_issued) issue(q_issued++);
-          }
-        } else {
-          __syncthreads();  // slot s fully consumed
-          if (tid == 0 && ok && q_issued < L && q_issued == q + NS) issue(q_issued++);
-        }
-        ++q;
+        ring.step(ok, jj & 1, j, PL, pos, nextp, more, issue);
       }
     }
+    pos = nextp;
   }
-  // after a timed-out wait: bounded drain of the loads that may be in flight
-  // (at most the last NS issued)
-  if (!ok && tid == 0) {
-    for (int r = q_issued - NS < 0 ? 0 : q_issued - NS; r < q_issued; ++r)
-      mbar_wait(&full[r % NS], (r / NS) & 1, nullptr);
-  }
+  ring.drain(ok);
+  __syncthreads();
   // per-CTA partial sums
   {
     constexpr int NPV = pzq_partials_per_cta<MODE>();
