@@ -26,6 +26,7 @@
 #include "advect_f2.cuh"
 #include "common.cuh"
 #include "dht.cuh"
+#include "grad_zq.cuh"
 #include "pfft.cuh"
 #include "pressure_zq.cuh"
 #include "ops.cuh"
@@ -1751,16 +1752,56 @@ int do_poisson(cup_handle* H) {
   return do_poisson_dc(H);
 }
 
+// Launches one k_grad_zq pass: out = in - dt/(2h) grad_c p; returns the grid
+// size (number of partials). Grids of nx 64, 128 or 256 take the
+// compile-time-nx kernels. Ring depth 4, measured: FP64 256^3 155 us (5: 162, 6:
+// 164), FP32 256x128x128 18.6 us with two CTAs per SM (6: 22.7, one CTA).
+template <typename T, bool REDUCE, int NXC>
+int launch_grad_sized(cup_handle* H, const char* name, void* const* in, void* const* out, const double* p, DtArg dt,
+                      int* grid_out) {
+  constexpr int TY = 4, NS = 4, CPT = 2;
+  GradMaps maps;
+  int rc = make_row_maps<double>(H, &maps.p, p, TY, 1);
+  for (int q = 0; q < 3 && !rc; ++q) rc = make_map(H, &maps.f[q], in[q], tma_dtype<T>(), sizeof(T), H->nx, TY, 1);
+  if (rc) return rc;
+  auto kern = k_grad_zq<T, REDUCE, TY, NS, CPT, NXC>;
+  const size_t smem = grad_smem_bytes<T, TY, NS>(H->nx) + 128;
+  const int threads = TY * H->nx / CPT;
+  int bpsm = 0;
+  if ((rc = prepare_kernel(H, kern, smem, threads, &bpsm))) return rc;
+  const int zc = planes_per_item(H, TY, 1, bpsm);
+  StreamGeom geo{H->nx, H->ny, H->nz, ilog2(H->nx), zc, H->ny / TY, (H->ny / TY) * (H->nz / zc)};
+  const int grid = std::min(geo.n_items, bpsm * H->num_sms);
+  if (grid > kPartialCap / 2) return fail(H, CUP_ERR_ARG, "too many CTAs for the partial buffers");
+  const GradParams prm{dt, H->h, {H->uinf[0], H->uinf[1], H->uinf[2]}, H->box, H->has_sphere ? 1 : 0};
+  rc = launch_named(H, name, [&]() -> int {
+    klaunch(H, kern, grid, threads, smem, maps, geo, (T*)out[0], (T*)out[1], (T*)out[2], partial(H, P_GRAD), prm,
+            H->derr);
+    CKL();
+    return CUP_OK;
+  });
+  if (grid_out) *grid_out = grid;
+  return rc;
+}
+template <typename T, bool REDUCE>
+int launch_grad(cup_handle* H, const char* name, void* const* in, void* const* out, const double* p, DtArg dt,
+                int* grid_out = nullptr) {
+  switch (H->nx) {
+    case 64: return launch_grad_sized<T, REDUCE, 64>(H, name, in, out, p, dt, grid_out);
+    case 128: return launch_grad_sized<T, REDUCE, 128>(H, name, in, out, p, dt, grid_out);
+    case 256: return launch_grad_sized<T, REDUCE, 256>(H, name, in, out, p, dt, grid_out);
+    default: break;
+  }
+  return launch_grad_sized<T, REDUCE, 0>(H, name, in, out, p, dt, grid_out);
+}
+
 template <typename T>
 int do_grad(cup_handle* H, DtArg dt) {
-  const void* pf[1] = {H->p};
-  OpGradP<T> op{(const T*)H->u, (const T*)H->v, (const T*)H->w, (T*)H->u, (T*)H->v, (T*)H->w, partial(H, P_GRAD),
-                dt, H->h, {H->uinf[0], H->uinf[1], H->uinf[2]}, H->box, H->has_sphere ? 1 : 0, H->nx, H->ny, H->nz};
-  // p is FP64 in both forms: the stream runs over an FP64 field.
+  void* u[3] = {H->u, H->v, H->w};
   H->grad_stride = 2;
   H->grad_max_off = 0;
   H->grad_ke_off = 1;
-  return launch_stream<double, 1, 1, 4, 4>(H, "grad_p", pf, op, &H->n_grad_partials);
+  return launch_grad<T, true>(H, "grad_p", u, u, H->p, dt, &H->n_grad_partials);
 }
 
 template <typename T>
@@ -2160,16 +2201,6 @@ int launch_adjoint(cup_handle* H, const char* name, const void* const* f, const 
   });
 }
 
-// out = in - dt/(2h) grad_c p (KernelGradP on given fields; out may equal in).
-template <typename T>
-int do_grad_fields(cup_handle* H, const char* name, void* const* in, void* const* out, const double* pbuf, DtArg dt) {
-  const void* pf[1] = {pbuf};
-  OpGradP<T> op{(const T*)in[0], (const T*)in[1], (const T*)in[2], (T*)out[0], (T*)out[1], (T*)out[2],
-                partial(H, P_GRAD), dt, H->h, {H->uinf[0], H->uinf[1], H->uinf[2]}, H->box, 0, H->nx, H->ny, H->nz};
-  int ngp = 0;
-  return launch_stream<double, 1, 1, 4, 4>(H, name, pf, op, &ngp);
-}
-
 // The projection P = I - G L^+ D of the pipeline (PressureRHS, the periodic
 // FFT solve in FP64, the gradient correction) applied to the fields `in`,
 // result in `out` (may equal `in`). D = -G^T on the periodic grid and L = D G
@@ -2179,7 +2210,7 @@ template <typename T>
 int do_project_fields(cup_handle* H, void* const* in, void* const* out, double* pbuf, DtArg dt) {
   int rc;
   if ((rc = do_solve_rhs_of<T>(H, "adjoint_rhs_dht_x", "adjoint_dht_x", in, pbuf, dt))) return rc;
-  return do_grad_fields<T>(H, "adjoint_grad_p", in, out, pbuf, dt);
+  return launch_grad<T, false>(H, "adjoint_grad_p", in, out, pbuf, dt);
 }
 
 // Adjoint of one step u_{n+1} = P(H(u_n)) with the dt given, at the state un:
@@ -2299,7 +2330,7 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
   }
   if ((rc = do_pressure_rhs<T>(H, dt, us, H->ab0))) return rc;
   if ((rc = fft_poisson(H, H->rhs, H->p_adj))) return rc;
-  if ((rc = do_grad_fields<T>(H, "adjoint_recompute_grad_p", us, us, H->p_adj, dt))) return rc;
+  if ((rc = launch_grad<T, false>(H, "adjoint_recompute_grad_p", us, us, H->p_adj, dt))) return rc;
   // 2. penalization and force
   const int gb = box_grid(H->box);
   const double lambda = H->cfg.DLM > 0 ? H->cfg.DLM / dtv : H->lambda;
@@ -2338,11 +2369,11 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
   }
   // 4. gradient correction, then the advection transposes
   if (H->cfg.scheme == CUP_SCHEME_REF) {
-    if ((rc = do_grad_fields<T>(H, "adjoint_grad_p", lam, mu, H->p_adj, dt))) return rc;
+    if ((rc = launch_grad<T, false>(H, "adjoint_grad_p", lam, mu, H->p_adj, dt))) return rc;
     if constexpr (F32) return launch_adjoint<T, 0, false, 4, 3, 2>(H, "adjoint_ref", un, mu, nullptr, lam, 0.0, 1.0, dt);
     else return launch_adjoint<T, 0, false, 2, 3, 1>(H, "adjoint_ref", un, mu, nullptr, lam, 0.0, 1.0, dt);
   }
-  if ((rc = do_grad_fields<T>(H, "adjoint_grad_p", lam, lam, H->p_adj, dt))) return rc;
+  if ((rc = launch_grad<T, false>(H, "adjoint_grad_p", lam, lam, H->p_adj, dt))) return rc;
   if constexpr (F32) {
     return adjoint_upwind_f32(H, un, st1, lam, mu, dt);
   } else {

@@ -206,54 +206,6 @@ struct Box {
   }
 };
 
-// KernelGradP (source/operators/PressureProjection.cpp:38-50):
-// u -= (dt/2h) (p(x+1) - p(x-1)) etc. Fused epilogue: per-CTA FP64 partials of
-// max |u + uinf| (the next calcMaxTimestep, source/operators/ProcessHelpers.h:74-99)
-// over cells outside the obstacle box (the penalization kernel covers the box)
-// and the kinetic energy sum |u|^2/2 (ComputeDissipation.cpp:47-116 pattern).
-template <typename T>
-struct OpGradP {
-  const T *su, *sv, *sw;  // u* (point-wise)
-  T *ou, *ov, *ow;        // projected velocity
-  double* partials;       // [gridDim.x][2]: max, ke
-  DtArg dt;
-  double h;
-  double uinf[3];
-  Box box;
-  int has_box;
-  int nx, ny, nz;
-  template <class C>
-  __device__ __forceinline__ void cell(const C& c, int x, int y, int gy, int gz, double* acc) const {
-    const double fac = -0.5 * dt.get() / h;
-    const double pE = c.v(0, x, y, 1, 0, 0), pW = c.v(0, x, y, -1, 0, 0);
-    const double pN = c.v(0, x, y, 0, 1, 0), pS = c.v(0, x, y, 0, -1, 0);
-    const double pB = c.v(0, x, y, 0, 0, 1), pF = c.v(0, x, y, 0, 0, -1);
-    const size_t o = gidx(x, gy, gz, nx, ny);
-    const double u = (double)su[o] + fac * (pE - pW);
-    const double v = (double)sv[o] + fac * (pN - pS);
-    const double w = (double)sw[o] + fac * (pB - pF);
-    const T tu = (T)u, tv = (T)v, tw = (T)w;
-    ou[o] = tu;
-    ov[o] = tv;
-    ow[o] = tw;
-    if (!(has_box && box.contains(x, gy, gz, nx, ny, nz))) {
-      const double m = fmax(fmax(fabs((double)tu + uinf[0]), fabs((double)tv + uinf[1])), fabs((double)tw + uinf[2]));
-      acc[0] = fmax(acc[0], m);
-    }
-    acc[1] += 0.5 * ((double)tu * tu + (double)tv * tv + (double)tw * tw);
-  }
-  __device__ void finish(double* acc, double* scratch) const {
-    double mx[1] = {acc[0]};
-    double sm[1] = {acc[1]};
-    block_reduce<1, true>(mx, scratch);
-    block_reduce<1, false>(sm, scratch + 32);
-    if (threadIdx.x == 0) {
-      partials[2 * blockIdx.x + 0] = mx[0];
-      partials[2 * blockIdx.x + 1] = sm[0];
-    }
-  }
-};
-
 // ---------------------------------------------------------------------------
 // Obstacle-box kernels. Sphere parameters live in device memory so that the
 // host can update them without relaunch changes.
