@@ -30,6 +30,7 @@
 #include "pfft.cuh"
 #include "pressure_zq.cuh"
 #include "ops.cuh"
+#include "spectral.cuh"
 #include "stencil.cuh"
 
 using namespace cup;
@@ -403,203 +404,6 @@ __global__ void k_finalize_residual(const double* p, int stride, int np, DevStat
   }
 }
 
-// ComputeDissipation (source/operators/ComputeDissipation.cpp:38-116): per
-// cell, vorticity, pressure power -(1-chi) h^3 grad p . u, viscous power
-// (1-chi) h^3 nu (u . lap u + 2 D:D), and the linear / angular invariants
-// about the domain centre; per-CTA FP64 partials of the 20 sums in the order
-// of the reference's reduction (:132-152). hCube = pow(h, 3), inv2h = 1/(2h),
-// invHh = 1/h^2 and the centre come from the host as the reference computes
-// them.
-template <typename T>
-__global__ void k_dissipation(const T* u, const T* v, const T* w, const double* p, const T* chi, int nx, int ny,
-                              int nz, double h, double nu, double hCube, double inv2h, double invHh, double cx,
-                              double cy, double cz, double* partials /* [gridDim.x][20] */) {
-  pdl_entry();
-  __shared__ double scratch[20 * 32];
-  double R[20];
-#pragma unroll
-  for (int k = 0; k < 20; ++k) R[k] = 0.0;
-  const size_t n = (size_t)nx * ny * nz;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((size_t)nx * ny));
-    const int xp = wrapi(x + 1, nx), xm = wrapi(x - 1, nx), yp = wrapi(y + 1, ny), ym = wrapi(y - 1, ny),
-              zp = wrapi(z + 1, nz), zm = wrapi(z - 1, nz);
-    const size_t o = i;
-    const size_t oE = gidx(xp, y, z, nx, ny), oW = gidx(xm, y, z, nx, ny), oN = gidx(x, yp, z, nx, ny),
-                 oS = gidx(x, ym, z, nx, ny), oB = gidx(x, y, zp, nx, ny), oF = gidx(x, y, zm, nx, ny);
-    const double X = chi ? (double)chi[o] : 0.0;
-    const double PX = (x + 0.5) * h - cx, PY = (y + 0.5) * h - cy, PZ = (z + 0.5) * h - cz;
-    const double uc = u[o], vc = v[o], wc = w[o];
-    const double uE = u[oE], uW = u[oW], uN = u[oN], uS = u[oS], uB = u[oB], uF = u[oF];
-    const double vE = v[oE], vW = v[oW], vN = v[oN], vS = v[oS], vB = v[oB], vF = v[oF];
-    const double wE = w[oE], wW = w[oW], wN = w[oN], wS = w[oS], wB = w[oB], wF = w[oF];
-    const double WX = inv2h * ((wN - wS) - (vB - vF));
-    const double WY = inv2h * ((uB - uF) - (wE - wW));
-    const double WZ = inv2h * ((vE - vW) - (uN - uS));
-    const double dPdx = inv2h * (p[oE] - p[oW]);
-    const double dPdy = inv2h * (p[oN] - p[oS]);
-    const double dPdz = inv2h * (p[oB] - p[oF]);
-    R[15] -= (1 - X) * hCube * (dPdx * uc + dPdy * vc + dPdz * wc);
-    const double lapU = invHh * (uE + uW + uN + uS + uB + uF - 6 * uc);
-    const double lapV = invHh * (vE + vW + vN + vS + vB + vF - 6 * vc);
-    const double lapW = invHh * (wE + wW + wN + wS + wB + wF - 6 * wc);
-    const double V1 = lapU * uc + lapV * vc + lapW * wc;
-    const double D11 = inv2h * (uE - uW);
-    const double D22 = inv2h * (vN - vS);
-    const double D33 = inv2h * (wB - wF);
-    const double D12 = inv2h * (uN - uS + vE - vW) / 2;
-    const double D13 = inv2h * (uB - uF + wE - wW) / 2;
-    const double D23 = inv2h * (wN - wS + vB - vF) / 2;
-    const double V2 = D11 * D11 + D22 * D22 + D33 * D33 + 2 * (D12 * D12 + D13 * D13 + D23 * D23);
-    R[16] += (1 - X) * hCube * nu * (V1 + 2 * V2);
-    R[0] += hCube * WX;
-    R[1] += hCube * WY;
-    R[2] += hCube * WZ;
-    R[3] += hCube / 2 * (PY * WZ - PZ * WY);
-    R[4] += hCube / 2 * (PZ * WX - PX * WZ);
-    R[5] += hCube / 2 * (PX * WY - PY * WX);
-    R[6] += hCube * uc;
-    R[7] += hCube * vc;
-    R[8] += hCube * wc;
-    R[9] += hCube / 3 * (PX * (PY * WY + PZ * WZ) - WX * (PY * PY + PZ * PZ));
-    R[10] += hCube / 3 * (PY * (PX * WX + PZ * WZ) - WY * (PX * PX + PZ * PZ));
-    R[11] += hCube / 3 * (PZ * (PX * WX + PY * WY) - WZ * (PX * PX + PY * PY));
-    R[12] += hCube * (PY * wc - PZ * vc);
-    R[13] += hCube * (PZ * uc - PX * wc);
-    R[14] += hCube * (PX * vc - PY * uc);
-    R[17] += hCube * (WX * uc + WY * vc + WZ * wc);
-    R[18] += hCube * (uc * uc + vc * vc + wc * wc) / 2;
-    R[19] += sqrt(WX * WX + WY * WY + WZ * WZ);
-  }
-  block_reduce<20, false>(R, scratch);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 20; ++k) partials[20 * blockIdx.x + k] = R[k];
-}
-
-// Spectral analysis and forcing (source/spectralOperators/SpectralManipFFTW.cpp:25-193,
-// SpectralForcing.cpp:23-86) on the separable Hartley coefficients of the
-// Poisson passes instead of FFTW's r2c spectrum. The separable transform
-// mixes the DFT coefficients of the 8 modes (+-kx, +-ky, +-kz) orthogonally,
-// and every quantity the reference takes per mode is a function of |k| (the
-// shell of the spectrum, 1/|k|, the 0 < k^2 <= 4 forcing band), so sums over
-// modes are the same: E = 1/2 (Hu^2 + Hv^2 + Hw^2) per separable mode is the
-// reference's mult/2 |U|^2 summed over the conjugate-symmetric full spectrum.
-// The vorticity sum is taken in physical space, where Parseval puts it: the
-// reference's eps is nu times the mean of |curl_c u|^2 (central differences).
-template <typename T>
-__global__ void k_widen(const T* __restrict__ src, double* __restrict__ dst, size_t n) {
-  pdl_entry();
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    dst[i] = (double)src[i];
-}
-
-// Per separable mode: E, E / |k| (the integral length), the binned spectrum
-// (bin floor(sqrt(kind) (nyquist - 1) / nyquist) for kind = ii^2 + jj^2 + kk^2
-// < nyquist^2) and, when filtering, the energy of the forcing band with every
-// other mode zeroed in place. Per-CTA partials: [tke, lIntegral, tkeFiltered,
-// nbin spectrum values]; the bins are summed with shared-memory atomics.
-__global__ void k_spectral_modes(double* hu, double* hv, double* hw, int nx, int ny, int nz, double wfx, double wfy,
-                                 double wfz, int nyquist, double nyq_scaling, int nbin, int filter,
-                                 double* partials) {
-  pdl_entry();
-  extern __shared__ double sbins[];
-  __shared__ double scratch[3 * 32];
-  for (int b = threadIdx.x; b < nbin; b += blockDim.x) sbins[b] = 0.0;
-  __syncthreads();
-  double acc[3] = {0, 0, 0};
-  const size_t n = (size_t)nx * ny * nz;
-  const long long nyq2 = (long long)nyquist * nyquist;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((size_t)nx * ny));
-    const long ii = x <= nx / 2 ? x : -(long)(nx - x);
-    const long jj = y <= ny / 2 ? y : -(long)(ny - y);
-    const long kk = z <= nz / 2 ? z : -(long)(nz - z);
-    const double kx = ii * wfx, ky = jj * wfy, kz = kk * wfz;
-    const double k2 = kx * kx + ky * ky + kz * kz;
-    const double U = hu[i], V = hv[i], W = hw[i];
-    const double E = 0.5 * (U * U + V * V + W * W);
-    acc[0] += E;
-    acc[1] += k2 > 0 ? E / sqrt(k2) : 0.0;
-    const long long kind = (long long)ii * ii + (long long)jj * jj + (long long)kk * kk;
-    if (kind < nyq2) {
-      const int b = (int)floor(sqrt((double)kind) * nyq_scaling);
-      if (b < nbin) atomicAdd(&sbins[b], E);
-    }
-    if (filter) {
-      if (k2 > 0 && k2 <= 4) {
-        acc[2] += E;
-      } else {
-        hu[i] = 0.0;
-        hv[i] = 0.0;
-        hw[i] = 0.0;
-      }
-    }
-  }
-  block_reduce<3, false>(acc, scratch);
-  const int stride = 3 + nbin;
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; ++k) partials[(size_t)stride * blockIdx.x + k] = acc[k];
-  for (int b = threadIdx.x; b < nbin; b += blockDim.x) partials[(size_t)stride * blockIdx.x + 3 + b] = sbins[b];
-}
-
-// Per-CTA partial sums of |curl_c u|^2 (central differences / 2h).
-template <typename T>
-__global__ void k_vorticity2(const T* u, const T* v, const T* w, int nx, int ny, int nz, double inv2h,
-                             double* partials) {
-  pdl_entry();
-  __shared__ double scratch[32];
-  double acc[1] = {0.0};
-  const size_t n = (size_t)nx * ny * nz;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((size_t)nx * ny));
-    const size_t oE = gidx(wrapi(x + 1, nx), y, z, nx, ny), oW = gidx(wrapi(x - 1, nx), y, z, nx, ny);
-    const size_t oN = gidx(x, wrapi(y + 1, ny), z, nx, ny), oS = gidx(x, wrapi(y - 1, ny), z, nx, ny);
-    const size_t oB = gidx(x, y, wrapi(z + 1, nz), nx, ny), oF = gidx(x, y, wrapi(z - 1, nz), nx, ny);
-    const double WX = inv2h * (((double)w[oN] - (double)w[oS]) - ((double)v[oB] - (double)v[oF]));
-    const double WY = inv2h * (((double)u[oB] - (double)u[oF]) - ((double)w[oE] - (double)w[oW]));
-    const double WZ = inv2h * (((double)v[oE] - (double)v[oW]) - ((double)u[oN] - (double)u[oS]));
-    acc[0] += WX * WX + WY * WY + WZ * WZ;
-  }
-  block_reduce<1, false>(acc, scratch);
-  if (threadIdx.x == 0) partials[blockIdx.x] = acc[0];
-}
-
-// f += factor * g (g FP64), rounded once to the storage type.
-template <typename T>
-__global__ void k_add_scaled(T* f, const double* g, double factor, size_t n) {
-  pdl_entry();
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    f[i] = (T)((double)f[i] + factor * g[i]);
-}
-
-// Diagnostics: kinetic energy and central-divergence norms (FP64).
-template <typename T>
-__global__ void k_diag(const T* u, const T* v, const T* w, int nx, int ny, int nz, double inv2h, double* partials) {
-  pdl_entry();
-  __shared__ double scratch[3 * 32];
-  double s[2] = {0, 0};
-  double m[1] = {0};
-  const size_t n = (size_t)nx * ny * nz;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(i % nx), y = (int)((i / nx) % ny), z = (int)(i / ((size_t)nx * ny));
-    const double uu = u[i], vv = v[i], ww = w[i];
-    s[0] += 0.5 * (uu * uu + vv * vv + ww * ww);
-    const double div =
-        inv2h * ((double)u[gidx(wrapi(x + 1, nx), y, z, nx, ny)] - (double)u[gidx(wrapi(x - 1, nx), y, z, nx, ny)] +
-                 (double)v[gidx(x, wrapi(y + 1, ny), z, nx, ny)] - (double)v[gidx(x, wrapi(y - 1, ny), z, nx, ny)] +
-                 (double)w[gidx(x, y, wrapi(z + 1, nz), nx, ny)] - (double)w[gidx(x, y, wrapi(z - 1, nz), nx, ny)]);
-    s[1] += div * div;
-    m[0] = fmax(m[0], fabs(div));
-  }
-  block_reduce<2, false>(s, scratch);
-  block_reduce<1, true>(m, scratch + 2 * 32);
-  if (threadIdx.x == 0) {
-    partials[3 * blockIdx.x + 0] = s[0];
-    partials[3 * blockIdx.x + 1] = s[1];
-    partials[3 * blockIdx.x + 2] = m[0];
-  }
-}
-
 // Periodic shift through the plane-streaming path (TestBoundaries restatement).
 struct OpShift {
   double* out;
@@ -835,7 +639,11 @@ struct cup_handle {
   void *au = nullptr, *av = nullptr, *aw = nullptr;
   double* p_adj = nullptr;
   // spectral analysis / forcing: FP64 Hartley coefficients of u, v, w (allocated on first use)
+  // (one allocation), the forcing band's coefficients, sums on their way to the
+  // host and the pinned buffer they land in
   double* spec[3] = {nullptr, nullptr, nullptr};
+  double* band_coef = nullptr;
+  double *dsum = nullptr, *hsum = nullptr;
   bool forcing = false;                 // SpectralForcing inside cup_step / cup_run
   double forcing_target = 0, forcing_rate = 0, forcing_prev_tke = 0;
   double forcing_stats[6] = {0, 0, 0, 0, 0, 0};
@@ -958,10 +766,11 @@ int launch_named(cup_handle* H, const char* name, F&& f) {
   return rc;
 }
 
+// nf: fields one after the other, as one of nf times the planes.
 int make_map(cup_handle* H, CUtensorMap* m, const void* base, CUtensorMapDataType dt, size_t elem, int bx, int by,
-             int bz) {
+             int bz, int nf = 1) {
   if (!get_encode()) return fail(H, CUP_ERR_CUDA, "cuTensorMapEncodeTiled entry point unavailable");
-  cuuint64_t dims[3] = {(cuuint64_t)H->nx, (cuuint64_t)H->ny, (cuuint64_t)H->nz};
+  cuuint64_t dims[3] = {(cuuint64_t)H->nx, (cuuint64_t)H->ny, (cuuint64_t)H->nz * nf};
   cuuint64_t strides[2] = {(cuuint64_t)H->nx * elem, (cuuint64_t)H->nx * H->ny * elem};
   cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
   cuuint32_t estr[3] = {1, 1, 1};
@@ -1055,45 +864,51 @@ int launch_stream(cup_handle* H, const char* name, const void* const* fields, co
   return CUP_OK;
 }
 
-// Pipelined Hartley x pass (k_dht_rows_pipe): rows of `buf` transformed in place.
-template <int M>
-int launch_rows_pipe_M(cup_handle* H, const char* name, double* buf) {
+// Pipelined Hartley x pass (k_dht_rows_pipe): the rows of nf fields (FP64, or
+// FP32 widened on the way) into out, one field after the other.
+template <int M, typename RIN>
+int launch_rows_pipe_M(cup_handle* H, const char* name, const RIN* const* f, int nf, double* out) {
   constexpr int N = 2 * M, TPL = M / 8;
   constexpr bool PAD = FFTPlan<M>::nstages > 1;
   constexpr int NB = 2;
   const int lpc = 256 / TPL;
-  const int nrows = H->ny * H->nz;
+  const RowsIn<RIN> in{{f[0], nf > 1 ? f[1] : nullptr, nf > 2 ? f[2] : nullptr}, H->ny * H->nz};
   const size_t smem = (size_t)NB * lpc * N * sizeof(double) + (PAD ? (size_t)lpc * 2 * (M + M / 8) * sizeof(double) : 0) +
                       FFTPlan<M>::rows_table_len() * sizeof(double2) + NB * sizeof(uint64_t) + 128;
-  auto kern = k_dht_rows_pipe<M, double, NB>;
+  auto kern = k_dht_rows_pipe<M, RIN, NB>;
   const int threads = lpc * TPL;
   int bpsm = 0;
   int rc = prepare_kernel(H, kern, smem, threads, &bpsm);
   if (rc) return rc;
-  const int ntiles = (nrows + lpc - 1) / lpc;
+  const int ntiles = nf * in.rows / lpc;  // ny nz is a multiple of 256 >= lpc
   const int grid = std::min(ntiles, bpsm * H->num_sms);
   return launch_named(H, name, [&]() -> int {
-    klaunch(H, kern, grid, threads, smem, (const double*)buf, buf, nrows, lpc, (const double2*)H->tw64[0], H->derr,
-            (const int*)nullptr);
+    klaunch(H, kern, grid, threads, smem, in, out, nf * in.rows, lpc, (const double2*)H->tw64[0], H->derr);
     CKL();
     return CUP_OK;
   });
 }
 
-int launch_rows_pipe(cup_handle* H, const char* name, double* buf) {
+template <typename RIN>
+int launch_rows_pipe(cup_handle* H, const char* name, const RIN* const* f, int nf, double* out) {
   switch (H->nx / 2) {
-    case 8: return launch_rows_pipe_M<8>(H, name, buf);
-    case 16: return launch_rows_pipe_M<16>(H, name, buf);
-    case 32: return launch_rows_pipe_M<32>(H, name, buf);
-    case 64: return launch_rows_pipe_M<64>(H, name, buf);
-    case 128: return launch_rows_pipe_M<128>(H, name, buf);
+    case 8: return launch_rows_pipe_M<8, RIN>(H, name, f, nf, out);
+    case 16: return launch_rows_pipe_M<16, RIN>(H, name, f, nf, out);
+    case 32: return launch_rows_pipe_M<32, RIN>(H, name, f, nf, out);
+    case 64: return launch_rows_pipe_M<64, RIN>(H, name, f, nf, out);
+    case 128: return launch_rows_pipe_M<128, RIN>(H, name, f, nf, out);
   }
   return fail(H, CUP_ERR_ARG, "unsupported nx %d", H->nx);
 }
+int launch_rows_pipe(cup_handle* H, const char* name, double* buf) {
+  const double* f[1] = {buf};
+  return launch_rows_pipe<double>(H, name, f, 1, buf);
+}
 
-// Hartley y or z pass (z: with the spectral divide and the inverse when DIVIDE), in place on buf.
+// Hartley y or z pass (z: with the spectral divide and the inverse when DIVIDE),
+// in place on buf; y: of nf fields one after the other.
 template <int M, int AXIS, bool DIVIDE>
-int launch_cols_M(cup_handle* H, double* buf) {
+int launch_cols_M(cup_handle* H, double* buf, int nf) {
   // 16 x-columns per tile (128-B rows), NB tile buffers; 256-long lines: the
   // 8-thread plan (radix 16, then radix 8 fused with the split)
   constexpr bool T8 = M == 128;
@@ -1101,7 +916,7 @@ int launch_cols_M(cup_handle* H, double* buf) {
   if (AXIS == 2 && H->cfg.z_halo)
     return fail(H, CUP_ERR_STATE, "a z-slab handle has no z transform (the Poisson solve runs over the ranks)");
   CUtensorMap map;
-  int rc = make_map(H, &map, buf, tma_dtype<double>(), sizeof(double), W, AXIS == 1 ? N : 1, AXIS == 2 ? N : 1);
+  int rc = make_map(H, &map, buf, tma_dtype<double>(), sizeof(double), W, AXIS == 1 ? N : 1, AXIS == 2 ? N : 1, nf);
   if (rc) return rc;
   const size_t smem = (size_t)NB * N * W * sizeof(double) + FFTPlan<M>::table_len() * sizeof(double2) +
                       NB * sizeof(uint64_t) + (DIVIDE ? (M / 2 + 1) * sizeof(double) : 0) + 128;
@@ -1111,7 +926,7 @@ int launch_cols_M(cup_handle* H, double* buf) {
   rc = prepare_kernel(H, kern, smem, threads, &bpsm);
   if (rc) return rc;
   const int ntx = H->nx / W;
-  const int ntiles = ntx * (AXIS == 1 ? H->nz : H->ny);
+  const int ntiles = ntx * (AXIS == 1 ? nf * H->nz : H->ny);
   const int grid = std::min(ntiles, bpsm * H->num_sms);
   SpectralParams sp{H->cosx, H->cosy, H->cosz, H->norm_factor, H->nx, H->spec_ny, H->nz, H->spec_y0};
   return launch_named(H, AXIS == 1 ? "dht_y" : "dht_z_solve", [&]() -> int {
@@ -1123,14 +938,14 @@ int launch_cols_M(cup_handle* H, double* buf) {
 }
 
 template <int AXIS, bool DIVIDE>
-int launch_cols(cup_handle* H, double* buf) {
+int launch_cols(cup_handle* H, double* buf, int nf = 1) {
   const int N = AXIS == 1 ? H->ny : H->nz;
   switch (N / 2) {
-    case 8: return launch_cols_M<8, AXIS, DIVIDE>(H, buf);
-    case 16: return launch_cols_M<16, AXIS, DIVIDE>(H, buf);
-    case 32: return launch_cols_M<32, AXIS, DIVIDE>(H, buf);
-    case 64: return launch_cols_M<64, AXIS, DIVIDE>(H, buf);
-    case 128: return launch_cols_M<128, AXIS, DIVIDE>(H, buf);
+    case 8: return launch_cols_M<8, AXIS, DIVIDE>(H, buf, nf);
+    case 16: return launch_cols_M<16, AXIS, DIVIDE>(H, buf, nf);
+    case 32: return launch_cols_M<32, AXIS, DIVIDE>(H, buf, nf);
+    case 64: return launch_cols_M<64, AXIS, DIVIDE>(H, buf, nf);
+    case 128: return launch_cols_M<128, AXIS, DIVIDE>(H, buf, nf);
   }
   return fail(H, CUP_ERR_ARG, "unsupported line length %d", N);
 }
@@ -2003,73 +1818,127 @@ int relocate_sphere(cup_handle* H) {
   return build_sphere_chi(H);
 }
 
-// The spectral sums of the current velocity (see k_spectral_modes): raw[0..2]
+// Column sums of per-CTA partials (max_col: that column's maximum) to
+// dsum[at..], stream-ordered.
+constexpr int kSumCap = 256;  // doubles of dsum / hsum (a spectrum has at most 127 bins)
+int sum_columns(cup_handle* H, const double* part, int np, int ncol, int max_col, int at) {
+  if (!H->dsum) {
+    CK(cudaMalloc(&H->dsum, kSumCap * sizeof(double)));
+    CK(cudaMallocHost(&H->hsum, kSumCap * sizeof(double)));
+  }
+  return launch_named(H, "sum_columns", [&]() -> int {
+    klaunch(H, k_reduce_columns, ncol, 256, 0, part, np, ncol, max_col, H->dsum + at);
+    CKL();
+    return CUP_OK;
+  });
+}
+// The first n sums in H->hsum, and the device error word: one synchronisation.
+int read_sums(cup_handle* H, int n) {
+  CK(cudaMemcpyAsync(H->hsum, H->dsum, n * sizeof(double), cudaMemcpyDeviceToHost, H->stream));
+  CK(cudaMemcpyAsync(H->hsum + kSumCap - 1, H->derr, sizeof(int), cudaMemcpyDeviceToHost, H->stream));
+  CK(cudaStreamSynchronize(H->stream));
+  int e;
+  memcpy(&e, H->hsum + kSumCap - 1, sizeof e);
+  return dev_error_status(H, e);
+}
+
+// Blocks and planes per block of the diagnostics that march down z: 16 planes,
+// or fewer until the grid fills the SMs a few times over.
+void march_grid(const cup_handle* H, int* zc, int* grid) {
+  const int per_plane = H->nx * H->ny / 256;
+  *zc = 16;
+  while (*zc > 4 && per_plane * (H->nz / *zc) < 4 * H->num_sms) *zc /= 2;
+  *grid = per_plane * (H->nz / *zc);
+}
+
+// The z transform of the three components in spec[0] with the mode sums.
+template <int M>
+int launch_z_modes_M(cup_handle* H, const ModeParams& mp, double* part, int* np) {
+  constexpr bool T8 = M == 128;
+  constexpr int N = 2 * M, W = 16;
+  CUtensorMap map;
+  int rc = make_map(H, &map, H->spec[0], tma_dtype<double>(), sizeof(double), W, 1, N, 3);
+  if (rc) return rc;
+  const size_t smem = (size_t)3 * N * W * sizeof(double) + FFTPlan<M>::table_len() * sizeof(double2) +
+                      mp.nbin * sizeof(double) + sizeof(uint64_t) + 128;
+  auto kern = k_dht_z_modes<M, T8>;
+  int bpsm = 0;
+  if ((rc = prepare_kernel(H, kern, smem, 128, &bpsm))) return rc;
+  const int ntiles = H->nx / W * H->ny;
+  *np = std::min({ntiles, bpsm * H->num_sms, kPartialCap / (3 + mp.nbin)});
+  return launch_named(H, "spectral_z_modes", [&]() -> int {
+    klaunch(H, kern, *np, 128, smem, map, mp, (const double2*)H->tw64[2], ntiles, part, H->derr);
+    CKL();
+    return CUP_OK;
+  });
+}
+int launch_z_modes(cup_handle* H, const ModeParams& mp, double* part, int* np) {
+  PFFT_DISPATCH(H->nz, (launch_z_modes_M<M>(H, mp, part, np)));
+}
+
+// The spectral sums of the current velocity (see k_dht_z_modes): raw[0..2]
 // = tke, lIntegral, tkeFiltered over the separable modes (unnormalised), raw[3]
 // = sum of |curl_c u|^2 over the cells; bins = the unnormalised spectrum
-// (nBin = max(N)/2 - 1 values, HITstatistics). filter: the coefficients in
-// spec[] keep only the forcing band afterwards.
-int do_spectral(cup_handle* H, bool filter, double raw[4], std::vector<double>& bins) {
-  if (!H->spec[0])
-    for (int c = 0; c < 3; ++c) CK(cudaMalloc(&H->spec[c], H->n * sizeof(double)));
-  const int grid = std::min<size_t>(H->num_sms * 4, (H->n + 255) / 256);
-  const void* f[3] = {H->u, H->v, H->w};
-  for (int c = 0; c < 3; ++c) {
-    int rc_ = launch_named(H, "spectral_widen", [&]() -> int {
-      if (H->fp32)
-        klaunch(H, k_widen<float>, grid, 256, 0, (const float*)f[c], H->spec[c], H->n);
-      else
-        klaunch(H, k_widen<double>, grid, 256, 0, (const double*)f[c], H->spec[c], H->n);
-      CKL();
-      return CUP_OK;
-    });
-    if (rc_) return rc_;
-    if ((rc_ = launch_rows_pipe(H, "spectral_dht_x", H->spec[c]))) return rc_;
-    if ((rc_ = launch_cols<1, false>(H, H->spec[c]))) return rc_;
-    if ((rc_ = launch_cols<2, false>(H, H->spec[c]))) return rc_;
+// (nBin = max(N)/2 - 1 values, HITstatistics). mp: the modes' parameters; with
+// mp.coef the coefficients of the forcing band are left there. spec[] then
+// holds the x and y transforms.
+int do_spectral(cup_handle* H, const ModeParams& mp, double raw[4], std::vector<double>& bins) {
+  int rc;
+  const char* nm = "spectral_dht_x";
+  if (H->fp32) {
+    const float* f[3] = {(const float*)H->u, (const float*)H->v, (const float*)H->w};
+    rc = launch_rows_pipe<float>(H, nm, f, 3, H->spec[0]);
+  } else {
+    const double* f[3] = {(const double*)H->u, (const double*)H->v, (const double*)H->w};
+    rc = launch_rows_pipe<double>(H, nm, f, 3, H->spec[0]);
   }
-  const int N = std::max(H->nx, std::max(H->ny, H->nz));
-  const int nyquist = N / 2, nbin = nyquist - 1;
-  const double wf[3] = {2.0 * M_PI / (H->nx * H->h), 2.0 * M_PI / (H->ny * H->h), 2.0 * M_PI / (H->nz * H->h)};
-  const double nyq_scaling = (nyquist - 1) / (double)nyquist;
-  const int stride = 3 + nbin;
-  if ((size_t)stride * grid > (size_t)kPartialCap) return fail(H, CUP_ERR_ARG, "spectrum too large for the partials");
+  int np = 0, zc, gv;
   double* part = partial(H, P_DIAG);
   double* pv = partial(H, P_RES);
-  {
-    int rc_ = launch_named(H, "spectral_modes", [&]() -> int {
-      klaunch(H, k_spectral_modes, grid, 256, nbin * sizeof(double), H->spec[0], H->spec[1], H->spec[2], H->nx, H->ny,
-                                                                        H->nz, wf[0], wf[1], wf[2], nyquist,
-                                                                        nyq_scaling, nbin, filter ? 1 : 0, part);
-      CKL();
-      return CUP_OK;
-    });
-    if (rc_) return rc_;
+  if (!rc) rc = launch_cols<1, false>(H, H->spec[0], 3);
+  if (!rc) rc = launch_z_modes(H, mp, part, &np);
+  if (rc) return rc;
+  march_grid(H, &zc, &gv);
+  rc = launch_named(H, "spectral_vorticity", [&]() -> int {
+    if (H->fp32)
+      klaunch(H, k_vorticity2<float>, gv, 256, 0, (const float*)H->u, (const float*)H->v, (const float*)H->w,
+              ilog2(H->nx), ilog2(H->ny), H->nz, zc, 0.5 / H->h, pv);
+    else
+      klaunch(H, k_vorticity2<double>, gv, 256, 0, (const double*)H->u, (const double*)H->v, (const double*)H->w,
+              ilog2(H->nx), ilog2(H->ny), H->nz, zc, 0.5 / H->h, pv);
+    CKL();
+    return CUP_OK;
+  });
+  if (!rc) rc = sum_columns(H, part, np, 3 + mp.nbin, -1, 0);
+  if (!rc) rc = sum_columns(H, pv, gv, 1, -1, 3 + mp.nbin);
+  if (!rc) rc = read_sums(H, 4 + mp.nbin);
+  if (rc) return rc;
+  for (int k = 0; k < 3; ++k) raw[k] = H->hsum[k];
+  raw[3] = H->hsum[3 + mp.nbin];
+  bins.assign(H->hsum + 3, H->hsum + 3 + mp.nbin);
+  return CUP_OK;
+}
+
+// The modes of the handle's grid; allocates the coefficient arrays on first use.
+int mode_params(cup_handle* H, ModeParams* mp) {
+  if (!H->spec[0]) {
+    CK(cudaMalloc(&H->spec[0], 3 * H->n * sizeof(double)));
+    H->spec[1] = H->spec[0] + H->n;
+    H->spec[2] = H->spec[1] + H->n;
+    CK(cudaMalloc(&H->band_coef, (size_t)3 * kBandN * kBandN * kBandN * sizeof(double)));
   }
-  {
-    int rc_ = launch_named(H, "spectral_vorticity", [&]() -> int {
-      if (H->fp32)
-        klaunch(H, k_vorticity2<float>, grid, 256, 0, (const float*)H->u, (const float*)H->v, (const float*)H->w,
-                                                          H->nx, H->ny, H->nz, 0.5 / H->h, pv);
-      else
-        klaunch(H, k_vorticity2<double>, grid, 256, 0, (const double*)H->u, (const double*)H->v,
-                                                           (const double*)H->w, H->nx, H->ny, H->nz, 0.5 / H->h, pv);
-      CKL();
-      return CUP_OK;
-    });
-    if (rc_) return rc_;
+  const int n[3] = {H->nx, H->ny, H->nz};
+  mp->nx = n[0], mp->ny = n[1], mp->nz = n[2];
+  mp->nyquist = std::max(H->nx, std::max(H->ny, H->nz)) / 2;
+  mp->nbin = mp->nyquist - 1;
+  mp->nyq_scaling = (mp->nyquist - 1) / (double)mp->nyquist;
+  for (int d = 0; d < 3; ++d) {
+    mp->wf[d] = 2.0 * M_PI / (n[d] * H->h);
+    // every mode with |i| wf <= 2 (one more index against rounding; its coefficients are zero)
+    mp->band[d] = (int)std::min((double)(n[d] / 2 - 1), std::floor(2.0 / mp->wf[d]) + 1);
   }
-  std::vector<double> hp((size_t)stride * grid), hv(grid);
-  CK(cudaMemcpyAsync(hp.data(), part, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, H->stream));
-  CK(cudaMemcpyAsync(hv.data(), pv, hv.size() * sizeof(double), cudaMemcpyDeviceToHost, H->stream));
-  CK(cudaStreamSynchronize(H->stream));
-  for (int k = 0; k < 4; ++k) raw[k] = 0.0;
-  bins.assign(nbin, 0.0);
-  for (int i = 0; i < grid; ++i) {
-    for (int k = 0; k < 3; ++k) raw[k] += hp[(size_t)stride * i + k];
-    for (int b = 0; b < nbin; ++b) bins[b] += hp[(size_t)stride * i + 3 + b];
-    raw[3] += hv[i];
-  }
-  return check_dev_error(H);
+  mp->coef = nullptr;
+  return CUP_OK;
 }
 
 // SpectralForcing::operator() (source/spectralOperators/SpectralForcing.cpp:23-86):
@@ -2077,12 +1946,20 @@ int do_spectral(cup_handle* H, bool filter, double raw[4], std::vector<double>& 
 // energy meets turbKinEn_target (or grows at enInjectionRate): u += fac/N H(H(u)
 // restricted to the band), fac = dt rate / (2 tke_band). out: totalKinEn,
 // largeModesKinEn, viscousDissip, dissipationRate, injectionRate, lIntegral.
+// A band of up to kBandMax modes a side (a box of side 2 pi has 2, and one more
+// index is carried) is summed mode by mode in one pass over the velocity (24
+// B/cell FP32, against nine FP64 transform passes and three updates); a wider
+// one (boxes of 4 pi and longer) goes through the inverse transforms.
 template <typename T>
 int do_spectral_forcing(cup_handle* H, double dt) {
   double raw[4];
   std::vector<double> bins;
-  int rc = do_spectral(H, true, raw, bins);
+  ModeParams mp;
+  int rc = mode_params(H, &mp);
   if (rc) return rc;
+  const bool small = std::max({mp.band[0], mp.band[1], mp.band[2]}) <= kBandMax;
+  if (small) mp.coef = H->band_coef;
+  if ((rc = do_spectral(H, mp, raw, bins))) return rc;
   const double NF = (double)H->n;  // normalizeFFT
   const double tke = raw[0] / (NF * NF), tkeF = raw[2] / (NF * NF);
   const double eps = H->cfg.nu * raw[3] / NF;
@@ -2097,25 +1974,42 @@ int do_spectral_forcing(cup_handle* H, double dt) {
   H->forcing_stats[3] = dissipationRate;
   H->forcing_stats[4] = rate;
   H->forcing_stats[5] = raw[0] > 0 ? raw[1] / raw[0] : 0.0;
-  if (fac > 0) {
-    H->forcing_prev_tke = tke + dt * rate;
-    void* f[3] = {H->u, H->v, H->w};
-    const int grid = std::min<size_t>(H->num_sms * 4, (H->n + 255) / 256);
-    for (int c = 0; c < 3; ++c) {
-      if ((rc = launch_rows_pipe(H, "spectral_dht_x", H->spec[c]))) return rc;
-      if ((rc = launch_cols<1, false>(H, H->spec[c]))) return rc;
-      if ((rc = launch_cols<2, false>(H, H->spec[c]))) return rc;
-      int rc_ = launch_named(H, "spectral_force", [&]() -> int {
-        klaunch(H, k_add_scaled<T>, grid, 256, 0, (T*)f[c], H->spec[c], fac / NF, H->n);
+  if (!(fac > 0)) {
+    H->forcing_prev_tke = tke;
+    return CUP_OK;
+  }
+  H->forcing_prev_tke = tke + dt * rate;
+  if (small) {
+    const int rpb = std::min(32, H->ny);
+    return launch_named(H, "spectral_force", [&]() -> int {
+      klaunch(H, k_force_band<T>, H->nz * (H->ny / rpb), 256, (size_t)rpb * 4 * kBandN * sizeof(double),
+              (T*)H->u, (T*)H->v, (T*)H->w, mp, fac / NF, rpb);
+      CKL();
+      return CUP_OK;
+    });
+  }
+  void* f[3] = {H->u, H->v, H->w};
+  const int grid = std::min<size_t>(H->num_sms * 4, (H->n + 255) / 256);
+  for (int c = 0; c < 3; ++c)
+    if ((rc = launch_cols<2, false>(H, H->spec[c]))) return rc;
+  rc = launch_named(H, "spectral_filter", [&]() -> int {
+    klaunch(H, k_spectral_filter, grid, 256, 0, H->spec[0], H->spec[1], H->spec[2], ilog2(H->nx), ilog2(H->ny), H->nz,
+            mp.wf[0], mp.wf[1], mp.wf[2]);
+    CKL();
+    return CUP_OK;
+  });
+  for (int c = 0; c < 3 && !rc; ++c) {
+    rc = launch_rows_pipe(H, "spectral_dht_x", H->spec[c]);
+    if (!rc) rc = launch_cols<1, false>(H, H->spec[c]);
+    if (!rc) rc = launch_cols<2, false>(H, H->spec[c]);
+    if (!rc)
+      rc = launch_named(H, "spectral_force", [&]() -> int {
+        klaunch(H, k_add_scaled<T>, grid, 256, 0, (T*)f[c], (const double*)H->spec[c], fac / NF, H->n);
         CKL();
         return CUP_OK;
       });
-      if (rc_) return rc_;
-    }
-  } else {
-    H->forcing_prev_tke = tke;
   }
-  return CUP_OK;
+  return rc;
 }
 
 // next_dt: finalize_step also computes the next step's CFL dt.
@@ -2722,7 +2616,7 @@ int cup_destroy(cup_handle* H) {
   cudaSetDevice(H->dev);
   if (H->stream) cudaStreamSynchronize(H->stream);
   drop_graph(H);
-  for (void* f : {H->aus, H->avs, H->aws, (void*)H->ab0, (void*)H->spec[0], (void*)H->spec[1], (void*)H->spec[2]})
+  for (void* f : {H->aus, H->avs, H->aws, (void*)H->ab0, (void*)H->spec[0], (void*)H->band_coef, (void*)H->dsum})
     if (f) cudaFree(f);
   for (void* f : {H->u, H->v, H->w, H->tu, H->tv, H->tw, H->u1, H->v1, H->w1, H->au, H->av, H->aw, (void*)H->p_adj,
                   H->chi, (void*)H->p, (void*)H->p_old, (void*)H->p_pred, (void*)H->rhs,
@@ -2732,6 +2626,7 @@ int cup_destroy(cup_handle* H) {
   prof_flush(H);
   for (cudaEvent_t e : H->ev_pool) cudaEventDestroy(e);
   if (H->hstate) cudaFreeHost(H->hstate);
+  if (H->hsum) cudaFreeHost(H->hsum);
   if (H->cap_stream) cudaStreamDestroy(H->cap_stream);
   if (H->own_stream && H->stream) cudaStreamDestroy(H->stream);
   delete H;
@@ -3511,35 +3406,28 @@ int cup_diagnostics(cup_handle* H, double out[3]) {
   REQUIRE_H(H);
   REQUIRE_WHOLE_GRID(H);
   if (!out) return fail(H, CUP_ERR_ARG, "null output");
-  const int grid = std::min<size_t>(H->num_sms * 4, (H->n + 255) / 256);
+  int zc, grid;
+  march_grid(H, &zc, &grid);
   double* part = partial(H, P_DIAG);
-  {
-    int rc_ = launch_named(H, "diag", [&]() -> int {
-      if (H->fp32)
-        klaunch(H, k_diag<float>, grid, 256, 0, (const float*)H->u, (const float*)H->v, (const float*)H->w, H->nx,
-                                                    H->ny, H->nz, 0.5 / H->h, part);
-      else
-        klaunch(H, k_diag<double>, grid, 256, 0, (const double*)H->u, (const double*)H->v, (const double*)H->w,
-                                                     H->nx, H->ny, H->nz, 0.5 / H->h, part);
-      CKL();
-      return CUP_OK;
-    });
-    if (rc_) return rc_;
-  }
-  std::vector<double> hp(3 * grid);
-  CK(cudaMemcpyAsync(hp.data(), part, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, H->stream));
-  CK(cudaStreamSynchronize(H->stream));
-  double ke = 0, d2 = 0, dm = 0;
-  for (int i = 0; i < grid; ++i) {
-    ke += hp[3 * i];
-    d2 += hp[3 * i + 1];
-    dm = std::max(dm, hp[3 * i + 2]);
-  }
+  int rc = launch_named(H, "diag", [&]() -> int {
+    if (H->fp32)
+      klaunch(H, k_diag<float>, grid, 256, 0, (const float*)H->u, (const float*)H->v, (const float*)H->w, ilog2(H->nx),
+              ilog2(H->ny), H->nz, zc, 0.5 / H->h, part);
+    else
+      klaunch(H, k_diag<double>, grid, 256, 0, (const double*)H->u, (const double*)H->v, (const double*)H->w,
+              ilog2(H->nx), ilog2(H->ny), H->nz, zc, 0.5 / H->h, part);
+    CKL();
+    return CUP_OK;
+  });
+  if (!rc) rc = sum_columns(H, part, grid, 3, 2, 0);
+  if (!rc) rc = read_sums(H, 3);
+  if (rc) return rc;
+  const double ke = H->hsum[0], d2 = H->hsum[1], dm = H->hsum[2];
   const double h3 = H->h * H->h * H->h;
   out[0] = ke * h3;
   out[1] = std::sqrt(d2 * h3);
   out[2] = dm;
-  return check_dev_error(H);
+  return CUP_OK;
 }
 
 int cup_spectral_analysis(cup_handle* H, double stats[7], double* spectrum, int nbin) {
@@ -3550,7 +3438,9 @@ int cup_spectral_analysis(cup_handle* H, double stats[7], double* spectrum, int 
   if (spectrum && nbin != N / 2 - 1) return fail(H, CUP_ERR_ARG, "spectrum needs max(N)/2 - 1 = %d bins", N / 2 - 1);
   double raw[4];
   std::vector<double> bins;
-  int rc = do_spectral(H, false, raw, bins);
+  ModeParams mp;
+  int rc = mode_params(H, &mp);
+  if (!rc) rc = do_spectral(H, mp, raw, bins);
   if (rc) return rc;
   const double NF = (double)H->n, nu = H->cfg.nu;
   const double tke = raw[0] / (NF * NF), eps = nu * raw[3] / NF;
@@ -3634,35 +3524,29 @@ int cup_compute_dissipation(cup_handle* H, double out[20]) {
   REQUIRE_H(H);
   REQUIRE_WHOLE_GRID(H);
   if (!out) return fail(H, CUP_ERR_ARG, "null output");
-  const int grid = std::min<size_t>(H->num_sms * 4, (H->n + 255) / 256);
+  int zc, grid;
+  march_grid(H, &zc, &grid);
   double* part = partial(H, P_DIAG);
   const double h = H->h;
   const double hCube = std::pow(h, 3), inv2h = .5 / h, invHh = 1 / (h * h);
   const double cx = H->nx * h / 2, cy = H->ny * h / 2, cz = H->nz * h / 2;  // extent / 2
-  {
-    int rc_ = launch_named(H, "dissipation", [&]() -> int {
-      if (H->fp32)
-        klaunch(H, k_dissipation<float>, grid, 256, 0, (const float*)H->u, (const float*)H->v, (const float*)H->w,
-                                                           H->p, H->has_sphere ? (const float*)H->chi : nullptr, H->nx,
-                                                           H->ny, H->nz, h, H->cfg.nu, hCube, inv2h, invHh, cx, cy, cz,
-                                                           part);
-      else
-        klaunch(H, k_dissipation<double>, grid, 256, 0, 
-            (const double*)H->u, (const double*)H->v, (const double*)H->w, H->p,
-            H->has_sphere ? (const double*)H->chi : nullptr, H->nx, H->ny, H->nz, h, H->cfg.nu, hCube, inv2h, invHh,
-            cx, cy, cz, part);
-      CKL();
-      return CUP_OK;
-    });
-    if (rc_) return rc_;
-  }
-  std::vector<double> hp(20 * (size_t)grid);
-  CK(cudaMemcpyAsync(hp.data(), part, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, H->stream));
-  CK(cudaStreamSynchronize(H->stream));
-  for (int k = 0; k < 20; ++k) out[k] = 0.0;
-  for (int i = 0; i < grid; ++i)
-    for (int k = 0; k < 20; ++k) out[k] += hp[20 * (size_t)i + k];
-  return check_dev_error(H);
+  int rc = launch_named(H, "dissipation", [&]() -> int {
+    if (H->fp32)
+      klaunch(H, k_dissipation<float>, grid, 256, 0, (const float*)H->u, (const float*)H->v, (const float*)H->w, H->p,
+              H->has_sphere ? (const float*)H->chi : nullptr, ilog2(H->nx), ilog2(H->ny), H->nz, zc, h, H->cfg.nu,
+              hCube, inv2h, invHh, cx, cy, cz, part);
+    else
+      klaunch(H, k_dissipation<double>, grid, 256, 0, (const double*)H->u, (const double*)H->v, (const double*)H->w,
+              H->p, H->has_sphere ? (const double*)H->chi : nullptr, ilog2(H->nx), ilog2(H->ny), H->nz, zc, h,
+              H->cfg.nu, hCube, inv2h, invHh, cx, cy, cz, part);
+    CKL();
+    return CUP_OK;
+  });
+  if (!rc) rc = sum_columns(H, part, grid, 20, -1, 0);
+  if (!rc) rc = read_sums(H, 20);
+  if (rc) return rc;
+  for (int k = 0; k < 20; ++k) out[k] = H->hsum[k];
+  return CUP_OK;
 }
 
 int cup_debug_shift(cup_handle* H, const double* f, double* out, int g, int dx, int dy, int dz, int where) {

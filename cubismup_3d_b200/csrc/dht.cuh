@@ -211,6 +211,15 @@ struct RowLinesPad {
     *reinterpret_cast<R2*>(base + l * pitch + 2 * (m + (m >> 3))) = v;
   }
 };
+// FP32 row lines read as FP64 (line l at base + l * pitch).
+struct RowLinesWiden {
+  const float* base;
+  int pitch;
+  __device__ __forceinline__ double2 ld(int l, int m) const {
+    const float2 v = *reinterpret_cast<const float2*>(base + l * pitch + 2 * m);
+    return make_double2(v.x, v.y);
+  }
+};
 // Column lines of a tile [n][W]: element n of line l at n*W + l.
 template <typename R>
 struct ColLines {
@@ -422,20 +431,21 @@ __device__ __forceinline__ void dht_post(const Acc& a, const R2* twp, int l, int
 // first stage's output when USE_PAD). Thread `t` of line `l`, M/8 per line.
 // The packed complex FFT stages of dht_lines (for M = 128 all but the last,
 // which dht_tail_to fuses with the even/odd split).
-template <int M, bool USE_PAD, typename R, class Acc, class P>
-__device__ __forceinline__ void fft_stages(const Acc& a, const P& pad, const typename Cplx<R>::T* tw, int l, int t,
-                                           bool active) {
+// in: where the first stage reads the line from (may share bytes with a, not with pad).
+template <int M, bool USE_PAD, typename R, class In, class Acc, class P>
+__device__ __forceinline__ void fft_stages(const In& in, const Acc& a, const P& pad, const typename Cplx<R>::T* tw,
+                                           int l, int t, bool active) {
   using R2 = typename Cplx<R>::T;
   using Pl = FFTPlan<M>;
   if constexpr (Pl::nstages == 1) {
-    fft_stage<M, 8, 1, true, R2>(a, a, tw, l, t, active);
+    fft_stage<M, 8, 1, true, R2>(in, a, tw, l, t, active);
   } else if constexpr (USE_PAD) {
-    fft_stage<M, 8, 1, false, R2>(a, pad, tw, l, t, active);
+    fft_stage<M, 8, 1, false, R2>(in, pad, tw, l, t, active);
     fft_stage<M, Pl::radix(1), 8, false, R2>(pad, a, tw + Pl::tw_off(1), l, t, active);
     if constexpr (Pl::nstages == 3 && M != 128)
       fft_stage<M, Pl::radix(2), 64, true, R2>(a, a, tw + Pl::tw_off(2), l, t, active);
   } else {
-    fft_stage<M, 8, 1, true, R2>(a, a, tw, l, t, active);
+    fft_stage<M, 8, 1, true, R2>(in, a, tw, l, t, active);
     fft_stage<M, Pl::radix(1), 8, true, R2>(a, a, tw + Pl::tw_off(1), l, t, active);
     if constexpr (Pl::nstages == 3 && M != 128)
       fft_stage<M, Pl::radix(2), 64, true, R2>(a, a, tw + Pl::tw_off(2), l, t, active);
@@ -529,7 +539,7 @@ __device__ __forceinline__ void dht_tail_to(const Acc& a, const AccO& ao, const 
 template <int M, bool USE_PAD, typename R, class Acc, class P, class Scale = NoScale>
 __device__ __forceinline__ void dht_lines(const Acc& a, const P& pad, const typename Cplx<R>::T* tw, int l, int t,
                                           bool active, const Scale& scale = Scale()) {
-  fft_stages<M, USE_PAD, R>(a, pad, tw, l, t, active);
+  fft_stages<M, USE_PAD, R>(a, a, pad, tw, l, t, active);
   dht_tail_to<M, R>(a, a, tw, l, t, active, scale);
 }
 
@@ -538,50 +548,51 @@ __device__ __forceinline__ void load_table(R2* dst, const R2* src, int n) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
+// Up to three input arrays of `rows` rows each, one after the other in the output.
+template <typename RIN>
+struct RowsIn {
+  const RIN* f[3];
+  int rows;
+};
+
 // Pipelined x pass: persistent CTAs walk tiles of lpc consecutive rows
-// (tile i of a CTA: rows (blockIdx.x + i gridDim.x) lpc ...) through NB
-// shared-memory buffers. The 1-D bulk loads of the next NB-1 tiles and the
-// bulk store of the previous tile overlap the transform of the current one;
-// the twiddle table is loaded once per CTA. (The 8-thread plan of the column
-// passes measured slower on rows: 16-strided stage-A writes need a padded
-// buffer and fewer threads share a row tile.)
-template <int M, typename R, int NB>
-__global__ void __launch_bounds__(256, 2) k_dht_rows_pipe(const R* __restrict__ in, R* __restrict__ out, int nrows,
-                                                          int lpc, const typename Cplx<R>::T* tw_g, int* err,
-                                                          const int* skip) {
+// (tile i of a CTA: rows (blockIdx.x + i gridDim.x) lpc ...; lpc divides
+// in.rows) through NB shared-memory buffers. The 1-D bulk loads of the next
+// NB-1 tiles and the bulk store of the previous tile overlap the transform of
+// the current one; the twiddle table is loaded once per CTA. FP32 input lands
+// in the upper half of its tile's buffer, which the first stage has read (a
+// block barrier) before FP64 values are written over it.
+template <int M, typename RIN, int NB>
+__global__ void __launch_bounds__(256, 2) k_dht_rows_pipe(const RowsIn<RIN> in, double* __restrict__ out, int nrows,
+                                                          int lpc, const double2* tw_g, int* err) {
   pdl_entry();
-  using R2 = typename Cplx<R>::T;
   static_assert(NB >= 2, "need at least two tile buffers");
-  if (skip && *skip) return;
   constexpr int N = 2 * M, TPL = M / 8;
   constexpr int TL = FFTPlan<M>::rows_table_len();
   constexpr bool PAD = FFTPlan<M>::nstages > 1;
   constexpr int PPITCH = 2 * (M + M / 8);
   extern __shared__ __align__(128) unsigned char smem_dyn[];
   unsigned char* smem_raw = smem_align128(smem_dyn);
-  R* bufs = reinterpret_cast<R*>(smem_raw);                 // NB * lpc * N
-  R* padb = bufs + (size_t)NB * lpc * N;                     // lpc * PPITCH
-  R2* tw = reinterpret_cast<R2*>(padb + (PAD ? (size_t)lpc * PPITCH : 0));
+  double* bufs = reinterpret_cast<double*>(smem_raw);        // NB * lpc * N
+  double* padb = bufs + (size_t)NB * lpc * N;                // lpc * PPITCH
+  double2* tw = reinterpret_cast<double2*>(padb + (PAD ? (size_t)lpc * PPITCH : 0));
   uint64_t* bar = reinterpret_cast<uint64_t*>(tw + TL);
   const int tid = threadIdx.x;
-  const int ntiles = (nrows + lpc - 1) / lpc;
+  const int ntiles = nrows / lpc;
   const int my = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+  const size_t in_off = (size_t)lpc * N * (sizeof(double) - sizeof(RIN));  // bytes
   if (tid == 0) {
     for (int b = 0; b < NB; ++b) mbar_init(&bar[b], 1);
     mbar_fence_init();
   }
   __syncthreads();
-  auto rows_of = [&](int i, int& row0, int& nr) {
-    row0 = (blockIdx.x + i * gridDim.x) * lpc;
-    nr = min(lpc, nrows - row0);
-  };
   auto issue = [&](int i) {
-    int row0, nr;
-    rows_of(i, row0, nr);
+    const int row0 = (blockIdx.x + i * gridDim.x) * lpc, f = row0 / in.rows;
     const int b = i % NB;
-    const uint32_t bytes = (uint32_t)((size_t)nr * N * sizeof(R));
+    const uint32_t bytes = (uint32_t)((size_t)lpc * N * sizeof(RIN));
     mbar_arrive_expect_tx(&bar[b], bytes);
-    bulk_load(bufs + (size_t)b * lpc * N, in + (size_t)row0 * N, bytes, &bar[b]);
+    bulk_load(reinterpret_cast<unsigned char*>(bufs + (size_t)b * lpc * N) + in_off,
+              in.f[f] + (size_t)(row0 - f * in.rows) * N, bytes, &bar[b]);
   };
   int issued = 0;
   if (tid == 0)
@@ -589,7 +600,7 @@ __global__ void __launch_bounds__(256, 2) k_dht_rows_pipe(const R* __restrict__ 
   load_table(tw, tw_g, TL);
   __syncthreads();
   const int l = tid / TPL, t = tid % TPL;
-  RowLinesPad<R> P{padb, PPITCH};
+  RowLinesPad<double> P{padb, PPITCH};
   bool ok = true;
   int done = 0;
   for (int i = 0; i < my; ++i) {
@@ -599,18 +610,22 @@ __global__ void __launch_bounds__(256, 2) k_dht_rows_pipe(const R* __restrict__ 
       bulk_wait_read<0>();
       issue(issued++);
     }
-    int row0, nr;
-    rows_of(i, row0, nr);
     const int b = i % NB;
     ok = __syncthreads_and(ok && mbar_wait(&bar[b], (i / NB) & 1, err));
     if (!ok) break;
-    R* rows = bufs + (size_t)b * lpc * N;
-    RowLines<R> A{rows, N};
-    dht_lines<M, PAD, R>(A, P, tw, l, t, l < nr);
+    double* rows = bufs + (size_t)b * lpc * N;
+    RowLines<double> A{rows, N};
+    if constexpr (sizeof(RIN) == 4) {
+      RowLinesWiden F{reinterpret_cast<const float*>(reinterpret_cast<unsigned char*>(rows) + in_off), N};
+      fft_stages<M, PAD, double>(F, A, P, tw, l, t, true);
+    } else {
+      fft_stages<M, PAD, double>(A, A, P, tw, l, t, true);
+    }
+    dht_tail_to<M, double>(A, A, tw, l, t, true, NoScale());
     fence_proxy_async_smem();
     __syncthreads();
     if (tid == 0) {
-      bulk_store(out + (size_t)row0 * N, rows, (uint32_t)((size_t)nr * N * sizeof(R)));
+      bulk_store(out + (size_t)(blockIdx.x + i * gridDim.x) * lpc * N, rows, (uint32_t)((size_t)lpc * N * sizeof(double)));
       bulk_commit();
     }
     done = i + 1;

@@ -91,3 +91,45 @@ def test_poisson_solve_of_device_arrays(oracle, cells, where):
     assert np.array_equal(sim.pressure(), p)
     assert np.array_equal(src.cpu().numpy(), rhs.ravel())
     sim.close()
+
+
+@pytest.mark.parametrize("cells", [(16, 16, 16), (32, 16, 64), (64, 128, 32), (256, 32, 16), (32, 16, 256)])
+@pytest.mark.parametrize("extent", [2 * np.pi, 5 * np.pi])
+def test_spectral_sums_and_forcing_band(oracle, cells, extent):
+    """Every line length of the mode-summing z pass, and the forcing of a band
+    summed mode by mode (side 2 pi) and through the transforms (side 5 pi)."""
+    nx, ny, nz = cells
+    nu, dt = 1e-2, 1e-2
+    u, v, w = (np.random.default_rng(k).standard_normal((nz, ny, nx)) for k in range(3))
+    tke0 = 0.5 * np.mean(u * u + v * v + w * w)
+    sim = make_sim(cells, extent, nu=nu, turbKinEn_target=1.3 * tke0)
+    sim.set_velocity(u, v, w)
+    got = sim.spectral_analysis()
+    ref, E, _ = oracle.spectral(u, v, w, sim.h, nu)
+    for k in ("tke", "eps", "uprime", "lambda", "Re_lambda", "l_integral", "tau_integral"):
+        assert got[k] == pytest.approx(ref[k], rel=1e-10), k
+    assert np.allclose(got["spectrum"], E, rtol=1e-9, atol=1e-13 * E.max())
+    op = sim.pipeline[2]
+    op(dt)
+    forced, st = oracle.spectral_forcing(u, v, w, sim.h, nu, dt, target_tke=1.3 * tke0)
+    for a, b in zip(sim.velocity(), forced):
+        assert rel_l2(a, b) < 1e-12
+    assert op.stats["largeModesKinEn"] == pytest.approx(st[1], rel=1e-10)
+    sim.close()
+
+
+@pytest.mark.parametrize("cells", [(16, 16, 16), (32, 64, 128), (256, 16, 32), (16, 256, 16)])
+def test_marching_diagnostics(oracle, cells):
+    """ComputeDissipation's sums and the divergence norms at several grids of the z march."""
+    nx, ny, nz = cells
+    sim = make_sim(cells, 2.0, nu=1e-3)
+    orc = oracle.OracleSim(*cells, 2.0, nu=1e-3, CFL=0.1, rampup=0, DLM=0.0, lambda_=1.0)
+    u = [0.5 * np.random.default_rng(k).standard_normal((nz, ny, nx)) for k in range(3)]
+    sim.set_velocity(*u)
+    orc.set_velocity(*u)
+    got, ref = np.array(list(sim.compute_dissipation().values())), orc.dissipation()
+    assert np.all(np.abs(got - ref) <= 1e-10 * np.abs(ref) + 1e-13 * np.abs(ref).max())
+    d, od = sim.diagnostics(), orc.diagnostics()
+    for k in ("ke", "div_l2", "div_max"):
+        assert d[k] == pytest.approx(od[k], rel=1e-12), k
+    sim.close()
