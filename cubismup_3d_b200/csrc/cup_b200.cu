@@ -92,15 +92,6 @@ __global__ void k_max_u(const T* u, const T* v, const T* w, size_t n, double ux,
   if (threadIdx.x == 0) partials[blockIdx.x] = m[0];
 }
 
-__global__ void k_finalize_max(const double* partials, int np, DevState* st) {
-  pdl_entry();
-  __shared__ double scratch[32];
-  double m[1] = {0.0};
-  for (int i = threadIdx.x; i < np; i += blockDim.x) m[0] = fmax(m[0], partials[i]);
-  block_reduce<1, true>(m, scratch);
-  if (threadIdx.x == 0) st->umax = m[0];
-}
-
 // Simulation::calcMaxTimestep (source/Simulation.cpp:403-424) on the device,
 // from st->umax and st->step.
 struct CflParams {
@@ -124,58 +115,89 @@ __device__ __forceinline__ void calc_dt_device(DevState* st, const CflParams& c)
   if (DLM > 0) st->lambda = DLM / dt;
 }
 
+// The maximum of np partials, and with next_dt the CFL time step from it.
 // step >= 0: the host's step counter, stored first (the ramp-up reads it).
-__global__ void k_calc_dt(DevState* st, double h, double nu, double CFL, int rampup, double DLM, int step = -1) {
+__global__ void k_finalize_max(const double* partials, int np, DevState* st, int next_dt, CflParams cfl, int step) {
+  pdl_entry();
+  __shared__ double scratch[32];
+  double m[1] = {0.0};
+  for (int i = threadIdx.x; i < np; i += blockDim.x) m[0] = fmax(m[0], partials[i]);
+  block_reduce<1, true>(m, scratch);
+  if (threadIdx.x == 0) {
+    st->umax = m[0];
+    if (step >= 0) st->step = step;
+    if (next_dt) calc_dt_device(st, cfl);
+  }
+}
+__global__ void k_calc_dt(DevState* st, CflParams cfl, int step) {
   pdl_entry();
   if (step >= 0) st->step = step;
-  calc_dt_device(st, CflParams{h, nu, CFL, rampup, DLM});
+  calc_dt_device(st, cfl);
 }
 
 // Host-side scalars into the device state without a pageable copy (which
 // would serialise the host with the stream): bit 1 dt (and lambda = DLM/dt
-// when DLM > 0), bit 2 lambda (when DLM <= 0), bit 4 step and time.
-enum { SET_DT = 1, SET_LAMBDA = 2, SET_CLOCK = 4 };
-__global__ void k_set_state(DevState* st, int what, double dt, double DLM, double lambda, int step, double time) {
+// when DLM > 0), bit 2 lambda (when DLM <= 0), bit 4 step and time; bit 8: then
+// the CFL time step (what k_calc_dt computes).
+enum { SET_DT = 1, SET_LAMBDA = 2, SET_CLOCK = 4, CALC_DT = 8 };
+__global__ void k_set_state(DevState* st, int what, double dt, double lambda, int step, double time, CflParams cfl) {
   pdl_entry();
   if (what & SET_DT) {
     st->dt = dt;
-    if (DLM > 0) st->lambda = DLM / dt;
+    if (cfl.DLM > 0) st->lambda = cfl.DLM / dt;
   }
-  if ((what & SET_LAMBDA) && !(DLM > 0)) st->lambda = lambda;
+  if ((what & SET_LAMBDA) && !(cfl.DLM > 0)) st->lambda = lambda;
   if (what & SET_CLOCK) {
     st->step = step;
     st->time = time;
   }
+  if (what & CALC_DT) calc_dt_device(st, cfl);
+}
+
+// Sum (or maximum) over np partials of one column by one warp; result in every
+// lane. Columns side by side instead of one block reduction after another: bound
+// by the latency of one block's loads and reduction; with the three merged
+// launches above 172 -> 167 us per FP32_DC step on 128x64x256.
+template <bool IS_MAX>
+__device__ __forceinline__ double warp_column(const double* p, int np, int stride, int col) {
+  double a = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x & 31; i < np; i += 32) {
+    const double x = p[(size_t)stride * i + col];
+    a = IS_MAX ? fmax(a, x) : a + x;
+  }
+  return IS_MAX ? warp_max(a) : warp_sum(a);
 }
 
 // End of step: umax (grid part outside the obstacle box, box part after
 // penalization), kinetic energy, force/torque; advances step and time.
 // next_dt: then the CFL time step of the next step (what k_calc_dt would
-// compute before it), saving its launch in a run of steps.
+// compute before it), saving its launch in a run of steps. 256 threads.
 __global__ void k_finalize_step(const double* pgrad, int ngrad, int gstride, int max_off, int ke_off,
                                 const double* ppen, int npen, DevState* st, double h3, int advance, int next_dt,
                                 CflParams cfl) {
   pdl_entry();
-  __shared__ double scratch[8 * 32];
-  double mx[1] = {0.0};
-  double s[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int i = threadIdx.x; i < ngrad; i += blockDim.x) {
-    mx[0] = fmax(mx[0], pgrad[gstride * i + max_off]);
-    s[6] += pgrad[gstride * i + ke_off];
+  // one warp per column: 0 the maximum, 1 the kinetic energy, 2-7 force and torque
+  __shared__ double s[8];
+  const int wid = threadIdx.x >> 5;
+  double v;
+  if (wid == 0) {
+    v = warp_column<true>(pgrad, ngrad, gstride, max_off);
+    if (npen > 0) v = fmax(v, warp_column<true>(ppen, npen, 8, 6));
+  } else if (wid == 1) {
+    v = warp_column<false>(pgrad, ngrad, gstride, ke_off);
+  } else {
+    v = warp_column<false>(ppen, npen, 8, wid - 2);
   }
-  for (int i = threadIdx.x; i < npen; i += blockDim.x) {
-    for (int k = 0; k < 6; ++k) s[k] += ppen[8 * i + k];
-    mx[0] = fmax(mx[0], ppen[8 * i + 6]);
-  }
-  block_reduce<7, false>(s, scratch);
-  block_reduce<1, true>(mx, scratch + 7 * 32);
+  if ((threadIdx.x & 31) == 0) s[wid] = v;
+  __syncthreads();
   if (threadIdx.x == 0) {
-    st->umax = mx[0];
-    st->ke = s[6] * h3;
+    st->umax = s[0];
+    st->ke = s[1] * h3;
     if (npen > 0) {
       for (int k = 0; k < 3; ++k) {
-        st->force[k] = s[k];
-        st->torque[k] = s[3 + k];
+        st->force[k] = s[2 + k];
+        st->torque[k] = s[5 + k];
       }
     }
     if (advance) {
@@ -186,19 +208,13 @@ __global__ void k_finalize_step(const double* pgrad, int ngrad, int gstride, int
   }
 }
 
-// Penalization-only finalize (operator-by-operator path).
-__global__ void k_finalize_pen(const double* ppen, int npen, DevState* st) {
+// Penalization-only finalize (operator-by-operator path); lambda as SET_LAMBDA. 192 threads.
+__global__ void k_finalize_pen(const double* ppen, int npen, DevState* st, double DLM, double lambda) {
   pdl_entry();
-  __shared__ double scratch[6 * 32];
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  for (int i = threadIdx.x; i < npen; i += blockDim.x)
-    for (int k = 0; k < 6; ++k) s[k] += ppen[8 * i + k];
-  block_reduce<6, false>(s, scratch);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; ++k) {
-      st->force[k] = s[k];
-      st->torque[k] = s[3 + k];
-    }
+  const int wid = threadIdx.x >> 5;
+  const double v = warp_column<false>(ppen, npen, 8, wid);
+  if ((threadIdx.x & 31) == 0) (wid < 3 ? st->force[wid] : st->torque[wid - 3]) = v;
+  if (threadIdx.x == 0 && !(DLM > 0)) st->lambda = lambda;
 }
 
 // PressureRHS correction factor (source/operators/PressureRHS.cpp:328-334).
@@ -220,9 +236,16 @@ __global__ void k_finalize_rhs_obstacle(const double* p, int np, DevState* st) {
   }
 }
 
-// Zeroes a field of es-byte elements (4: FP32, 8: FP64) on a box.
-__global__ void k_clear_box(void* f, size_t es, Box box, int nx, int ny, int nz) {
+// Zeroes a field of es-byte elements (4: FP32, 8: FP64) on a box, and moves the
+// sphere's position in the device parameters (stream-ordered).
+__global__ void k_clear_box(void* f, size_t es, Box box, int nx, int ny, int nz, SphereParams* sp, double px, double py,
+                            double pz) {
   pdl_entry();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sp->position[0] = px;
+    sp->position[1] = py;
+    sp->position[2] = pz;
+  }
   const long long n = box.count();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const int x = wrapi(box.lo[0] + (int)(i % box.n[0]), nx);
@@ -234,14 +257,6 @@ __global__ void k_clear_box(void* f, size_t es, Box box, int nx, int ny, int nz)
     else
       static_cast<double*>(f)[o] = 0.0;
   }
-}
-
-// The sphere's position in the device parameters (stream-ordered).
-__global__ void k_set_sphere_position(SphereParams* sp, double x, double y, double z) {
-  pdl_entry();
-  sp->position[0] = x;
-  sp->position[1] = y;
-  sp->position[2] = z;
 }
 
 // Grid centre of mass (source/operators/ObstaclesCreate.cpp:230-256) -> SphereParams.
@@ -367,13 +382,12 @@ __global__ void k_rigid_update(const double* partials, int np, SphereParams* sp,
 __global__ void k_finalize_residual(const double* p, int stride, int np, DevState* st, double tol, int k,
                                     int min_iter, int max_iter, double inv_class_cells) {
   pdl_entry();
-  __shared__ double scratch[18 * 32];
   if (k > 0 && st->converged) return;
-  double s[18];
-  for (int j = 0; j < 18; ++j) s[j] = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x)
-    for (int j = 0; j < 18; ++j) s[j] += p[(size_t)stride * i + j];
-  block_reduce<18, false>(s, scratch);
+  // one warp per sum (576 threads)
+  __shared__ double s[18];
+  const double v = warp_column<false>(p, np, stride, threadIdx.x >> 5);
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
+  __syncthreads();
   if (threadIdx.x == 0) {
     double res2, b2;
     if (k == 0) {
@@ -1437,7 +1451,7 @@ int launch_pzq(cup_handle* H, const char* name, double* pw, double* partials, co
 int launch_finalize_residual(cup_handle* H, const double* partials, int stride, int grid, int k) {
   const double inv_class = 8.0 / (double)H->n;
   return launch_named(H, "finalize_residual", [&]() -> int {
-    klaunch(H, k_finalize_residual, 1, 256, 0, partials, stride, grid, H->dstate, dc_tol(H), k, dc_min_iter(H),
+    klaunch(H, k_finalize_residual, 1, 18 * 32, 0, partials, stride, grid, H->dstate, dc_tol(H), k, dc_min_iter(H),
             dc_max_iter(H), inv_class);
     CKL();
     return CUP_OK;
@@ -1535,7 +1549,7 @@ int do_poisson_dc(cup_handle* H) {
     if ((rc = launch_stream<double, 1, 2, 4, 6>(H, "dc_residual", pf, op, &grid, k > 0 ? conv : nullptr))) return rc;
     {
       int rc_ = launch_named(H, "finalize_residual", [&]() -> int {
-        klaunch(H, k_finalize_residual, 1, 256, 0, partial(H, P_RES), 18, grid, H->dstate, tol, k, min_iter, max_iter,
+        klaunch(H, k_finalize_residual, 1, 18 * 32, 0, partial(H, P_RES), 18, grid, H->dstate, tol, k, min_iter, max_iter,
                 inv_class);
         CKL();
         return CUP_OK;
@@ -1651,8 +1665,13 @@ int do_surface_forces(cup_handle* H, double* part, int gb) {
   });
 }
 
+CflParams cfl_params(const cup_handle* H) {
+  return CflParams{H->h, H->cfg.nu, H->cfg.CFL, H->cfg.rampup, H->cfg.DLM};
+}
+
+// next_dt: then the CFL time step, for the host's step counter.
 template <typename T>
-int do_max_u(cup_handle* H) {
+int do_max_u(cup_handle* H, int next_dt = 0) {
   const int grid = std::min<size_t>(H->num_sms * 4, (H->n + 255) / 256);
   {
     int rc_ = launch_named(H, "max_u", [&]() -> int {
@@ -1665,7 +1684,8 @@ int do_max_u(cup_handle* H) {
   }
   {
     int rc_ = launch_named(H, "finalize_max", [&]() -> int {
-      klaunch(H, k_finalize_max, 1, 256, 0, partial(H, P_MAX), grid, H->dstate);
+      klaunch(H, k_finalize_max, 1, 256, 0, partial(H, P_MAX), grid, H->dstate, next_dt, cfl_params(H),
+              next_dt ? H->step : -1);
       CKL();
       return CUP_OK;
     });
@@ -1798,23 +1818,16 @@ int relocate_sphere(cup_handle* H) {
   {
     const Box old = H->box;
     const int gb = box_grid(old);
+    const double* pos = H->sphere.position;
     int rc_ = launch_named(H, "sphere_clear", [&]() -> int {
-      klaunch(H, k_clear_box, gb, kBoxThreads, 0, H->chi, es, old, H->nx, H->ny, H->nz);
+      klaunch(H, k_clear_box, gb, kBoxThreads, 0, H->chi, es, old, H->nx, H->ny, H->nz, H->sp_dev, pos[0], pos[1],
+              pos[2]);
       CKL();
       return CUP_OK;
     });
     if (rc_) return rc_;
   }
   sphere_box(H);
-  {
-    const double* pos = H->sphere.position;
-    int rc_ = launch_named(H, "sphere_position", [&]() -> int {
-      klaunch(H, k_set_sphere_position, 1, 1, 0, H->sp_dev, pos[0], pos[1], pos[2]);
-      CKL();
-      return CUP_OK;
-    });
-    if (rc_) return rc_;
-  }
   return build_sphere_chi(H);
 }
 
@@ -2052,7 +2065,7 @@ int do_step(cup_handle* H, DtArg dt, const double* lambda_dev, int advance, int 
       klaunch(H, k_finalize_step, 1, 256, 0, partial(H, P_GRAD), H->n_grad_partials, H->grad_stride,
                                             H->grad_max_off, H->grad_ke_off, partial(H, P_PEN), H->n_pen_partials,
                                             H->dstate, H->h * H->h * H->h, advance,
-                                            next_dt, CflParams{H->h, H->cfg.nu, H->cfg.CFL, H->cfg.rampup, H->cfg.DLM});
+                                            next_dt, cfl_params(H));
       CKL();
       return CUP_OK;
     });
@@ -2975,18 +2988,17 @@ int cup_calc_max_timestep(cup_handle* H, double* dt) {
     if (dt) *dt = H->dt;
     return CUP_OK;
   }
+  // (the device keeps its own step counter in sync with the host mirror)
   if (!H->umax_fresh) {
-    if ((rc = DISPATCH_T(H, do_max_u))) return rc;
+    if ((rc = DISPATCH_T(H, do_max_u, 1))) return rc;
     H->umax_fresh = true;
-  }
-  {
-    // the device keeps its own step counter in sync with the host mirror
-    int rc_ = launch_named(H, "calc_dt", [&]() -> int {
-      klaunch(H, k_calc_dt, 1, 1, 0, H->dstate, H->h, H->cfg.nu, H->cfg.CFL, H->cfg.rampup, H->cfg.DLM, H->step);
+  } else {
+    rc = launch_named(H, "calc_dt", [&]() -> int {
+      klaunch(H, k_calc_dt, 1, 1, 0, H->dstate, cfl_params(H), H->step);
       CKL();
       return CUP_OK;
     });
-    if (rc_) return rc_;
+    if (rc) return rc;
   }
   if ((rc = read_state(H))) return rc;
   H->dt = H->hstate->dt;
@@ -3106,19 +3118,11 @@ int cup_penalize(cup_handle* H, double dt, double force_torque[6]) {
     if (force_torque) std::fill(force_torque, force_torque + 6, 0.0);
     return CUP_OK;
   }
-  {
-    int rc_ = launch_named(H, "set_state", [&]() -> int {
-      klaunch(H, k_set_state, 1, 1, 0, H->dstate, SET_LAMBDA, 0.0, H->cfg.DLM, H->lambda, 0, 0.0);
-      CKL();
-      return CUP_OK;
-    });
-    if (rc_) return rc_;
-  }
   int rc = DISPATCH_T(H, do_penalize, DtArg{dt, nullptr}, (const double*)nullptr);
   if (rc) return rc;
   {
     int rc_ = launch_named(H, "finalize_pen", [&]() -> int {
-      klaunch(H, k_finalize_pen, 1, 256, 0, partial(H, P_PEN), H->n_pen_partials, H->dstate);
+      klaunch(H, k_finalize_pen, 1, 192, 0, partial(H, P_PEN), H->n_pen_partials, H->dstate, H->cfg.DLM, H->lambda);
       CKL();
       return CUP_OK;
     });
@@ -3167,7 +3171,7 @@ int cup_step(cup_handle* H, double dt, cup_step_stats* stats) {
   // device dt/lambda follow the host values for this step
   {
     int rc_ = launch_named(H, "set_dt", [&]() -> int {
-      klaunch(H, k_set_state, 1, 1, 0, H->dstate, SET_DT | SET_LAMBDA, dt, H->cfg.DLM, H->lambda, 0, 0.0);
+      klaunch(H, k_set_state, 1, 1, 0, H->dstate, SET_DT | SET_LAMBDA, dt, H->lambda, 0, 0.0, cfl_params(H));
       CKL();
       return CUP_OK;
     });
@@ -3313,16 +3317,16 @@ int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
     if ((rc = DISPATCH_T(H, do_max_u))) return rc;
     H->umax_fresh = true;
   }
-  {
-    int rc_ = launch_named(H, "set_state", [&]() -> int {
-      klaunch(H, k_set_state, 1, 1, 0, H->dstate, SET_LAMBDA | SET_CLOCK, 0.0, H->cfg.DLM, H->lambda, H->step,
-                                          H->time);
-      CKL();
-      return CUP_OK;
-    });
-    if (rc_) return rc_;
-  }
-  if ((H->has_sphere && H->sphere_moves) || H->forcing) {
+  // the clock, and the dt of the first step when the steps chain it on the device
+  const bool host_dt = (H->has_sphere && H->sphere_moves) || H->forcing;
+  rc = launch_named(H, "set_state", [&]() -> int {
+    klaunch(H, k_set_state, 1, 1, 0, H->dstate, SET_LAMBDA | SET_CLOCK | (host_dt || nsteps == 0 ? 0 : CALC_DT), 0.0,
+            H->lambda, H->step, H->time, cfl_params(H));
+    CKL();
+    return CUP_OK;
+  });
+  if (rc) return rc;
+  if (host_dt) {
     // a moving sphere's box follows its position on the host, and the
     // forcing's injection needs dt there: dt is read back every step
     // (calcMaxTimestep + timestep, as the reference runs them)
@@ -3335,15 +3339,7 @@ int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
     return CUP_OK;
   }
   for (int i = 0; i < nsteps;) {
-    // the dt of step i > 0 comes from the end of step i - 1
-    if (i == 0) {
-      int rc_ = launch_named(H, "calc_dt", [&]() -> int {
-        klaunch(H, k_calc_dt, 1, 1, 0, H->dstate, H->h, H->cfg.nu, H->cfg.CFL, H->cfg.rampup, H->cfg.DLM, -1);
-        CKL();
-        return CUP_OK;
-      });
-      if (rc_) return rc_;
-    }
+    // (the dt of step i > 0 comes from the end of step i - 1)
     // steady state: whole graphs of kGraphSteps steps, each computing the
     // next step's dt; the steps of the run's tail from one-step graphs (the
     // last one computes no next dt)
