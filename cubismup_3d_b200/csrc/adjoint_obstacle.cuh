@@ -107,7 +107,7 @@ __global__ void k_adj_penalize(T* lu, T* lv, T* lw, const T* su, const T* sv, co
 }
 
 // Per-CTA partials of sum over the corrected surface cells of b1 q.
-// rhs_sums: (S, positive, negative surface sums) and corr of the forward RHS.
+// rhs_sums: (S, positive, negative surface sums) and corr of the forward RHS; b0: on the box.
 template <typename T>
 __global__ void k_adj_rhs_sum(const double* q, const double* b0, const T* chi, Box box, int nx, int ny, int nz,
                               const double* rhs_sums, const double* corr, double* partials /* [gridDim.x] */) {
@@ -122,7 +122,7 @@ __global__ void k_adj_rhs_sum(const double* q, const double* b0, const T* chi, B
     const int y = wrapi(box.lo[1] + (int)((i / box.n[0]) % box.n[1]), ny);
     const int z = wrapi(box.lo[2] + (int)(i / ((long long)box.n[0] * box.n[1])), nz);
     const size_t o = gidx(x, y, z, nx, ny);
-    const double b1 = b0[o] - (double)chi[o] * b0[o];
+    const double b1 = b0[i] - (double)chi[o] * b0[i];
     if ((rs.sigma > 0 ? b1 > 0 : b1 < 0) && chi_surface(chi, x, y, z, nx, ny, nz)) acc[0] += b1 * q[o];
   }
   block_reduce<1, false>(acc, scratch);
@@ -145,7 +145,7 @@ __global__ void k_adj_rhs_apply(double* q, const double* b0, const T* chi, Box b
     const int y = wrapi(box.lo[1] + (int)((i / box.n[0]) % box.n[1]), ny);
     const int z = wrapi(box.lo[2] + (int)(i / ((long long)box.n[0] * box.n[1])), nz);
     const size_t o = gidx(x, y, z, nx, ny);
-    const double X = chi[o], B0 = b0[o], Q = q[o];
+    const double X = chi[o], B0 = b0[i], Q = q[o];
     const double b1 = B0 - X * B0;
     // weight of the cell in the corrected surface set: 1 inside it; 1/2 for
     // a surface b1 of exactly 0 that a perturbation can move (chi < 1), the

@@ -632,9 +632,9 @@ struct cup_handle {
   double sphere_quat[4] = {1, 0, 0, 0};      // Obstacle::quaternion
   SphereParams* sp_dev = nullptr;
   Box box{};
-  // FP32_DC with the sphere: the RHS's obstacle terms on the box (b2 - b0,
-  // box order) that the z-queue passes add to the b they recompute from u*,
-  // and the box array the obstacle kernels work on; box_cap: their length
+  // with the sphere: the RHS's obstacle terms on the box (b2 - b0, box order)
+  // that the passes forming b from u* add to it, and the box array the obstacle
+  // kernels work on; box_cap: their length
   double* box_delta = nullptr;
   double* box_b = nullptr;
   long long box_cap = 0;
@@ -662,7 +662,7 @@ struct cup_handle {
   double forcing_target = 0, forcing_rate = 0, forcing_prev_tke = 0;
   double forcing_stats[6] = {0, 0, 0, 0, 0, 0};
   // obstacle adjoint scratch: the velocity before penalization u** (T) and the
-  // RHS before its obstacle terms b0 (FP64), recomputed per adjoint step
+  // RHS before its obstacle terms b0 (FP64, on the box), recomputed per adjoint step
   void *aus = nullptr, *avs = nullptr, *aws = nullptr;
   double* ab0 = nullptr;
   // cup_run in steady state: kGraphSteps steps captured once as a CUDA graph
@@ -1073,8 +1073,9 @@ int launch_pfft_z(cup_handle* H, const char* name, T* in, double* out, const int
 }
 
 // First x pass of the FP64 solve on the RHS formed from f (RHS never stored).
+// box: plus the obstacle's terms on its box (H->box_delta).
 template <int M, typename T>
-int launch_pfft_x_rhs_M(cup_handle* H, const char* name, void* const* f, double* out, DtArg dt) {
+int launch_pfft_x_rhs_M(cup_handle* H, const char* name, void* const* f, double* out, DtArg dt, bool box) {
   constexpr int WARPS = 4;
   using Rw = PRows<M>;
   const size_t smem = (size_t)WARPS * Rw::ELEMS * sizeof(double) + M * sizeof(double2) + 128;
@@ -1085,14 +1086,15 @@ int launch_pfft_x_rhs_M(cup_handle* H, const char* name, void* const* f, double*
   const int ntiles = H->ny * H->nz / Rw::ROWS;
   return launch_named(H, name, [&]() -> int {
     klaunch(H, kern, (ntiles + WARPS - 1) / WARPS, 32 * WARPS, smem, (const T*)f[0], (const T*)f[1], (const T*)f[2], out,
-            dt, H->h, H->ny, H->nz, ntiles, (const double2*)H->ptw64[0]);
+            dt, H->h, H->ny, H->nz, ntiles, (const double2*)H->ptw64[0], H->box,
+            box ? (const double*)H->box_delta : nullptr);
     CKL();
     return CUP_OK;
   });
 }
 template <typename T>
-int launch_pfft_x_rhs(cup_handle* H, const char* name, void* const* f, double* out, DtArg dt) {
-  PFFT_DISPATCH(H->nx, (launch_pfft_x_rhs_M<M, T>(H, name, f, out, dt)));
+int launch_pfft_x_rhs(cup_handle* H, const char* name, void* const* f, double* out, DtArg dt, bool box) {
+  PFFT_DISPATCH(H->nx, (launch_pfft_x_rhs_M<M, T>(H, name, f, out, dt, box)));
 }
 
 // The passes of an FP64 solve after the first x pass, from `work` to `out`.
@@ -1306,16 +1308,12 @@ int do_advect_diffuse(cup_handle* H, DtArg dt) {
 }
 
 template <typename T>
-int do_pressure_rhs(cup_handle* H, DtArg dt, void* const* fields = nullptr, double* save_b0 = nullptr) {
+int do_pressure_rhs(cup_handle* H, DtArg dt) {
   int rc;
   const void* uvw[3] = {H->u, H->v, H->w};
-  if (fields)
-    for (int q = 0; q < 3; ++q) uvw[q] = fields[q];
   OpPressureRHS<T> op{H->rhs, dt, H->h, H->nx, H->ny};
   rc = launch_stream<T, 3, 1, 4, 4>(H, "pressure_rhs", uvw, op);
   if (rc) return rc;
-  // the RHS before its obstacle terms (the obstacle adjoint linearises them there)
-  if (save_b0) CK(cudaMemcpyAsync(save_b0, H->rhs, H->n * sizeof(double), cudaMemcpyDeviceToDevice, H->stream));
   if (H->has_sphere) {
     const int gb = box_grid(H->box);
     {
@@ -1348,16 +1346,21 @@ int do_pressure_rhs(cup_handle* H, DtArg dt, void* const* fields = nullptr, doub
   return CUP_OK;
 }
 
-// The sphere's RHS terms on its box for the FP32 defect correction: b0 of u*
+// The sphere's RHS terms on its box, for the passes that form b from u*: b0 of u*
 // on the box, the obstacle terms (bulk source, surface sums, correction) on
 // that box array, and H->box_delta = b2 - b0.
-template <typename T>
-int do_box_rhs_terms(cup_handle* H, DtArg dt) {
+// D: the type the velocity differences are formed in, as the pass that adds
+// box_delta does; f: the fields (u* of the step), save_b0: a copy of b0 on the box.
+// Against forming b as an array first (37 us at 256x128x128, then read again):
+// an obstacle gradient of 4 steps there 3.92 -> 3.78 ms.
+template <typename T, typename D>
+int do_box_rhs_terms(cup_handle* H, DtArg dt, void* const* f, double* save_b0 = nullptr) {
   if (H->box.count() > H->box_cap) return fail(H, CUP_ERR_STATE, "obstacle box larger than its buffers");
   const int gb = box_grid(H->box);
   int rc = launch_named(H, "box_rhs_obstacle", [&]() -> int {
-    klaunch(H, k_box_rhs_obstacle<T>, gb, kBoxThreads, 0, (const T*)H->u, (const T*)H->v, (const T*)H->w,
-            (const T*)H->chi, H->box, H->nx, H->ny, H->nz, dt, H->h, H->box_b, H->box_delta, partial(H, P_RHSOB));
+    klaunch(H, k_box_rhs_obstacle<T, D>, gb, kBoxThreads, 0, (const T*)f[0], (const T*)f[1], (const T*)f[2],
+            (const T*)H->chi, H->box, H->nx, H->ny, H->nz, dt, H->h, H->box_b, H->box_delta, save_b0,
+            partial(H, P_RHSOB));
     CKL();
     return CUP_OK;
   });
@@ -1562,16 +1565,25 @@ int do_poisson_dc(cup_handle* H) {
   return CUP_OK;
 }
 
-// FP64 solve with the RHS of the fields f computed inside the first x pass (no RHS array).
+// FP64 solve with the RHS of the fields f computed inside the first x pass (no
+// RHS array). box: with the obstacle's terms (after do_box_rhs_terms of f).
 template <typename T>
-int do_solve_rhs_of(cup_handle* H, const char* name_rhs, const char* name_x, void* const* f, double* out, DtArg dt) {
+int do_solve_rhs_of(cup_handle* H, const char* name_rhs, const char* name_x, void* const* f, double* out, DtArg dt,
+                    bool box = false) {
   if (H->spec_ny != H->ny) {
     const void* cf[3] = {f[0], f[1], f[2]};
     OpPressureRHS<T> op{H->rhs, dt, H->h, H->nx, H->ny};
     int rc = launch_stream<T, 3, 1, 4, 4>(H, "pressure_rhs", cf, op);
+    if (!rc && box)
+      rc = launch_named(H, "box_add", [&]() -> int {
+        klaunch(H, k_box_add, box_grid(H->box), kBoxThreads, 0, H->rhs, (const double*)H->box_delta, H->box, H->nx,
+                H->ny, H->nz);
+        CKL();
+        return CUP_OK;
+      });
     return rc ? rc : fft_poisson(H, H->rhs, out);
   }
-  int rc = launch_pfft_x_rhs<T>(H, name_rhs, f, H->rhs, dt);
+  int rc = launch_pfft_x_rhs<T>(H, name_rhs, f, H->rhs, dt, box);
   return rc ? rc : pfft_finish(H, name_x, H->rhs, out);
 }
 
@@ -2045,16 +2057,13 @@ int do_step(cup_handle* H, DtArg dt, const double* lambda_dev, int advance, int 
     // RHS, defect correction and gradient correction in z-queue passes. The
     // sphere's RHS terms need global sums over the RHS first: they are formed on
     // its box and added back by the passes, which recompute the rest of b from u*
-    if (H->has_sphere && (rc = do_box_rhs_terms<T>(H, dt))) return rc;
+    void* us[3] = {H->u, H->v, H->w};
+    if (H->has_sphere && (rc = do_box_rhs_terms<T, float>(H, dt, us))) return rc;
     if ((rc = do_pressure_dc_zq<T>(H, dt))) return rc;
   } else {
-    if (H->has_sphere) {
-      if ((rc = do_pressure_rhs<T>(H, dt))) return rc;
-      if ((rc = do_poisson(H))) return rc;
-    } else {
-      void* us[3] = {H->u, H->v, H->w};
-      if ((rc = do_solve_rhs_of<T>(H, "rhs_dht_x", "dht_x", us, H->p, dt))) return rc;
-    }
+    void* us[3] = {H->u, H->v, H->w};
+    if (H->has_sphere && (rc = do_box_rhs_terms<T, double>(H, dt, us))) return rc;
+    if ((rc = do_solve_rhs_of<T>(H, "rhs_dht_x", "dht_x", us, H->p, dt, H->has_sphere))) return rc;
     if ((rc = do_grad<T>(H, dt))) return rc;
   }
   // UpdateObstacles: the free dofs' velocities from the pre-penalization flow
@@ -2235,8 +2244,8 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
     if ((rc = launch_advect<T, 1, 4, 4, 2>(H, "adjoint_recompute_stage1", un, un, st1, dt))) return rc;
     if ((rc = launch_advect<T, 2, 4, 4, 2>(H, "adjoint_recompute_stage2", st1, un, us, dt))) return rc;
   }
-  if ((rc = do_pressure_rhs<T>(H, dt, us, H->ab0))) return rc;
-  if ((rc = fft_poisson(H, H->rhs, H->p_adj))) return rc;
+  if ((rc = do_box_rhs_terms<T, double>(H, dt, us, H->ab0))) return rc;
+  if ((rc = do_solve_rhs_of<T>(H, "adjoint_rhs_dht_x", "adjoint_dht_x", us, H->p_adj, dt, true))) return rc;
   if ((rc = launch_grad<T, false>(H, "adjoint_recompute_grad_p", us, us, H->p_adj, dt))) return rc;
   // 2. penalization and force
   const int gb = box_grid(H->box);
@@ -2813,7 +2822,7 @@ int cup_add_sphere(cup_handle* H, const cup_sphere* s) {
   }
   sp.lambda_factor = 1.0;
   sphere_box(H);
-  if (H->fp32) {
+  {
     // the box spans at most 2 (R + 3h) / h + 5 cells per axis wherever the sphere moves
     const int N[3] = {H->nx, H->ny, H->nz};
     long long cap = 1;
@@ -3260,7 +3269,7 @@ int cup_adjoint_step_obstacle(cup_handle* H, const void* un, const void* vn, con
   if (!H->ab0) {
     const size_t es = H->fp32 ? sizeof(float) : sizeof(double);
     for (void** f : {&H->aus, &H->avs, &H->aws}) CK(cudaMalloc(f, H->n * es));
-    CK(cudaMalloc(&H->ab0, H->n * sizeof(double)));
+    CK(cudaMalloc(&H->ab0, H->box_cap * sizeof(double)));
   }
   void* s3[3] = {const_cast<void*>(un), const_cast<void*>(vn), const_cast<void*>(wn)};
   void* l3[3] = {lu, lv, lw};

@@ -368,15 +368,30 @@ __device__ __forceinline__ double div_b(double facB, T dxy, T wzp, T wzm) {
   return facB * (double)(dxy + (wzp - wzm));
 }
 
-// The first half of the RHS obstacle terms on the box, for passes that
-// recompute b0 = KernelPressureRHS(u*) (source/operators/PressureRHS.cpp:51-76)
-// themselves: b0 at each box cell (in the operation order of the z-queue
-// passes' b from u*) into d, b1 = b0 - chi b0 into b (box [z][y][x] order), and
-// the partial sums of k_rhs_obstacle (bulk source, positive / negative surface
-// b1). k_rhs_obstacle_correct<T, true> then turns d into b2 - b0.
-template <typename T>
+// f += d on a box (d in box order).
+__global__ void k_box_add(double* f, const double* d, Box box, int nx, int ny, int nz) {
+  pdl_entry();
+  const long long n = box.count();
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const int x = wrapi(box.lo[0] + (int)(i % box.n[0]), nx);
+    const int y = wrapi(box.lo[1] + (int)((i / box.n[0]) % box.n[1]), ny);
+    const int z = wrapi(box.lo[2] + (int)(i / ((long long)box.n[0] * box.n[1])), nz);
+    f[gidx(x, y, z, nx, ny)] += d[i];
+  }
+}
+
+// The first half of the RHS obstacle terms on the box, for passes that form
+// b0 = KernelPressureRHS(u*) (source/operators/PressureRHS.cpp:51-76)
+// themselves: b0 at each box cell into d, b1 = b0 - chi b0 into b (box
+// [z][y][x] order), and the partial sums of k_rhs_obstacle (bulk source,
+// positive / negative surface b1). k_rhs_obstacle_correct<T, true> then turns d
+// into b2 - b0. D: b0 in the operation order of the pass that adds it back:
+// float as the z-queue passes (div_xy, div_b), double as k_pfft_x_rhs.
+// save_b0 (may be nullptr): b0 kept.
+template <typename T, typename D>
 __global__ void k_box_rhs_obstacle(const T* u, const T* v, const T* w, const T* chi, Box box, int nx, int ny, int nz,
-                                   DtArg dt, double h, double* b, double* d, double* partials /* [gridDim.x][3] */) {
+                                   DtArg dt, double h, double* b, double* d, double* save_b0,
+                                   double* partials /* [gridDim.x][3] */) {
   pdl_entry();
   __shared__ double scratch[3 * 32];
   const double facB = 0.5 * h * h / dt.get();
@@ -389,7 +404,11 @@ __global__ void k_box_rhs_obstacle(const T* u, const T* v, const T* w, const T* 
     const size_t oxp = gidx(wrapi(x + 1, nx), y, z, nx, ny), oxm = gidx(wrapi(x - 1, nx), y, z, nx, ny);
     const size_t oyp = gidx(x, wrapi(y + 1, ny), z, nx, ny), oym = gidx(x, wrapi(y - 1, ny), z, nx, ny);
     const size_t ozp = gidx(x, y, wrapi(z + 1, nz), nx, ny), ozm = gidx(x, y, wrapi(z - 1, nz), nx, ny);
-    const double b0 = div_b<T>(facB, div_xy<T>(u[oxp], u[oxm], v[oyp], v[oym]), w[ozp], w[ozm]);
+    double b0;
+    if constexpr (sizeof(D) == 4)
+      b0 = div_b<T>(facB, div_xy<T>(u[oxp], u[oxm], v[oyp], v[oym]), w[ozp], w[ozm]);
+    else
+      b0 = facB * ((double)u[oxp] - (double)u[oxm] + (double)v[oyp] - (double)v[oym] + (double)w[ozp] - (double)w[ozm]);
     const double X = chi[gidx(x, y, z, nx, ny)];
     const double dXx = (double)chi[oxp] - (double)chi[oxm];
     const double dXy = (double)chi[oyp] - (double)chi[oym];
@@ -402,6 +421,7 @@ __global__ void k_box_rhs_obstacle(const T* u, const T* v, const T* w, const T* 
     acc[2] -= bSurface * r * (r < 0);
     b[i] = r;
     d[i] = b0;
+    if (save_b0) save_b0[i] = b0;
   }
   block_reduce<3, false>(acc, scratch);
   if (threadIdx.x == 0)

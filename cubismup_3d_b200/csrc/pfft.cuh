@@ -607,12 +607,13 @@ __global__ void __launch_bounds__(32 * WARPS) k_pfft_x(const S* in, S* out, S* o
 // Forward x pass of the pressure RHS b = (h^2 / 2 dt) div u* (KernelPressureRHS,
 // source/operators/PressureRHS.cpp:51-76), which never goes to HBM: a thread
 // forms the elements m = t + R2 r of its row (cells 2m, 2m+1) from paired loads
-// of u, v, w, straight into stage A's registers.
-template <int M, typename T, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS) k_pfft_x_rhs(const T* __restrict__ u, const T* __restrict__ v_,
+// of u, v, w, straight into stage A's registers. bdelta (may be nullptr): the
+// obstacle's RHS terms on its box, added there.
+template <int M, typename T, int WARPS, int MINB = 1>
+__global__ void __launch_bounds__(32 * WARPS, MINB) k_pfft_x_rhs(const T* __restrict__ u, const T* __restrict__ v_,
                                                           const T* __restrict__ w, double* __restrict__ out, DtArg dt,
                                                           double h, int ny, int nz, int ntiles,
-                                                          const double2* tw_g) {
+                                                          const double2* tw_g, const Box box, const double* bdelta) {
   pdl_entry();
   using P = PPlan<M>;
   using Rw = PRows<M>;
@@ -645,6 +646,20 @@ __global__ void __launch_bounds__(32 * WARPS) k_pfft_x_rhs(const T* __restrict__
     const T2 vN = VN[m], vS = VS[m], wB = WB[m], wF = WF[m];
     a[r].x = fac * ((double)u0.y - uW + (double)vN.x - (double)vS.x + (double)wB.x - (double)wF.x);
     a[r].y = fac * (uE - (double)u0.x + (double)vN.y - (double)vS.y + (double)wB.y - (double)wF.y);
+  }
+  if (bdelta) {
+    int dy = y - box.lo[1], dz = z - box.lo[2];
+    dy += dy < 0 ? ny : 0;
+    dz += dz < 0 ? nz : 0;
+    if (dy < box.n[1] && dz < box.n[2]) {
+      const double* bd = bdelta + (size_t)box.n[0] * (dy + (size_t)box.n[1] * dz);
+#pragma unroll
+      for (int r = 0; r < P::R1; ++r) {
+        const int d0 = (2 * (t + P::R2 * r) - box.lo[0]) & (N - 1), d1 = (d0 + 1) & (N - 1);
+        if (d0 < box.n[0]) a[r].x += bd[d0];
+        if (d1 < box.n[0]) a[r].y += bd[d1];
+      }
+    }
   }
   prow_fwd<M>(a, reinterpret_cast<double2*>(buf) + l * M, tw, t);
   fence_proxy_async_smem();

@@ -133,3 +133,29 @@ def test_marching_diagnostics(oracle, cells):
     for k in ("ke", "div_l2", "div_max"):
         assert d[k] == pytest.approx(od[k], rel=1e-12), k
     sim.close()
+
+
+@pytest.mark.parametrize("cells,position,radius", [((64, 32, 32), (0.02, 0.49, 0.25), 0.1),  # box over the edges of x and y
+                                                   ((32, 16, 64), (0.3, 0.12, 0.99), 0.1),   # all of y, over the edge of z
+                                                   ((16, 16, 16), (0.5, 0.5, 0.9), 0.4)])    # all of every axis
+def test_sphere_rhs_terms_in_the_x_pass(cells, position, radius):
+    """The step adds the obstacle's RHS terms to the RHS that it forms inside
+    the first x pass; PressureRHS and PressureProjection go through an RHS
+    array. The two differ by the rounding of b: a few 1e-16 of u per step."""
+    from cubismup_3d_b200 import Sphere
+    u = [0.3 * c for c in np.random.default_rng(4).standard_normal((3, cells[2], cells[1], cells[0]))]
+    out = []
+    for fused in (True, False):
+        sim = make_sim(cells, 1.0, nu=1e-3, lambda_=1e6, bImplicitPenalization=True)
+        sim.add_obstacle(Sphere(radius=radius, position=position, enforcedVelocity=(1.0, 0.2, 0.0),
+                                bForcedInSimFrame=(True, True, True), bFixFrameOfRef=(True, True, True)))
+        sim.set_velocity(*u)
+        if fused:
+            sim.timestep(1e-3)
+        else:
+            for op in sim.pipeline[:6]:
+                op(1e-3)
+        out.append(sim.velocity())
+        sim.close()
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and rel_l2(a, b) < 1e-13
