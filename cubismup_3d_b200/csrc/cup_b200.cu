@@ -2183,9 +2183,10 @@ int launch_adjoint_f2_sized(cup_handle* H, const char* name, const void* const* 
 
 // The two transposed upwind3 stages of an FP32 adjoint step: mu = 1/2 S'(u1)^T
 // lam*, then lam = 1/2 lam* + S'(u^n)^T mu (lam* = the projected adjoint, in
-// lam on entry). 4-row tiles, a 3-deep ring and one pair per thread measured
-// best at 256^3: 1.235 ms per adjoint step against 1.52 ms with 2-row tiles
-// and a 4-deep ring, and 2.17 ms for the scalar kernels (k_adjoint_zq).
+// lam on entry). 4-row tiles and one pair per thread measured best at
+// 256^3: 1.235 ms per adjoint step against 1.52 ms with 2-row tiles, and 2.17
+// ms for the scalar kernels (k_adjoint_zq). The ring is 4 deep: two planes in
+// flight while a plane and the one before it are read.
 int adjoint_upwind_f32(cup_handle* H, void* const* un, void* const* st1, void* const* lam, void* const* mu, DtArg dt) {
   int rc;
   if ((rc = launch_adjoint_f2_sized<false, 4, 4, 1>(H, "adjoint_stage2", st1, lam, nullptr, mu, 0.0, 0.5, dt)))
