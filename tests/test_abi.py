@@ -92,3 +92,21 @@ def test_rollout_checkpoint_interval():
     assert checkpoint_interval(100, 50_000_000, 10 ** 9) == 8
     with pytest.raises(MemoryError):
         checkpoint_interval(100, 50_000_000, 10 ** 6)
+
+
+def test_auto_checkpoint_interval_uses_cached_memory(monkeypatch):
+    """K = 1 without asking the driver when torch's unused whole segments hold
+    every state; else the smallest K in half of the device's free memory."""
+    import types
+    import torch
+    from cubismup_3d_b200 import adjoint
+    sim = types.SimpleNamespace(sd=types.SimpleNamespace(device=0), shape=(10, 10, 10), storage_dtype=torch.float32)
+    asked = []
+    stats = {"reserved_bytes.all.current": 1000_000, "active_bytes.all.current": 800_000,
+             "inactive_split_bytes.all.current": 80_000}
+    monkeypatch.setattr(torch.cuda, "memory_stats", lambda d: stats)
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: asked.append(d) or (16 * 12_000, 1 << 30))
+    assert adjoint._auto_interval(sim, 10) == 1 and not asked     # 10 states of 12000 bytes: all of 120000
+    assert adjoint._auto_interval(sim, 11) == 2 and asked == [0]  # 6 checkpoints + 1 state in 96000
+    monkeypatch.setattr(torch.cuda, "memory_stats", lambda d: {})  # an allocator without these figures
+    assert adjoint._auto_interval(sim, 8) == 1 and len(asked) == 2
