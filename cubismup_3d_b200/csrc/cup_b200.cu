@@ -1843,14 +1843,17 @@ int relocate_sphere(cup_handle* H) {
   return build_sphere_chi(H);
 }
 
+constexpr int kSumCap = 256;  // doubles of dsum / hsum (a spectrum has at most 127 bins)
+int alloc_sums(cup_handle* H) {
+  if (!H->dsum) CK(cudaMalloc(&H->dsum, kSumCap * sizeof(double)));
+  if (!H->hsum) CK(cudaMallocHost(&H->hsum, kSumCap * sizeof(double)));
+  return CUP_OK;
+}
 // Column sums of per-CTA partials (max_col: that column's maximum) to
 // dsum[at..], stream-ordered.
-constexpr int kSumCap = 256;  // doubles of dsum / hsum (a spectrum has at most 127 bins)
 int sum_columns(cup_handle* H, const double* part, int np, int ncol, int max_col, int at) {
-  if (!H->dsum) {
-    CK(cudaMalloc(&H->dsum, kSumCap * sizeof(double)));
-    CK(cudaMallocHost(&H->hsum, kSumCap * sizeof(double)));
-  }
+  int rc = alloc_sums(H);
+  if (rc) return rc;
   return launch_named(H, "sum_columns", [&]() -> int {
     klaunch(H, k_reduce_columns, ncol, 256, 0, part, np, ncol, max_col, H->dsum + at);
     CKL();
@@ -1976,7 +1979,7 @@ int mode_params(cup_handle* H, ModeParams* mp) {
 // B/cell FP32, against nine FP64 transform passes and three updates); a wider
 // one (boxes of 4 pi and longer) goes through the inverse transforms.
 template <typename T>
-int do_spectral_forcing(cup_handle* H, double dt) {
+int do_spectral_forcing(cup_handle* H, DtArg step_dt) {
   double raw[4];
   std::vector<double> bins;
   ModeParams mp;
@@ -1984,7 +1987,19 @@ int do_spectral_forcing(cup_handle* H, double dt) {
   if (rc) return rc;
   const bool small = std::max({mp.band[0], mp.band[1], mp.band[2]}) <= kBandMax;
   if (small) mp.coef = H->band_coef;
+  // a dt chained on the device comes to the host with the sums: one
+  // synchronisation a step, where reading it before the step took a second one
+  // (the injection needs it, the advection before it does not)
+  if ((rc = alloc_sums(H))) return rc;
+  double* dt_host = H->hsum + kSumCap - 2;
+  if (step_dt.dev) CK(cudaMemcpyAsync(dt_host, step_dt.dev, sizeof(double), cudaMemcpyDeviceToHost, H->stream));
   if ((rc = do_spectral(H, mp, raw, bins))) return rc;
+  if (step_dt.dev) {
+    H->dt = *dt_host;
+    if (!(H->dt > 0)) return fail(H, CUP_ERR_ARG, "dt must be > 0");
+    if (H->cfg.DLM > 0) H->lambda = H->cfg.DLM / H->dt;
+  }
+  const double dt = step_dt.dev ? H->dt : step_dt.host;
   const double NF = (double)H->n;  // normalizeFFT
   const double tke = raw[0] / (NF * NF), tkeF = raw[2] / (NF * NF);
   const double eps = H->cfg.nu * raw[3] / NF;
@@ -2049,10 +2064,7 @@ int do_step(cup_handle* H, DtArg dt, const double* lambda_dev, int advance, int 
   }
   if ((rc = do_advect_diffuse<T>(H, dt))) return rc;
   // SpectralForcing follows AdvectionDiffusion (source/Simulation.cpp:330-340)
-  if (H->forcing) {
-    if (dt.dev) return fail(H, CUP_ERR_STATE, "spectral forcing needs the step's dt on the host");
-    if ((rc = do_spectral_forcing<T>(H, dt.host))) return rc;
-  }
+  if (H->forcing && (rc = do_spectral_forcing<T>(H, dt))) return rc;
   if constexpr (std::is_same<T, float>::value) {
     // RHS, defect correction and gradient correction in z-queue passes. The
     // sphere's RHS terms need global sums over the RHS first: they are formed on
@@ -3327,23 +3339,20 @@ int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
     if ((rc = DISPATCH_T(H, do_max_u))) return rc;
     H->umax_fresh = true;
   }
-  // the clock, and the dt of the first step when the steps chain it on the device
-  const bool host_dt = (H->has_sphere && H->sphere_moves) || H->forcing;
+  // the clock, and the dt of the first step; each step then ends with the next one's
   rc = launch_named(H, "set_state", [&]() -> int {
-    klaunch(H, k_set_state, 1, 1, 0, H->dstate, SET_LAMBDA | SET_CLOCK | (host_dt || nsteps == 0 ? 0 : CALC_DT), 0.0,
-            H->lambda, H->step, H->time, cfl_params(H));
+    klaunch(H, k_set_state, 1, 1, 0, H->dstate, SET_LAMBDA | SET_CLOCK | (nsteps ? CALC_DT : 0), 0.0, H->lambda, H->step,
+            H->time, cfl_params(H));
     CKL();
     return CUP_OK;
   });
   if (rc) return rc;
-  if (host_dt) {
-    // a moving sphere's box follows its position on the host, and the
-    // forcing's injection needs dt there: dt is read back every step
-    // (calcMaxTimestep + timestep, as the reference runs them)
+  if (H->has_sphere && H->sphere_moves) {
+    // a moving sphere's box follows its position on the host: dt is read back
+    // every step (calcMaxTimestep + timestep, as the reference runs them)
     for (int i = 0; i < nsteps; ++i) {
-      double dt = 0;
-      if ((rc = cup_calc_max_timestep(H, &dt))) return rc;
-      if ((rc = cup_step(H, dt, nullptr))) return rc;
+      if ((rc = read_state(H))) return rc;
+      if ((rc = cup_step(H, H->hstate->dt, nullptr))) return rc;
     }
     if (stats) return fill_stats(H, stats);
     return CUP_OK;
@@ -3363,16 +3372,22 @@ int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
       }
     }
     rc = DISPATCH_T(H, do_step, DtArg{0.0, &H->dstate->dt}, (const double*)&H->dstate->lambda, 1,
-                    i + 1 < nsteps ? 1 : 0);
+                    H->forcing || i + 1 < nsteps ? 1 : 0);
     if (rc) return rc;
     H->steps_run += 1;
+    if (H->forcing) {  // the host has this step's dt
+      H->step += 1;
+      H->time += H->dt;
+    }
     ++i;
   }
   if ((rc = read_state(H))) return rc;
   H->step = H->hstate->step;
   H->time = H->hstate->time;
-  H->dt = H->hstate->dt;
-  if (H->cfg.DLM > 0) H->lambda = H->hstate->lambda;
+  if (!H->forcing) {  // (with forcing, each step's injection has read them)
+    H->dt = H->hstate->dt;
+    if (H->cfg.DLM > 0) H->lambda = H->hstate->lambda;
+  }
   if (stats) return fill_stats(H, stats);
   return CUP_OK;
 }
@@ -3481,7 +3496,7 @@ int cup_spectral_forcing(cup_handle* H, double dt, double stats[6]) {
   if (!(dt > 0)) return fail(H, CUP_ERR_ARG, "dt must be > 0");
   reset_pressure_history(H);
   H->umax_fresh = false;
-  int rc = DISPATCH_T(H, do_spectral_forcing, dt);
+  int rc = DISPATCH_T(H, do_spectral_forcing, DtArg{dt, nullptr});
   if (rc) return rc;
   if (stats)
     for (int k = 0; k < 6; ++k) stats[k] = H->forcing_stats[k];
