@@ -23,46 +23,6 @@ struct DtArg {
   __device__ __forceinline__ double get() const { return dev ? *dev : host; }
 };
 
-// ---------------------------------------------------------------------------
-// KernelAdvectDiffuse (source/operators/AdvectionDiffusion.cpp:111-144):
-// central 2nd-order advection + 7-point diffusion, explicit Euler, into tmp.
-template <typename T>
-struct OpAdvectDiffuseRef {
-  T *ou, *ov, *ow;
-  DtArg dt;
-  double h, nu;
-  double uinf[3];
-  int nx, ny;
-  template <class C>
-  __device__ __forceinline__ void cell(const C& c, int x, int y, int gy, int gz, double* acc) const {
-    const double dtv = dt.get();
-    const T facA = (T)(-dtv / (2 * h));
-    const T facD = (T)((nu / h) * (dtv / h));
-    const T Lu = c.v(0, x, y, 0, 0, 0), Lv = c.v(1, x, y, 0, 0, 0), Lw = c.v(2, x, y, 0, 0, 0);
-    const T uE = c.v(0, x, y, 1, 0, 0), uW = c.v(0, x, y, -1, 0, 0), uN = c.v(0, x, y, 0, 1, 0),
-            uS = c.v(0, x, y, 0, -1, 0), uB = c.v(0, x, y, 0, 0, 1), uF = c.v(0, x, y, 0, 0, -1);
-    const T vE = c.v(1, x, y, 1, 0, 0), vW = c.v(1, x, y, -1, 0, 0), vN = c.v(1, x, y, 0, 1, 0),
-            vS = c.v(1, x, y, 0, -1, 0), vB = c.v(1, x, y, 0, 0, 1), vF = c.v(1, x, y, 0, 0, -1);
-    const T wE = c.v(2, x, y, 1, 0, 0), wW = c.v(2, x, y, -1, 0, 0), wN = c.v(2, x, y, 0, 1, 0),
-            wS = c.v(2, x, y, 0, -1, 0), wB = c.v(2, x, y, 0, 0, 1), wF = c.v(2, x, y, 0, 0, -1);
-    const T dudx = uE - uW, dvdx = vE - vW, dwdx = wE - wW;
-    const T dudy = uN - uS, dvdy = vN - vS, dwdy = wN - wS;
-    const T dudz = uB - uF, dvdz = vB - vF, dwdz = wB - wF;
-    const T u = Lu + (T)uinf[0], v = Lv + (T)uinf[1], w = Lw + (T)uinf[2];
-    const T duD = uN + uS + uE + uW + uF + uB - Lu * 6;
-    const T dvD = vN + vS + vE + vW + vF + vB - Lv * 6;
-    const T dwD = wN + wS + wE + wW + wF + wB - Lw * 6;
-    const T duA = u * dudx + v * dudy + w * dudz;
-    const T dvA = u * dvdx + v * dvdy + w * dvdz;
-    const T dwA = u * dwdx + v * dwdy + w * dwdz;
-    const size_t o = gidx(x, gy, gz, nx, ny);
-    ou[o] = Lu + facA * duA + facD * duD;
-    ov[o] = Lv + facA * dvA + facD * dvD;
-    ow[o] = Lw + facA * dwA + facD * dwD;
-  }
-  __device__ void finish(double*, double*) const {}
-};
-
 // Third-order upwind-biased first derivative (times 6h) by the sign of the
 // advecting velocity a: a > 0 -> (2f+1 + 3f0 - 6f-1 + f-2), else
 // (-f+2 + 6f+1 - 3f0 - 2f-1). Not in the reference snapshot, whose
@@ -72,50 +32,6 @@ template <typename T>
 __device__ __forceinline__ T up3(T a, T fm2, T fm1, T f0, T fp1, T fp2) {
   return a > (T)0 ? ((T)2 * fp1 + (T)3 * f0 - (T)6 * fm1 + fm2) : (-fp2 + (T)6 * fp1 - (T)3 * f0 - (T)2 * fm1);
 }
-
-// One RK2 (Heun) stage of upwind3 advection + 7-point diffusion:
-//   stage 1: out = f + dt A(f)
-//   stage 2: out = 0.5 (f^n + (f1 + dt A(f1)))      (f^n read point-wise)
-template <typename T, bool STAGE2>
-struct OpUpwind3Stage {
-  const T *bu, *bv, *bw;  // f^n, stage 2 only
-  T *ou, *ov, *ow;
-  DtArg dt;
-  double h, nu;
-  double uinf[3];
-  int nx, ny;
-  template <class C>
-  __device__ __forceinline__ void cell(const C& c, int x, int y, int gy, int gz, double* acc) const {
-    const double dtv = dt.get();
-    const T facA = (T)(-dtv / (6 * h));
-    const T facD = (T)((nu / h) * (dtv / h));
-    const T uu = c.v(0, x, y, 0, 0, 0) + (T)uinf[0];
-    const T vv = c.v(1, x, y, 0, 0, 0) + (T)uinf[1];
-    const T ww = c.v(2, x, y, 0, 0, 0) + (T)uinf[2];
-    const size_t o = gidx(x, gy, gz, nx, ny);
-    T* outs[3] = {ou, ov, ow};
-    const T* bases[3] = {bu, bv, bw};
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const T f0 = c.v(q, x, y, 0, 0, 0);
-      const T fxm2 = c.v(q, x, y, -2, 0, 0), fxm1 = c.v(q, x, y, -1, 0, 0), fxp1 = c.v(q, x, y, 1, 0, 0),
-              fxp2 = c.v(q, x, y, 2, 0, 0);
-      const T fym2 = c.v(q, x, y, 0, -2, 0), fym1 = c.v(q, x, y, 0, -1, 0), fyp1 = c.v(q, x, y, 0, 1, 0),
-              fyp2 = c.v(q, x, y, 0, 2, 0);
-      const T fzm2 = c.v(q, x, y, 0, 0, -2), fzm1 = c.v(q, x, y, 0, 0, -1), fzp1 = c.v(q, x, y, 0, 0, 1),
-              fzp2 = c.v(q, x, y, 0, 0, 2);
-      const T dx = up3(uu, fxm2, fxm1, f0, fxp1, fxp2);
-      const T dy = up3(vv, fym2, fym1, f0, fyp1, fyp2);
-      const T dz = up3(ww, fzm2, fzm1, f0, fzp1, fzp2);
-      const T lap = fyp1 + fym1 + fxp1 + fxm1 + fzm1 + fzp1 - f0 * 6;
-      const T adv = uu * dx + vv * dy + ww * dz;
-      const T t = f0 + facA * adv + facD * lap;
-      if (STAGE2) outs[q][o] = (T)0.5 * (bases[q][o] + t);
-      else outs[q][o] = t;
-    }
-  }
-  __device__ void finish(double*, double*) const {}
-};
 
 // KernelPressureRHS (source/operators/PressureRHS.cpp:51-76):
 // rhs = (h^2 / 2dt) (du/dx + dv/dy + dw/dz) with central differences, i.e.
