@@ -51,7 +51,7 @@ def kernel_bytes(name: str, fp32: bool) -> float:
         "upwind3_stage1": 6 * s,
         "upwind3_stage2": 9 * s,
         "pressure_rhs": 3 * s + 8,
-        "rhs_dht_x": 3 * s + 8,          # FP64: u* in, RHS rows transformed in smem, x-transform out
+        "rhs_dht_x": 3 * s + 8,          # FP64: u* in, RHS rows formed in registers, x-transform out
         "dht_x": 2 * w,
         "dht_y": 2 * w,
         "dht_z_solve": 2 * w,
