@@ -28,7 +28,9 @@
 // so the three components share them and a tap costs one FMA (about 50 FP64
 // instructions per cell); the neighbours swap weights with the sign of a, the
 // second upwind cell is one select (x: of its address). A thread's two columns
-// are two rows of one x (six row loads serve both).
+// are two rows of one x (six row loads serve both). SELECT: both one-sided
+// stencils instead, for runs that amplify rounding (amplifies_rounding in
+// cup_b200.cu has the rule and the figures).
 #pragma once
 
 #include "common.cuh"
@@ -73,12 +75,22 @@ __device__ __forceinline__ UpW<T> up_weights(T a, T absA, T facD) {
   return w;
 }
 
+// The pieces of the SELECT form, FP64, with every rounding spelled out: left to
+// the compiler, which products are fused depends on the code around them.
+// The one-sided difference of a's sign (up3).
+__device__ __forceinline__ double up3_rn(double a, double fm2, double fm1, double f0, double fp1, double fp2) {
+  const double p = __dadd_rn(__fma_rn(-6.0, fm1, __fma_rn(3.0, f0, __dmul_rn(2.0, fp1))), fm2);
+  const double n = __fma_rn(-2.0, fm1, __fma_rn(-3.0, f0, __fma_rn(6.0, fp1, -fp2)));
+  return a > 0.0 ? p : n;
+}
+
 // blockDim.x * CPT must equal TY * nx (<= 512 threads).
 // NXC: nx fixed at compile time (0: read from g); fixed, the stencil's
 // shared-memory offsets are immediates.
 // Columns of a thread: SCHEME 0, tid + i blockDim.x; upwind3, rows CPT (tid / nx) + i of x = tid % nx.
 // bu, bv, bw: u^n of stage 2 (else unused).
-template <typename T, int SCHEME, int TY, int NS, int CPT, int NXC = 0>
+// SELECT (upwind3): the update from both one-sided stencils and a select (up3).
+template <typename T, int SCHEME, int TY, int NS, int CPT, int NXC = 0, bool SELECT = false>
 __global__ void __launch_bounds__(512) k_advect_zq(const __grid_constant__ AdvectMaps maps, const StreamGeom g,
                                                   const T* __restrict__ bu, const T* __restrict__ bv,
                                                   const T* __restrict__ bw, T* __restrict__ ou, T* __restrict__ ov,
@@ -86,7 +98,7 @@ __global__ void __launch_bounds__(512) k_advect_zq(const __grid_constant__ Advec
                                                   double uy, double uz, int* err) {
   pdl_entry();
   constexpr int G = AdvectTraits<SCHEME>::G;
-  constexpr bool UP = SCHEME != 0, BASE = SCHEME == 2;
+  constexpr bool UP = SCHEME != 0, BASE = SCHEME == 2, TAPS = UP && !SELECT;
   constexpr int ROWS = TY + 2 * G;
   constexpr int Q = 2 * G + 1;
   // a G-row halo box starting at y0 - G (wrapped) stays inside [0, ny) only if y0 is a multiple of TY >= G
@@ -119,7 +131,7 @@ __global__ void __launch_bounds__(512) k_advect_zq(const __grid_constant__ Advec
     if constexpr (UP) cy[i] = CPT * cy[i] + i;
   }
   const double dtv = dt.get();
-  const T facA = (T)(SCHEME == 0 ? -dtv / (2 * h) : dtv / (6 * h));  // upwind3: the B of the weights over |a|
+  const T facA = (T)(SCHEME == 0 ? -dtv / (2 * h) : (TAPS ? dtv : -dtv) / (6 * h));  // TAPS: the B of the weights over |a|
   const T facD = (T)((nu / h) * (dtv / h));
   const T uinf[3] = {(T)ux, (T)uy, (T)uz};
 
@@ -173,7 +185,7 @@ __global__ void __launch_bounds__(512) k_advect_zq(const __grid_constant__ Advec
             for (int i = 0; i < CPT; ++i) {
               const T ww = qv[2][QC][i] + uinf[2];
               T outv[3];
-              if constexpr (UP) {
+              if constexpr (TAPS) {
                 const UpW<T> wz = up_weights(ww, facA, facD);
                 const T cz = (T)3 * wz.far - (T)2 * facD;
 #pragma unroll
@@ -190,9 +202,15 @@ __global__ void __launch_bounds__(512) k_advect_zq(const __grid_constant__ Advec
 #pragma unroll
                 for (int f = 0; f < 3; ++f) {
                   const T f0 = qv[f][QC][i];
-                  const T dz = qv[f][QP1][i] - qv[f][QM1][i];
                   const T lz = qv[f][QM1][i] + qv[f][QP1][i];
-                  outv[f] = f0 + part[f][i] + facA * (ww * dz) + facD * (lz - f0 * 6);
+                  if constexpr (UP) {
+                    const T dz = up3_rn(ww, qv[f][QM2][i], qv[f][QM1][i], f0, qv[f][QP1][i], qv[f][QP2][i]);
+                    const T s = __fma_rn(facA, __dmul_rn(ww, dz), __dadd_rn(f0, part[f][i]));
+                    outv[f] = __fma_rn(facD, __fma_rn(f0, -6.0, lz), s);
+                  } else {
+                    const T dz = qv[f][QP1][i] - qv[f][QM1][i];
+                    outv[f] = f0 + part[f][i] + facA * (ww * dz) + facD * (lz - f0 * 6);
+                  }
                 }
               }
               if constexpr (BASE) {
@@ -212,15 +230,17 @@ __global__ void __launch_bounds__(512) k_advect_zq(const __grid_constant__ Advec
             if constexpr (UP) {
               const int x = cx[0], r = G + cy[0];
               const int xm1 = (x - 1) & mask, xp1 = (x + 1) & mask, xm2 = (x - 2) & mask, xp2 = (x + 2) & mask;
-              UpW<T> wx[CPT], wy[CPT];
-              T cxy[CPT];
-              int xfar[CPT];
+              [[maybe_unused]] UpW<T> wx[CPT], wy[CPT];
+              [[maybe_unused]] T cxy[CPT];
+              [[maybe_unused]] int xfar[CPT];
+              if constexpr (TAPS) {
 #pragma unroll
-              for (int i = 0; i < CPT; ++i) {
-                wx[i] = up_weights(qv[0][QX][i] + uinf[0], facA, facD);
-                wy[i] = up_weights(qv[1][QX][i] + uinf[1], facA, facD);
-                cxy[i] = (T)3 * (wx[i].far + wy[i].far) - (T)4 * facD;
-                xfar[i] = wx[i].pos ? xm2 : xp2;
+                for (int i = 0; i < CPT; ++i) {
+                  wx[i] = up_weights(qv[0][QX][i] + uinf[0], facA, facD);
+                  wy[i] = up_weights(qv[1][QX][i] + uinf[1], facA, facD);
+                  cxy[i] = (T)3 * (wx[i].far + wy[i].far) - (T)4 * facD;
+                  xfar[i] = wx[i].pos ? xm2 : xp2;
+                }
               }
 #pragma unroll
               for (int f = 0; f < 3; ++f) {
@@ -233,13 +253,22 @@ __global__ void __launch_bounds__(512) k_advect_zq(const __grid_constant__ Advec
 #pragma unroll
                 for (int i = 0; i < CPT; ++i) {
                   const T* Fx = F + i * nx;
-                  T acc = cxy[i] * row[G + i] + wx[i].far * Fx[xfar[i]];
-                  acc += wx[i].m1 * Fx[xm1];
-                  acc += wx[i].p1 * Fx[xp1];
-                  acc += wy[i].far * (wy[i].pos ? row[i] : row[i + 4]);
-                  acc += wy[i].m1 * row[i + 1];
-                  acc += wy[i].p1 * row[i + 3];
-                  part[f][i] = acc;
+                  if constexpr (TAPS) {
+                    T acc = cxy[i] * row[G + i] + wx[i].far * Fx[xfar[i]];
+                    acc += wx[i].m1 * Fx[xm1];
+                    acc += wx[i].p1 * Fx[xp1];
+                    acc += wy[i].far * (wy[i].pos ? row[i] : row[i + 4]);
+                    acc += wy[i].m1 * row[i + 1];
+                    acc += wy[i].p1 * row[i + 3];
+                    part[f][i] = acc;
+                  } else {
+                    const T uu = qv[0][QX][i] + uinf[0], vv = qv[1][QX][i] + uinf[1];
+                    const T fxm1 = Fx[xm1], fxp1 = Fx[xp1], fym1 = row[i + 1], fyp1 = row[i + 3];
+                    const T dx = up3_rn(uu, Fx[xm2], fxm1, row[G + i], fxp1, Fx[xp2]);
+                    const T dy = up3_rn(vv, row[i], fym1, row[G + i], fyp1, row[i + 4]);
+                    const T adv = __fma_rn(uu, dx, __dmul_rn(vv, dy));
+                    part[f][i] = __fma_rn(facD, fyp1 + fym1 + fxp1 + fxm1, __dmul_rn(facA, adv));
+                  }
                 }
               }
             } else {

@@ -919,6 +919,25 @@ int launch_rows_pipe(cup_handle* H, const char* name, double* buf) {
   return launch_rows_pipe<double>(H, name, f, 1, buf);
 }
 
+// First Hartley x pass of the RHS formed from f (RHS never stored).
+template <int M, typename T>
+int launch_rows_rhs_M(cup_handle* H, const char* name, void* const* f, double* out, DtArg dt) {
+  constexpr int N = 2 * M, TPL = M / 8, lpc = 256 / TPL;
+  constexpr bool PAD = FFTPlan<M>::nstages > 1;
+  const size_t smem = (size_t)lpc * N * sizeof(double) + (PAD ? (size_t)lpc * 2 * (M + M / 8) * sizeof(double) : 0) +
+                      FFTPlan<M>::rows_table_len() * sizeof(double2) + 128;
+  auto kern = k_dht_rows_rhs<M, T>;
+  int bpsm = 0;
+  int rc = prepare_kernel(H, kern, smem, 256, &bpsm);
+  if (rc) return rc;
+  return launch_named(H, name, [&]() -> int {
+    klaunch(H, kern, H->ny * H->nz / lpc, 256, smem, (const T*)f[0], (const T*)f[1], (const T*)f[2], out, dt, H->h, H->ny,
+            H->nz, lpc, (const double2*)H->tw64[0]);
+    CKL();
+    return CUP_OK;
+  });
+}
+
 // Hartley y or z pass (z: with the spectral divide and the inverse when DIVIDE),
 // in place on buf; y: of nf fields one after the other.
 template <int M, int AXIS, bool DIVIDE>
@@ -1097,6 +1116,11 @@ int launch_pfft_x_rhs(cup_handle* H, const char* name, void* const* f, double* o
   PFFT_DISPATCH(H->nx, (launch_pfft_x_rhs_M<M, T>(H, name, f, out, dt, box)));
 }
 
+template <typename T>
+int launch_rows_rhs(cup_handle* H, const char* name, void* const* f, double* out, DtArg dt) {
+  PFFT_DISPATCH(H->nx, (launch_rows_rhs_M<M, T>(H, name, f, out, dt)));
+}
+
 // The passes of an FP64 solve after the first x pass, from `work` to `out`.
 int pfft_finish(cup_handle* H, const char* name_x, double* work, double* out, double* out2 = nullptr) {
   int rc;
@@ -1106,19 +1130,40 @@ int pfft_finish(cup_handle* H, const char* name_x, double* work, double* out, do
   return launch_pfft_x<double, PROW_INV>(H, name_x, work, out, out2, 1, nullptr);
 }
 
-// p = f . b over the three axes, FP64, the RHS in `work` (overwritten). A
-// handle whose z pass belongs to a pencil of a decomposed grid
-// (cup_set_spectral_window) runs the Hartley passes that the decomposed solve uses.
+// The same with Hartley passes.
+int hartley_finish(cup_handle* H, const char* name_x, double* work, double* out) {
+  int rc;
+  const double* f[1] = {work};
+  if ((rc = launch_cols<1, false>(H, work))) return rc;
+  if ((rc = launch_cols<2, true>(H, work))) return rc;
+  if ((rc = launch_cols<1, false>(H, work))) return rc;
+  return launch_rows_pipe<double>(H, name_x, f, 1, out);
+}
+
+// Whether a step of the handle's CFL number can be beyond its stability limit,
+// in FP64. Explicit diffusion and upwind3 damp the shortest wave by 12 nu dt / h^2
+// + 4 umax dt / h a step, which may not exceed 2, and dt = CFL min(h^2 / nu, h /
+// umax): with CFL <= 1/8 the step is stable whatever the flow. Beyond, a run
+// amplifies the rounding of its steps (at CFL 0.5 and nu = 0.01 on sides of 256
+// cells up to 1e9 times in 38 steps), so that any other order of the same
+// arithmetic shows in its FP64 results: the four taps of the upwind stages and
+// the packed transforms of the pressure, either alone, moved u by 1e-9 to 5e-7.
+// Such runs keep their arithmetic: the one-sided stencils of both signs
+// (k_advect_zq, SELECT) and the Hartley passes of dht.cuh for the pressure. An
+// upwind3 step takes 55 us then instead of 42 at 64^3, 146 instead of 117 at
+// 128^3, 975 instead of 780 at 256^3. FP32 runs take the same passes either way:
+// their order of arithmetic also depends on how their sums are split.
+bool amplifies_rounding(const cup_handle* H) { return !H->fp32 && H->cfg.CFL > 0.125; }
+
+// p = f . b over the three axes, FP64, the RHS in `work` (overwritten). Handles
+// whose steps can amplify rounding (amplifies_rounding) run the Hartley passes,
+// and one whose z pass belongs to a pencil of a decomposed grid
+// (cup_set_spectral_window) those that the decomposed solve uses.
 int fft_poisson(cup_handle* H, double* work, double* out) {
   int rc;
-  if (H->spec_ny != H->ny) {
+  if (H->spec_ny != H->ny || amplifies_rounding(H)) {
     if ((rc = launch_rows_pipe(H, "dht_x", work))) return rc;
-    if ((rc = launch_cols<1, false>(H, work))) return rc;
-    if ((rc = launch_cols<2, true>(H, work))) return rc;
-    if ((rc = launch_cols<1, false>(H, work))) return rc;
-    if ((rc = launch_rows_pipe(H, "dht_x", work))) return rc;
-    CK(cudaMemcpyAsync(out, work, H->n * sizeof(double), cudaMemcpyDeviceToDevice, H->stream));
-    return CUP_OK;
+    return hartley_finish(H, "dht_x", work, out);
   }
   if ((rc = launch_pfft_x<double, PROW_FWD>(H, "dht_x", work, work, nullptr, 0, nullptr))) return rc;
   return pfft_finish(H, "dht_x", work, out);
@@ -1179,7 +1224,7 @@ int read_state(cup_handle* H) {
 // the compile-time-nx kernels; other shapes the same kernel with runtime sizes.
 // (The planes per item stay a runtime count: unrolling a whole 20-plane item
 // measured slower for the FP64 stages than the 10-plane loop.)
-template <typename T, int SCHEME, int TY, int NS, int CPT, int NXC>
+template <typename T, int SCHEME, int TY, int NS, int CPT, int NXC, bool SELECT>
 int launch_advect_sized(cup_handle* H, const char* name, void* const* in, void* const* base, void* const* out,
                         DtArg dt) {
   constexpr int G = AdvectTraits<SCHEME>::G;
@@ -1194,7 +1239,7 @@ int launch_advect_sized(cup_handle* H, const char* name, void* const* in, void* 
   }
   if (NXC && NXC != H->nx) return fail(H, CUP_ERR_ARG, "advection specialisation mismatch");
   const size_t smem = advect_smem_bytes<T, SCHEME, TY, NS>(H->nx) + 128;
-  auto kern = k_advect_zq<T, SCHEME, TY, NS, CPT, NXC>;
+  auto kern = k_advect_zq<T, SCHEME, TY, NS, CPT, NXC, SELECT>;
   const int threads = cells / CPT;
   int bpsm = 0;
   int rc = prepare_kernel(H, kern, smem, threads, &bpsm);
@@ -1210,15 +1255,15 @@ int launch_advect_sized(cup_handle* H, const char* name, void* const* in, void* 
   });
 }
 
-template <typename T, int SCHEME, int TY, int NS, int CPT>
+template <typename T, int SCHEME, int TY, int NS, int CPT, bool SELECT = false>
 int launch_advect(cup_handle* H, const char* name, void* const* in, void* const* base, void* const* out, DtArg dt) {
   switch (H->nx) {
-    case 64: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 64>(H, name, in, base, out, dt);
-    case 128: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 128>(H, name, in, base, out, dt);
-    case 256: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 256>(H, name, in, base, out, dt);
+    case 64: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 64, SELECT>(H, name, in, base, out, dt);
+    case 128: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 128, SELECT>(H, name, in, base, out, dt);
+    case 256: return launch_advect_sized<T, SCHEME, TY, NS, CPT, 256, SELECT>(H, name, in, base, out, dt);
     default: break;
   }
-  return launch_advect_sized<T, SCHEME, TY, NS, CPT, 0>(H, name, in, base, out, dt);
+  return launch_advect_sized<T, SCHEME, TY, NS, CPT, 0, SELECT>(H, name, in, base, out, dt);
 }
 
 // Launches one packed-FP32 upwind3 stage (k_advect_zq_f2): `in` stencil
@@ -1277,6 +1322,13 @@ int upwind_stage2_f32(cup_handle* H, const char* name, void* const* in, void* co
   return launch_advect_f2_sized<true, 4, 6, 1>(H, name, in, base, out, dt);
 }
 
+// FP64 upwind3 stage (shared like the FP32 ones): `base` the stage-2 point-wise u^n.
+template <typename T, int STAGE>
+int upwind_stage_f64(cup_handle* H, const char* name, void* const* in, void* const* base, void* const* out, DtArg dt) {
+  if (amplifies_rounding(H)) return launch_advect<T, STAGE, 4, 4, 2, true>(H, name, in, base, out, dt);
+  return launch_advect<T, STAGE, 4, 4, 2>(H, name, in, base, out, dt);
+}
+
 template <typename T>
 int do_advect_diffuse(cup_handle* H, DtArg dt) {
   constexpr bool F32 = std::is_same<T, float>::value;
@@ -1295,8 +1347,8 @@ int do_advect_diffuse(cup_handle* H, DtArg dt) {
       if ((rc = upwind_stage1_f32(H, "upwind3_stage1", uvw, st1, dt))) return rc;
       rc = upwind_stage2_f32(H, "upwind3_stage2", st1, uvw, tmp, dt);
     } else {
-      if ((rc = launch_advect<T, 1, 4, 4, 2>(H, "upwind3_stage1", uvw, uvw, st1, dt))) return rc;
-      rc = launch_advect<T, 2, 4, 4, 2>(H, "upwind3_stage2", st1, uvw, tmp, dt);
+      if ((rc = upwind_stage_f64<T, 1>(H, "upwind3_stage1", uvw, uvw, st1, dt))) return rc;
+      rc = upwind_stage_f64<T, 2>(H, "upwind3_stage2", st1, uvw, tmp, dt);
     }
   }
   if (rc) return rc;
@@ -1570,6 +1622,11 @@ int do_poisson_dc(cup_handle* H) {
 template <typename T>
 int do_solve_rhs_of(cup_handle* H, const char* name_rhs, const char* name_x, void* const* f, double* out, DtArg dt,
                     bool box = false) {
+  if constexpr (std::is_same<T, double>::value)
+    if (amplifies_rounding(H) && H->spec_ny == H->ny && !box) {
+      int rc = launch_rows_rhs<T>(H, name_rhs, f, H->rhs, dt);
+      return rc ? rc : hartley_finish(H, name_x, H->rhs, out);
+    }
   if (H->spec_ny != H->ny) {
     const void* cf[3] = {f[0], f[1], f[2]};
     OpPressureRHS<T> op{H->rhs, dt, H->h, H->nx, H->ny};
@@ -2074,8 +2131,13 @@ int do_step(cup_handle* H, DtArg dt, const double* lambda_dev, int advance, int 
     if ((rc = do_pressure_dc_zq<T>(H, dt))) return rc;
   } else {
     void* us[3] = {H->u, H->v, H->w};
-    if (H->has_sphere && (rc = do_box_rhs_terms<T, double>(H, dt, us))) return rc;
-    if ((rc = do_solve_rhs_of<T>(H, "rhs_dht_x", "dht_x", us, H->p, dt, H->has_sphere))) return rc;
+    if (H->has_sphere && amplifies_rounding(H)) {
+      if ((rc = do_pressure_rhs<T>(H, dt))) return rc;
+      if ((rc = do_poisson(H))) return rc;
+    } else {
+      if (H->has_sphere && (rc = do_box_rhs_terms<T, double>(H, dt, us))) return rc;
+      if ((rc = do_solve_rhs_of<T>(H, "rhs_dht_x", "dht_x", us, H->p, dt, H->has_sphere))) return rc;
+    }
     if ((rc = do_grad<T>(H, dt))) return rc;
   }
   // UpdateObstacles: the free dofs' velocities from the pre-penalization flow
@@ -2222,7 +2284,7 @@ int do_adjoint_step(cup_handle* H, void* const* un, void* const* lam, DtArg dt) 
     if ((rc = upwind_stage1_f32(H, "adjoint_recompute_stage1", un, st1, dt))) return rc;
     return adjoint_upwind_f32(H, un, st1, lam, mu, dt);
   } else {
-    if ((rc = launch_advect<T, 1, 4, 4, 2>(H, "adjoint_recompute_stage1", un, un, st1, dt))) return rc;
+    if ((rc = upwind_stage_f64<T, 1>(H, "adjoint_recompute_stage1", un, un, st1, dt))) return rc;
     if ((rc = launch_adjoint<T, 1, false, 2, 3, 1>(H, "adjoint_stage2", st1, lam, nullptr, mu, 0.0, 0.5, dt))) return rc;
     return launch_adjoint<T, 1, true, 2, 3, 1>(H, "adjoint_stage1", un, mu, lam, lam, 0.5, 1.0, dt);
   }
@@ -2254,8 +2316,8 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
     if ((rc = upwind_stage1_f32(H, "adjoint_recompute_stage1", un, st1, dt))) return rc;
     if ((rc = upwind_stage2_f32(H, "adjoint_recompute_stage2", st1, un, us, dt))) return rc;
   } else {
-    if ((rc = launch_advect<T, 1, 4, 4, 2>(H, "adjoint_recompute_stage1", un, un, st1, dt))) return rc;
-    if ((rc = launch_advect<T, 2, 4, 4, 2>(H, "adjoint_recompute_stage2", st1, un, us, dt))) return rc;
+    if ((rc = upwind_stage_f64<T, 1>(H, "adjoint_recompute_stage1", un, un, st1, dt))) return rc;
+    if ((rc = upwind_stage_f64<T, 2>(H, "adjoint_recompute_stage2", st1, un, us, dt))) return rc;
   }
   if ((rc = do_box_rhs_terms<T, double>(H, dt, us, H->ab0))) return rc;
   if ((rc = do_solve_rhs_of<T>(H, "adjoint_rhs_dht_x", "adjoint_dht_x", us, H->p_adj, dt, true))) return rc;

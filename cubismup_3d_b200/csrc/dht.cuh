@@ -2,9 +2,10 @@
 // Poisson solve (cup_poisson_pass, the device replacement of
 // PoissonSolverPeriodic's FFTW-MPI r2c / _solve / c2r,
 // source/poisson/PoissonSolverPeriodic.cpp:15-146) and of the spectral analysis
-// and forcing, which need the coefficients themselves. (The solve of a whole
-// grid runs the packed transforms of pfft.cuh, whose bins mix the even and odd
-// cells and are of no use to a caller.)
+// and forcing, which need the coefficients themselves, and of the FP64 solves
+// whose rounding is kept (amplifies_rounding in cup_b200.cu). (The other solves
+// of a whole grid run the packed transforms of pfft.cuh, whose bins mix the even
+// and odd cells and are of no use to a caller.)
 //
 // p = H(f . H(b)) with H the separable real Hartley transform
 // H[k] = Re X[k] - Im X[k] (X the unnormalised DFT) applied along x, y and z,
@@ -772,6 +773,45 @@ __global__ void __launch_bounds__(W * (T8 ? 8 : M / 8)) k_dht_cols_pipe(const __
     // after a timed-out wait: bounded drain of the loads still in flight
     if (!ok)
       for (int r = done; r < issued; ++r) mbar_wait(&bar[r % NB], (r / NB) & 1, nullptr);
+  }
+}
+
+// x pass of the pressure RHS b = (h^2 / 2 dt) div u* (KernelPressureRHS,
+// source/operators/PressureRHS.cpp:51-76), formed in the rows' shared memory:
+// lpc rows per CTA of 256 threads, nrows a multiple of lpc.
+template <int M, typename T>
+__global__ void __launch_bounds__(256) k_dht_rows_rhs(const T* __restrict__ u, const T* __restrict__ v,
+                                                      const T* __restrict__ w, double* __restrict__ out, DtArg dt,
+                                                      double h, int ny, int nz, int lpc, const double2* tw_g) {
+  pdl_entry();
+  constexpr int N = 2 * M, TPL = M / 8, TL = FFTPlan<M>::rows_table_len(), PPITCH = 2 * (M + M / 8);
+  constexpr bool PAD = FFTPlan<M>::nstages > 1;
+  extern __shared__ __align__(128) unsigned char smem_dyn[];
+  unsigned char* smem_raw = smem_align128(smem_dyn);
+  double* rows = reinterpret_cast<double*>(smem_raw);  // lpc * N
+  double* padb = rows + (size_t)lpc * N;               // lpc * PPITCH
+  double2* tw = reinterpret_cast<double2*>(padb + (PAD ? (size_t)lpc * PPITCH : 0));
+  const int row0 = blockIdx.x * lpc;
+  load_table(tw, tw_g, TL);
+  const double fac = 0.5 * h * h / dt.get();
+  for (int i = threadIdx.x; i < lpc * N; i += blockDim.x) {
+    const int l = i / N, x = i - l * N;
+    const int r = row0 + l, y = r % ny, z = r / ny;
+    const double uE = u[gidx((x + 1) & (N - 1), y, z, N, ny)], uW = u[gidx((x - 1) & (N - 1), y, z, N, ny)];
+    const double vN = v[gidx(x, wrapi(y + 1, ny), z, N, ny)], vS = v[gidx(x, wrapi(y - 1, ny), z, N, ny)];
+    const double wB = w[gidx(x, y, wrapi(z + 1, nz), N, ny)], wF = w[gidx(x, y, wrapi(z - 1, nz), N, ny)];
+    rows[i] = fac * (uE - uW + vN - vS + wB - wF);
+  }
+  __syncthreads();
+  RowLines<double> A{rows, N};
+  RowLinesPad<double> P{padb, PPITCH};
+  dht_lines<M, PAD, double>(A, P, tw, threadIdx.x / TPL, threadIdx.x % TPL, true);
+  fence_proxy_async_smem();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    bulk_store(out + (size_t)row0 * N, rows, (uint32_t)((size_t)lpc * N * sizeof(double)));
+    bulk_commit();
+    bulk_wait_all();
   }
 }
 

@@ -159,3 +159,50 @@ def test_sphere_rhs_terms_in_the_x_pass(cells, position, radius):
         sim.close()
     for a, b in zip(*out):
         assert np.isfinite(a).all() and rel_l2(a, b) < 1e-13
+
+
+@pytest.mark.parametrize("cells", [(256, 16, 16), (16, 16, 256), (64, 256, 32)])
+def test_run_beyond_the_stability_limit_keeps_its_rounding(cells):
+    """38 FP64 upwind3 steps at CFL 0.5 with 12 nu dt / h^2 above 2: the run
+    amplifies the rounding of its steps more than 1e9 times, so its results are
+    those of one order of arithmetic only. The golden file holds the 1D factors
+    of the initial velocity (the products below are exact in their order) and
+    512 velocity values of the library before it had a second form of the FP64
+    upwind3 stages and of the pressure solve; the second form is 1e-7 to 1e-3
+    away. Equal arithmetic gives equal bits; 1e-9 is what FP64 results are held to."""
+    import os
+    g = np.load(os.path.join(os.path.dirname(__file__), "golden", "amplified_rounding_fp64.npz"))
+    sx, sy, sz = (g[f"sin{n}"] for n in cells)
+    cx, cy, cz = (g[f"cos{n}"] for n in cells)
+
+    def p(a, b, c):
+        return c[:, None, None] * b[None, :, None] * a[None, None, :]
+
+    u0 = (p(sx, cy, cz) + 0.0625 * p(cx, sy, sz), -p(cx, sy, cz) + 0.0625 * p(sx, sy, cz), 0.0625 * p(sx, cy, sz))
+    sim = make_sim(cells, 2 * np.pi, nu=0.01, CFL=0.5, scheme="upwind3_rk2")
+    sim.set_velocity(*u0)
+    sim.run_steps(38)
+    key = "x".join(map(str, cells))
+    got = np.stack(sim.velocity()).ravel()[g["at" + key]]
+    assert rel_l2(got, g["u" + key]) < 1e-9
+    sim.close()
+
+
+@pytest.mark.parametrize("cells", LINES)
+@pytest.mark.parametrize("scheme", ["upwind3_rk2", "ref"])
+def test_step_of_both_stability_ranges_every_line_length(oracle, cells, scheme):
+    """One FP64 step of a CFL number above 1/8 (Hartley passes, RHS formed in
+    the x pass, one-sided stencils of both signs) and of one below, with the
+    same dt, against the oracle: a few hundred roundings of u and p each."""
+    nx, ny, nz = cells
+    u = np.random.default_rng(sum(cells)).standard_normal((3, nz, ny, nx))
+    for CFL in (0.125, 0.13):
+        sim = make_sim(cells, 2.0, nu=1e-3, CFL=CFL, scheme=scheme)
+        orc = oracle.OracleSim(*cells, 2.0, nu=1e-3, CFL=CFL, rampup=0, DLM=0.0, lambda_=1.0, scheme=scheme)
+        sim.set_velocity(*u)
+        orc.set_velocity(*u)
+        sim.timestep(1e-3)
+        orc.timestep(1e-3)
+        for a, b in zip(sim.velocity(), orc.velocity()):
+            assert rel_l2(a, b) < 1e-12, CFL
+        sim.close()
