@@ -2268,13 +2268,27 @@ int adjoint_upwind_f32(cup_handle* H, void* const* un, void* const* st1, void* c
   return launch_adjoint_f2_sized<true, 4, 4, 1>(H, "adjoint_stage1", un, mu, lam, lam, 0.5, 1.0, dt);
 }
 
+// The projection reads its fields in 16-byte pieces: *in = f, or `copy` with the
+// fields copied there when one of them lies between such boundaries.
+template <typename T>
+int aligned_fields(cup_handle* H, void* const* f, void* const* copy, void* const** in) {
+  *in = f;
+  if (((uintptr_t)f[0] | (uintptr_t)f[1] | (uintptr_t)f[2]) % 16 == 0) return CUP_OK;
+  for (int q = 0; q < 3; ++q)
+    CK(cudaMemcpyAsync(copy[q], f[q], H->n * sizeof(T), cudaMemcpyDeviceToDevice, H->stream));
+  *in = copy;
+  return CUP_OK;
+}
+
 template <typename T>
 int do_adjoint_step(cup_handle* H, void* const* un, void* const* lam, DtArg dt) {
   constexpr bool F32 = std::is_same<T, float>::value;
   int rc;
   void* mu[3] = {H->au, H->av, H->aw};
   if (H->cfg.scheme == CUP_SCHEME_REF) {
-    if ((rc = do_project_fields<T>(H, lam, mu, H->p_adj, dt))) return rc;
+    void* const* in;
+    if ((rc = aligned_fields<T>(H, lam, mu, &in))) return rc;
+    if ((rc = do_project_fields<T>(H, in, mu, H->p_adj, dt))) return rc;
     if constexpr (F32) return launch_adjoint<T, 0, false, 4, 3, 2>(H, "adjoint_ref", un, mu, nullptr, lam, 0.0, 1.0, dt);
     else return launch_adjoint<T, 0, false, 2, 3, 1>(H, "adjoint_ref", un, mu, nullptr, lam, 0.0, 1.0, dt);
   }
@@ -2339,7 +2353,9 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
     if (rc_) return rc_;
   }
   // 3. projection with the transposed obstacle RHS terms
-  if ((rc = do_solve_rhs_of<T>(H, "adjoint_rhs_dht_x", "adjoint_dht_x", lam, H->p_adj, dt))) return rc;
+  void* const* in;
+  if ((rc = aligned_fields<T>(H, lam, mu, &in))) return rc;
+  if ((rc = do_solve_rhs_of<T>(H, "adjoint_rhs_dht_x", "adjoint_dht_x", in, H->p_adj, dt))) return rc;
   const double kappa = dtv * dtv / (H->h * H->h * H->h);  // dJ/db2 = kappa q
   {
     int rc_ = launch_named(H, "adjoint_rhs_obstacle", [&]() -> int {
@@ -2360,7 +2376,7 @@ int do_adjoint_step_obstacle(cup_handle* H, void* const* un, void* const* lam, D
   }
   // 4. gradient correction, then the advection transposes
   if (H->cfg.scheme == CUP_SCHEME_REF) {
-    if ((rc = launch_grad<T, false>(H, "adjoint_grad_p", lam, mu, H->p_adj, dt))) return rc;
+    if ((rc = launch_grad<T, false>(H, "adjoint_grad_p", in, mu, H->p_adj, dt))) return rc;
     if constexpr (F32) return launch_adjoint<T, 0, false, 4, 3, 2>(H, "adjoint_ref", un, mu, nullptr, lam, 0.0, 1.0, dt);
     else return launch_adjoint<T, 0, false, 2, 3, 1>(H, "adjoint_ref", un, mu, nullptr, lam, 0.0, 1.0, dt);
   }
@@ -3307,6 +3323,14 @@ static int check_adjoint_fields(cup_handle* H, const void* un, const void* vn, c
       if (st[a] == lm[b]) return fail(H, CUP_ERR_ARG, "the state and the adjoint fields must not alias");
       if (a < b && (lm[a] == lm[b] || st[a] == st[b])) return fail(H, CUP_ERR_ARG, "field pointers must be distinct");
     }
+  // TMA reads the state, and the upwind3 transposes read and write the adjoint
+  // fields in pieces of up to 16 bytes (the central scheme stores single values)
+  const uintptr_t es = H->fp32 ? sizeof(float) : sizeof(double);
+  const uintptr_t al = H->cfg.scheme == CUP_SCHEME_REF ? es : 16;
+  for (int a = 0; a < 3; ++a) {
+    if ((uintptr_t)st[a] % 16) return fail(H, CUP_ERR_ARG, "the state's fields must be aligned to 16 bytes");
+    if ((uintptr_t)lm[a] % al) return fail(H, CUP_ERR_ARG, "the adjoint fields must be aligned to %d bytes", (int)al);
+  }
   return CUP_OK;
 }
 

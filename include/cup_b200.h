@@ -279,6 +279,8 @@ int cup_prepare_run(struct cup_handle* h, int nsteps, int* captured);
  * must not alias the state. Upwind signs are frozen at the state; the projection
  * is applied as the exact (FP64 FFT) symmetric projector. The handle's own
  * velocity and pressure are untouched; its stage and RHS scratch are overwritten.
+ * un, vn, wn are aligned to 16 bytes, and so are lu, lv, lw with the upwind3 scheme
+ * (central scheme: to their type), else CUP_ERR_ARG.
  * Handles with an obstacle return CUP_ERR_ARG; handles with spectral forcing on
  * return CUP_ERR_STATE (the forcing has no adjoint). Stream-ordered, no host sync. */
 int cup_adjoint_step(struct cup_handle* h, const void* un, const void* vn, const void* wn, double dt, void* lu,

@@ -206,3 +206,54 @@ def test_step_of_both_stability_ranges_every_line_length(oracle, cells, scheme):
         for a, b in zip(sim.velocity(), orc.velocity()):
             assert rel_l2(a, b) < 1e-12, CFL
         sim.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_dc"])
+@pytest.mark.parametrize("scheme", ["upwind3_rk2", "ref"])
+@pytest.mark.parametrize("sphere", [False, True])
+def test_adjoint_step_of_unaligned_fields(precision, scheme, sphere):
+    """Adjoint fields between 16-byte boundaries: the central scheme takes them
+    (as it takes any address of their type) with the bits of aligned ones, the
+    upwind3 scheme refuses them, and both refuse such a state, before anything
+    is launched."""
+    import torch
+    from cubismup_3d_b200 import Sphere
+    cells = (64, 32, 32)
+    sim = make_sim(cells, 1.0, nu=1e-3, lambda_=1e6, bImplicitPenalization=True, precision=precision, scheme=scheme)
+    if sphere:
+        sim.add_obstacle(Sphere(radius=0.1, position=(0.5, 0.25, 0.25), enforcedVelocity=(1.0, 0.0, 0.0),
+                                bForcedInSimFrame=(True, True, True), bFixFrameOfRef=(True, True, True)))
+    t = sim.storage_dtype
+    g = torch.Generator(device="cuda").manual_seed(2)
+    shape, n = (3,) + cells[::-1], 3 * 64 * 32 * 32
+    a, lam0 = (torch.randn(shape, generator=g, device="cuda", dtype=t) for _ in range(2))
+
+    def at(x, k):  # a copy of x that starts k elements after a 256-byte boundary
+        return torch.empty(n + 4, dtype=t, device="cuda")[k:k + n].view(shape).copy_(x)
+
+    def step(state, lam):
+        if not sphere:
+            sim.adjoint_step(state, 1e-3, lam)
+            return [lam]
+        g_chi = torch.zeros(sim.shape, dtype=torch.float64, device="cuda")
+        g_vel = torch.zeros(3, dtype=torch.float64, device="cuda")
+        sim.adjoint_step_obstacle(state, 1e-3, lam, (1.0, 0.0, 0.0), g_chi, g_vel)
+        return [lam, g_chi, g_vel]
+
+    want = step(a, at(lam0, 0))
+    for k in (1, 2, 3):
+        lam = at(lam0, k)
+        if lam.data_ptr() % 16 == 0:
+            continue
+        if scheme == "ref":
+            for x, y in zip(step(a, lam), want):
+                assert torch.equal(x, y)
+        else:
+            with pytest.raises(ValueError):
+                step(a, lam)
+            assert torch.equal(lam, lam0)
+    lam = at(lam0, 0)
+    with pytest.raises(ValueError):
+        step(at(a, 1), lam)
+    assert torch.equal(lam, lam0)
+    sim.close()
