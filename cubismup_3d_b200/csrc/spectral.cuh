@@ -67,13 +67,15 @@ __global__ void __launch_bounds__(128) k_dht_z_modes(const __grid_constant__ CUt
   const long long nyq2 = (long long)mp.nyquist * mp.nyquist;
   double acc[3] = {0, 0, 0};
   uint32_t ph = 0;
+  bool ok = true;
   for (int i = blockIdx.x; i < ntiles; i += gridDim.x, ph ^= 1) {
     const int x0 = (i % ntx) * W, y = i / ntx;
     if (tid == 0) {
       mbar_arrive_expect_tx(bar, (uint32_t)(3 * N * W * sizeof(double)));
       for (int c = 0; c < 3; ++c) tma_load_3d(tile + c * N * W, &map, x0, y, c * N, bar);
     }
-    if (!__syncthreads_and(mbar_wait(bar, ph, err))) return;
+    ok = __syncthreads_and(mbar_wait(bar, ph, err));
+    if (!ok) break;
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
       ColLines<double> A{tile + c * N * W, W};
@@ -136,6 +138,8 @@ __global__ void __launch_bounds__(128) k_dht_z_modes(const __grid_constant__ CUt
     fence_proxy_async_smem();
     __syncthreads();
   }
+  // after a timed-out wait: bounded drain of the tile's loads, which write to this block's shared memory
+  if (!ok && tid == 0) mbar_wait(bar, ph, nullptr);
   block_reduce<3, false>(acc, scratch);
   const int stride = 3 + mp.nbin;
   if (tid == 0)
