@@ -302,7 +302,7 @@ def adjoint_cost(torch, sim, stream, reps: int = 10) -> dict:
     # forward and backward time per step, the checkpoint interval chosen by the
     # memory budget (every state kept: no recomputation) and K = 8 (one
     # forward recompute per step in the backward)
-    from cubismup_3d_b200.adjoint import _auto_interval, rollout
+    from cubismup_3d_b200.adjoint import _interval, rollout
     n = 16
     u0 = sim.velocity_raw()
     for label, K in (("auto", None), ("K8", 8)):
@@ -317,7 +317,7 @@ def adjoint_cost(torch, sim, stream, reps: int = 10) -> dict:
             e[2].record(stream)
             torch.cuda.synchronize()
         f_ms, b_ms = e[0].elapsed_time(e[1]) / n, e[1].elapsed_time(e[2]) / n
-        out[f"rollout_{label}"] = {"steps": n, "checkpoint_every": K if K else _auto_interval(sim, n),
+        out[f"rollout_{label}"] = {"steps": n, "checkpoint_every": K if K else _interval(sim, n),
                                    "forward_ms_per_step": f_ms, "backward_ms_per_step": b_ms,
                                    "backward_over_forward": b_ms / f_ms,
                                    "backward_over_forward_step": b_ms / fwd}

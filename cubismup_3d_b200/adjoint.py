@@ -13,8 +13,8 @@ the segment's checkpoint, recomputes the segment's states forward and applies
 the adjoint steps in reverse. Peak extra memory is (n/K + K) velocity fields
 for n steps and checkpoint interval K, so long rollouts fit in HBM. By default
 (``checkpoint_every=None``) K is the smallest interval whose checkpoints fit
-in half of the device's free memory, or 1 when every state fits into what
-torch's allocator holds unused: K = 1 (every state kept, no
+in half of the device's free memory, or 1 when every state fits into half of
+what torch's allocator holds unused: K = 1 (every state kept, no
 recomputation, the backward is the adjoint steps alone) whenever the rollout
 fits, which on a 180 GB device covers the benchmark rollouts with room to
 spare.
@@ -58,9 +58,10 @@ def checkpoint_interval(nsteps: int, state_bytes: int, budget_bytes: int) -> int
     raise MemoryError(f"a {nsteps}-step rollout of {state_bytes}-byte states does not fit {budget_bytes} bytes")
 
 
-def _auto_interval(sim: Simulation, nsteps: int) -> int:
+def _auto_interval(sim: Simulation, nsteps: int, rest: int = 0) -> int:
+    """``rest``: further fields of a state's size that torch's unused memory has to hold for K = 1."""
     state = 3 * sim.storage_dtype.itemsize * int(torch.Size(sim.shape).numel())
-    # Every state fits into memory that torch already holds and uses for nothing
+    # Every state (and the rest) fits into memory that torch already holds and uses for nothing
     # (whole segments: it can hand them out or give them back to the device): K =
     # 1, as the driver's figure could not lower it. That figure takes a driver
     # call of 0.1-1 ms, tens of ms on a busy host; a gradient whose blocks a
@@ -69,10 +70,19 @@ def _auto_interval(sim: Simulation, nsteps: int) -> int:
     m = torch.cuda.memory_stats(sim.sd.device)
     cached = (m.get("reserved_bytes.all.current", 0) - m.get("active_bytes.all.current", 0)
               - m.get("inactive_split_bytes.all.current", 0))
-    if nsteps * state <= cached:
+    if (nsteps + rest) * state <= cached:
         return 1
     free, _ = torch.cuda.mem_get_info(sim.sd.device)
     return checkpoint_interval(nsteps, state, free // 2)
+
+
+def _interval(sim: Simulation, nsteps: int) -> int:
+    """K of a gradient. The states may take half of the memory they are counted
+    against, torch's or the device's: the other half is for the adjoint fields,
+    the gradients, what the caller computes between forward and backward (four
+    states' worth at least, where there are fewer steps), and for what cannot be
+    handed out (torch counts the unused memory of graph pools as well)."""
+    return _auto_interval(sim, nsteps, rest=max(nsteps, 4))
 
 
 class Rollout(torch.autograd.Function):
@@ -84,7 +94,7 @@ class Rollout(torch.autograd.Function):
             raise ValueError("rollout: the discrete adjoint does not support obstacles")
         if sim.forcing:
             raise ValueError("rollout: spectral forcing has no discrete adjoint")
-        K = _auto_interval(sim, len(dts)) if checkpoint_every is None else int(checkpoint_every)
+        K = _interval(sim, len(dts)) if checkpoint_every is None else int(checkpoint_every)
         if K < 1:
             raise ValueError("checkpoint_every must be >= 1")
         dts = [float(d) for d in dts]
@@ -135,7 +145,7 @@ def obstacle_gradients(sim: Simulation, u0: torch.Tensor, dts: Sequence[float], 
         raise ValueError("obstacle_gradients: the simulation has no obstacle")
     if sim.forcing:
         raise ValueError("obstacle_gradients: spectral forcing has no discrete adjoint")
-    K = _auto_interval(sim, len(dts)) if checkpoint_every is None else int(checkpoint_every)
+    K = _interval(sim, len(dts)) if checkpoint_every is None else int(checkpoint_every)
     if K < 1:
         raise ValueError("checkpoint_every must be >= 1")
     dts = [float(d) for d in dts]

@@ -110,3 +110,33 @@ def test_auto_checkpoint_interval_uses_cached_memory(monkeypatch):
     assert adjoint._auto_interval(sim, 11) == 2 and asked == [0]  # 6 checkpoints + 1 state in 96000
     monkeypatch.setattr(torch.cuda, "memory_stats", lambda d: {})  # an allocator without these figures
     assert adjoint._auto_interval(sim, 8) == 1 and len(asked) == 2
+
+
+def test_checkpoint_interval_of_a_gradient_leaves_headroom(monkeypatch):
+    """A rollout keeps every state without asking the driver only when torch's
+    unused memory holds them twice (and four more at least): the adjoint fields,
+    the gradients and the caller's loss need room too."""
+    import types
+    import torch
+    from cubismup_3d_b200 import adjoint
+    u = torch.zeros(3, 10, 10, 10)
+    kept, asked = [], []
+    sim = types.SimpleNamespace(sd=types.SimpleNamespace(device=0), shape=(10, 10, 10), storage_dtype=torch.float32,
+                                obstacles=[], forcing=False, step=0, time=0.0,
+                                bind_torch_stream=lambda: None, set_velocity_raw=lambda t: None,
+                                velocity_raw=lambda: kept.append(1) or u.clone(), _advance=lambda dt: None)
+
+    def checkpoints(n):
+        kept.clear(), asked.clear()
+        adjoint.rollout(sim, u, [0.1] * n)
+        return len(kept) - 1  # the last one is the result
+
+    # 10 states of 12000 bytes unused in torch's cache; half of the device's free memory holds 4
+    monkeypatch.setattr(torch.cuda, "memory_stats", lambda d: {"reserved_bytes.all.current": 120_000})
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda d: asked.append(d) or (8 * 12_000, 1 << 30))
+    assert checkpoints(5) == 5 and not asked
+    assert checkpoints(6) == 3 and asked == [0]  # K = 2: 3 checkpoints and 1 recomputed state
+    assert checkpoints(4) == 4 and not asked
+    monkeypatch.setattr(torch.cuda, "memory_stats", lambda d: {"reserved_bytes.all.current": 5 * 12_000})
+    assert checkpoints(1) == 1 and not asked     # 1 + 4 states
+    assert checkpoints(2) == 2 and asked == [0]
