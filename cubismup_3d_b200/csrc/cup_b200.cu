@@ -3440,8 +3440,10 @@ int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
       if ((rc = read_state(H))) return rc;
       if ((rc = cup_step(H, H->hstate->dt, nullptr))) return rc;
     }
-    if (stats) return fill_stats(H, stats);
-    return CUP_OK;
+    if (!stats) return CUP_OK;
+    rc = fill_stats(H, stats);
+    if (nsteps) stats->dt = H->dt;  // the last step's (the device state holds the next one's)
+    return rc;
   }
   for (int i = 0; i < nsteps;) {
     // (the dt of step i > 0 comes from the end of step i - 1)
@@ -3458,7 +3460,7 @@ int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
       }
     }
     rc = DISPATCH_T(H, do_step, DtArg{0.0, &H->dstate->dt}, (const double*)&H->dstate->lambda, 1,
-                    H->forcing || i + 1 < nsteps ? 1 : 0);
+                    i + 1 < nsteps ? 1 : 0);
     if (rc) return rc;
     H->steps_run += 1;
     if (H->forcing) {  // the host has this step's dt
@@ -3470,10 +3472,8 @@ int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
   if ((rc = read_state(H))) return rc;
   H->step = H->hstate->step;
   H->time = H->hstate->time;
-  if (!H->forcing) {  // (with forcing, each step's injection has read them)
-    H->dt = H->hstate->dt;
-    if (H->cfg.DLM > 0) H->lambda = H->hstate->lambda;
-  }
+  H->dt = H->hstate->dt;
+  if (H->cfg.DLM > 0) H->lambda = H->hstate->lambda;
   if (stats) return fill_stats(H, stats);
   return CUP_OK;
 }

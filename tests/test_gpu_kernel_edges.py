@@ -257,3 +257,41 @@ def test_adjoint_step_of_unaligned_fields(precision, scheme, sphere):
         step(at(a, 1), lam)
     assert torch.equal(lam, lam0)
     sim.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_dc"])
+@pytest.mark.parametrize("kind", ["free", "forced", "moving"])
+def test_run_steps_like_single_steps(precision, kind, tmp_path, monkeypatch):
+    """run_steps chains dt on the device (forced runs read it back with the mode
+    sums, runs with a moving sphere before each step): the same launches with
+    the same dt as calcMaxTimestep + timestep, so the same bits, clock and
+    statistics, dt being the last step's."""
+    import ctypes as C
+    from cubismup_3d_b200 import Sphere, _lib as L
+    monkeypatch.chdir(tmp_path)  # timestep of a forced run writes forcingData.dat
+    cells, n = (64, 32, 32), 5
+    u = [0.2 * c for c in np.random.default_rng(8).standard_normal((3,) + cells[::-1])]
+    out = []
+    for chained in (True, False):
+        kw = {"forced": dict(turbKinEn_target=0.1), "moving": dict(lambda_=1e6, bImplicitPenalization=True)}.get(kind, {})
+        sim = make_sim(cells, 2 * np.pi if kind == "forced" else 1.0, nu=1e-3, precision=precision,
+                       scheme="upwind3_rk2", **kw)
+        if kind == "moving":
+            sim.add_obstacle(Sphere(radius=0.1, position=(0.5, 0.25, 0.25), enforcedVelocity=(1.0, 0.0, 0.0),
+                                    bForcedInSimFrame=(True, True, True)))
+        sim.set_velocity(*u)
+        if chained:
+            st = sim.run_steps(n)
+        else:
+            for _ in range(n):
+                st = sim.timestep(sim.calcMaxTimestep())
+        assert sim.dt == st.dt and sim.step == st.step == n and sim.time == st.time
+        forcing = (C.c_double * 6)()
+        L.check(L.lib().cup_get_forcing_stats(sim._h, forcing), sim._h, "forcing stats")
+        assert (forcing[0] > 0) == (kind == "forced")  # totalKinEn of the last step's forcing
+        out.append((st.dt, st.time, st.umax, st.kinetic_energy, list(st.force) + forcing[:], sim.velocity(), sim.calcMaxTimestep()))
+        sim.close()
+    a, b = out
+    assert a[:5] == b[:5] and a[6] == b[6]
+    for x, y in zip(a[5], b[5]):
+        assert np.array_equal(x, y)
