@@ -1156,12 +1156,10 @@ int hartley_finish(cup_handle* H, const char* name_x, double* work, double* out)
 bool amplifies_rounding(const cup_handle* H) { return !H->fp32 && H->cfg.CFL > 0.125; }
 
 // p = f . b over the three axes, FP64, the RHS in `work` (overwritten). Handles
-// whose steps can amplify rounding (amplifies_rounding) run the Hartley passes,
-// and one whose z pass belongs to a pencil of a decomposed grid
-// (cup_set_spectral_window) those that the decomposed solve uses.
+// whose steps can amplify rounding (amplifies_rounding) run the Hartley passes.
 int fft_poisson(cup_handle* H, double* work, double* out) {
   int rc;
-  if (H->spec_ny != H->ny || amplifies_rounding(H)) {
+  if (amplifies_rounding(H)) {
     if ((rc = launch_rows_pipe(H, "dht_x", work))) return rc;
     return hartley_finish(H, "dht_x", work, out);
   }
@@ -1623,23 +1621,10 @@ template <typename T>
 int do_solve_rhs_of(cup_handle* H, const char* name_rhs, const char* name_x, void* const* f, double* out, DtArg dt,
                     bool box = false) {
   if constexpr (std::is_same<T, double>::value)
-    if (amplifies_rounding(H) && H->spec_ny == H->ny && !box) {
+    if (amplifies_rounding(H) && !box) {
       int rc = launch_rows_rhs<T>(H, name_rhs, f, H->rhs, dt);
       return rc ? rc : hartley_finish(H, name_x, H->rhs, out);
     }
-  if (H->spec_ny != H->ny) {
-    const void* cf[3] = {f[0], f[1], f[2]};
-    OpPressureRHS<T> op{H->rhs, dt, H->h, H->nx, H->ny};
-    int rc = launch_stream<T, 3, 1, 4, 4>(H, "pressure_rhs", cf, op);
-    if (!rc && box)
-      rc = launch_named(H, "box_add", [&]() -> int {
-        klaunch(H, k_box_add, box_grid(H->box), kBoxThreads, 0, H->rhs, (const double*)H->box_delta, H->box, H->nx,
-                H->ny, H->nz);
-        CKL();
-        return CUP_OK;
-      });
-    return rc ? rc : fft_poisson(H, H->rhs, out);
-  }
   int rc = launch_pfft_x_rhs<T>(H, name_rhs, f, H->rhs, dt, box);
   return rc ? rc : pfft_finish(H, name_x, H->rhs, out);
 }
@@ -2582,6 +2567,14 @@ int run_graph(cup_handle* H, int nsteps, int next_dt, bool* ran) {
       return fail(H, CUP_ERR_STATE, "%s needs a whole grid (this handle holds a z-slab)", __func__); \
   } while (0)
 
+// Entry points that solve on the handle's own grid refuse a handle whose z pass
+// is that of a pencil of a larger grid (cup_set_spectral_window).
+#define REQUIRE_OWN_SPECTRUM(H)                                                                               \
+  do {                                                                                                        \
+    if ((H)->spec_ny != (H)->ny)                                                                              \
+      return fail(H, CUP_ERR_STATE, "%s needs the handle's own spectrum (it has a spectral window)", __func__); \
+  } while (0)
+
 extern "C" {
 
 int cup_create(const cup_config* cfg, cup_handle** out) {
@@ -2972,6 +2965,7 @@ int cup_set_graphs(cup_handle* H, int on) {
 int cup_prepare_run(cup_handle* H, int nsteps, int* captured) {
   REQUIRE_H(H);
   REQUIRE_WHOLE_GRID(H);
+  REQUIRE_OWN_SPECTRUM(H);
   if (captured) *captured = 0;
   if (nsteps < 0) return fail(H, CUP_ERR_ARG, "nsteps must be >= 0");
   if (!graph_ok(H)) return CUP_OK;
@@ -3179,6 +3173,7 @@ int cup_poisson_pass(cup_handle* H, double* buf, int pass) {
 int cup_poisson_solve(cup_handle* H, cup_solve_stats* stats) {
   REQUIRE_H(H);
   REQUIRE_WHOLE_GRID(H);
+  REQUIRE_OWN_SPECTRUM(H);
   reset_pressure_history(H);
   int rc = do_poisson(H);
   if (rc) return rc;
@@ -3265,6 +3260,7 @@ static int fill_stats(cup_handle* H, cup_step_stats* st) {
 int cup_step(cup_handle* H, double dt, cup_step_stats* stats) {
   REQUIRE_H(H);
   REQUIRE_WHOLE_GRID(H);
+  REQUIRE_OWN_SPECTRUM(H);
   if (!(dt > 0)) return fail(H, CUP_ERR_ARG, "dt must be > 0");
   H->dt = dt;
   if (H->cfg.DLM > 0) H->lambda = H->cfg.DLM / dt;
@@ -3338,6 +3334,7 @@ int cup_adjoint_step(cup_handle* H, const void* un, const void* vn, const void* 
                      void* lw) {
   REQUIRE_H(H);
   REQUIRE_WHOLE_GRID(H);
+  REQUIRE_OWN_SPECTRUM(H);
   if (!(dt > 0)) return fail(H, CUP_ERR_ARG, "dt must be > 0");
   if (H->has_sphere) return fail(H, CUP_ERR_ARG, "cup_adjoint_step: the handle has an obstacle (use cup_adjoint_step_obstacle)");
   if (H->forcing)
@@ -3354,6 +3351,7 @@ int cup_adjoint_step_obstacle(cup_handle* H, const void* un, const void* vn, con
                               void* lv, void* lw, const double w_force[3], double* g_chi, double* g_vel) {
   REQUIRE_H(H);
   REQUIRE_WHOLE_GRID(H);
+  REQUIRE_OWN_SPECTRUM(H);
   if (!(dt > 0)) return fail(H, CUP_ERR_ARG, "dt must be > 0");
   if (!H->has_sphere) return fail(H, CUP_ERR_ARG, "cup_adjoint_step_obstacle: the handle has no obstacle");
   if (H->sphere_moves)
@@ -3419,6 +3417,7 @@ int cup_set_velocity_raw(cup_handle* H, const void* u, const void* v, const void
 int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
   REQUIRE_H(H);
   REQUIRE_WHOLE_GRID(H);
+  REQUIRE_OWN_SPECTRUM(H);
   if (nsteps < 0) return fail(H, CUP_ERR_ARG, "nsteps must be >= 0");
   int rc;
   if (!H->umax_fresh) {
@@ -3481,6 +3480,7 @@ int cup_run(cup_handle* H, int nsteps, cup_step_stats* stats) {
 int cup_poisson_solve_field(cup_handle* H, const double* rhs, double* p, int where) {
   REQUIRE_H(H);
   REQUIRE_WHOLE_GRID(H);
+  REQUIRE_OWN_SPECTRUM(H);
   reset_pressure_history(H);
   if (!rhs || !p || !valid_where(where)) return fail(H, CUP_ERR_ARG, "bad poisson arguments");
   const cudaMemcpyKind in = where == CUP_WHERE_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
@@ -3495,7 +3495,7 @@ int cup_poisson_solve_field(cup_handle* H, const double* rhs, double* p, int whe
     return x + bytes <= y || y + bytes <= x;
   };
   int rc;
-  if (where == CUP_WHERE_DEVICE && !H->fp32 && H->spec_ny == H->ny && (uintptr_t)rhs % 16 == 0 &&
+  if (where == CUP_WHERE_DEVICE && !H->fp32 && (uintptr_t)rhs % 16 == 0 &&
       (uintptr_t)p % 16 == 0 && apart(p, H->rhs) && apart(p, H->p) && (rhs == H->rhs || apart(rhs, H->rhs))) {
     if ((rc = launch_pfft_x<double, PROW_FWD>(H, "dht_x", rhs, H->rhs, nullptr, 0, nullptr))) return rc;
     if ((rc = pfft_finish(H, "dht_x", H->rhs, H->p, p))) return rc;

@@ -284,18 +284,6 @@ __device__ __forceinline__ double div_b(double facB, T dxy, T wzp, T wzm) {
   return facB * (double)(dxy + (wzp - wzm));
 }
 
-// f += d on a box (d in box order).
-__global__ void k_box_add(double* f, const double* d, Box box, int nx, int ny, int nz) {
-  pdl_entry();
-  const long long n = box.count();
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int x = wrapi(box.lo[0] + (int)(i % box.n[0]), nx);
-    const int y = wrapi(box.lo[1] + (int)((i / box.n[0]) % box.n[1]), ny);
-    const int z = wrapi(box.lo[2] + (int)(i / ((long long)box.n[0] * box.n[1])), nz);
-    f[gidx(x, y, z, nx, ny)] += d[i];
-  }
-}
-
 // The first half of the RHS obstacle terms on the box, for passes that form
 // b0 = KernelPressureRHS(u*) (source/operators/PressureRHS.cpp:51-76)
 // themselves: b0 at each box cell into d, b1 = b0 - chi b0 into b (box

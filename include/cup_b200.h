@@ -232,7 +232,9 @@ int cup_poisson_reset(struct cup_handle* h);
  * spectral divide is local too; a second all-to-all and the y and x passes
  * finish. cubismup_3d_b200/slab.py orchestrates it over torch.distributed. */
 /* Makes the handle's z pass that of the pencil y in [y0, y0 + ny) of a grid
- * ny_global cells long in y (the global cos table, null modes and 1/N). */
+ * ny_global cells long in y (the global cos table, null modes and 1/N). A handle
+ * with such a window (ny_global other than its ny) runs single passes only: whole
+ * solves and steps return CUP_ERR_STATE. */
 int cup_set_spectral_window(struct cup_handle* h, int y0, int ny_global);
 /* One FP64 pass of the Poisson solve, in place on the device array buf of the
  * handle's nx*ny*nz cells ([z][y][x]): pass 0 the Hartley transform of every

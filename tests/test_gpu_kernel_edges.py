@@ -295,3 +295,37 @@ def test_run_steps_like_single_steps(precision, kind, tmp_path, monkeypatch):
     assert a[:5] == b[:5] and a[6] == b[6]
     for x, y in zip(a[5], b[5]):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_dc"])
+def test_whole_solves_refuse_a_spectral_window(precision):
+    """A handle whose z pass is that of a pencil of a larger grid refuses whole
+    solves and steps before it changes anything; its single passes run, and a
+    window of its own grid gives the solves back."""
+    import ctypes as C
+    import torch
+    from cubismup_3d_b200 import _lib as L
+    cells = (32, 16, 16)
+    sim = make_sim(cells, 1.0, nu=1e-3, precision=precision)
+    sim.bind_torch_stream()
+    u = np.random.default_rng(1).standard_normal((3,) + cells[::-1])
+    sim.set_velocity(*u)
+    before = sim.velocity_raw()
+    H, lib = sim._h, L.lib()
+    L.check(lib.cup_set_spectral_window(H, 16, 32), H, "window")
+    rhs, p = (torch.ones(sim.shape, dtype=torch.float64, device="cuda") for _ in range(2))
+    lam, count = torch.zeros_like(before), C.c_int()
+    for call in (lambda: lib.cup_step(H, 1e-3, None), lambda: lib.cup_run(H, 1, None),
+                 lambda: lib.cup_prepare_run(H, 1, C.byref(count)), lambda: lib.cup_poisson_solve(H, None),
+                 lambda: lib.cup_pressure_projection(H, 1e-3, None),
+                 lambda: lib.cup_poisson_solve_field(H, C.c_void_p(rhs.data_ptr()), C.c_void_p(p.data_ptr()),
+                                                     L.CUP_WHERE_DEVICE),
+                 lambda: lib.cup_adjoint_step(H, *[C.c_void_p(before[i].data_ptr()) for i in range(3)], 1e-3,
+                                              *[C.c_void_p(lam[i].data_ptr()) for i in range(3)])):
+        assert call() == L.CUP_ERR_STATE
+    assert torch.equal(sim.velocity_raw(), before) and torch.equal(p, torch.ones_like(p))
+    L.check(lib.cup_poisson_pass(H, C.c_void_p(rhs.data_ptr()), 2), H, "pass")
+    L.check(lib.cup_set_spectral_window(H, 0, 16), H, "window")
+    sim.timestep(1e-3)
+    assert np.isfinite(sim.velocity_raw().cpu().numpy()).all()
+    sim.close()
