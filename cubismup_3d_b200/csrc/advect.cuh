@@ -40,8 +40,7 @@
 namespace cup {
 
 struct AdvectMaps {
-  RowMaps f[3];         // stencil fields
-  CUtensorMap base[3];  // (k_advect_zq_f2, stage 2) point-wise fields, box {nx, TY, 1}
+  RowMaps f[3];  // stencil fields
 };
 
 // SCHEME 0: central2 (reference) Euler; 1: upwind3 stage 1; 2: upwind3 stage 2.

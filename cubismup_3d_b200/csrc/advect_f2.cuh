@@ -51,6 +51,11 @@ __device__ __forceinline__ float2 apply5(const Weights5& k, float2 fm2, float2 f
   return fma2(k.m2, fm2, fma2(k.m1, fm1, fma2(k.c0, f0, fma2(k.p1, fp1, mul2(k.p2, fp2)))));
 }
 
+struct AdvectF2Maps {
+  RowMaps f[3];         // stencil fields
+  CUtensorMap base[3];  // (stage 2) point-wise fields, box {nx, TY, 1}
+};
+
 // Ring bytes: TY + 4 rows of the three fields per slot, in stage 2 also TY rows of u^n.
 template <bool STAGE2, int TY, int NS>
 constexpr size_t advect_f2_smem_bytes(int nx) {
@@ -62,7 +67,7 @@ constexpr size_t advect_f2_smem_bytes(int nx) {
 // NXC: nx fixed at compile time (0: read from g): every shared-memory offset of
 // the stencil is then an immediate on a per-thread base register.
 template <bool STAGE2, int TY, int NS, int PPT, int NXC = 0>
-__global__ void __launch_bounds__(512) k_advect_zq_f2(const __grid_constant__ AdvectMaps maps, const StreamGeom g,
+__global__ void __launch_bounds__(512) k_advect_zq_f2(const __grid_constant__ AdvectF2Maps maps, const StreamGeom g,
                                                      float* __restrict__ ou, float* __restrict__ ov,
                                                      float* __restrict__ ow, DtArg dt, double h, double nu, double ux,
                                                      double uy, double uz, int* err) {

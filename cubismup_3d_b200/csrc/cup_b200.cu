@@ -963,8 +963,7 @@ int launch_cols_M(cup_handle* H, double* buf, int nf) {
   const int grid = std::min(ntiles, bpsm * H->num_sms);
   SpectralParams sp{H->cosx, H->cosy, H->cosz, H->norm_factor, H->nx, H->spec_ny, H->nz, H->spec_y0};
   return launch_named(H, AXIS == 1 ? "dht_y" : "dht_z_solve", [&]() -> int {
-    klaunch(H, kern, grid, threads, smem, map, ntx, ntiles, (const double2*)H->tw64[AXIS], sp, H->derr,
-            (const int*)nullptr);
+    klaunch(H, kern, grid, threads, smem, map, ntx, ntiles, (const double2*)H->tw64[AXIS], sp, H->derr);
     CKL();
     return CUP_OK;
   });
@@ -1080,7 +1079,7 @@ int launch_pfft_z_M(cup_handle* H, const char* name, T* in, double* out, const i
   const int grid = std::min(ntiles, bpsm * H->num_sms);
   const PSpectral sp{H->pcos[0], H->pcos[1], H->pcos[2], H->pnorm};
   return launch_named(H, name, [&]() -> int {
-    klaunch(H, kern, grid, Tile::THREADS, smem, map_in, map_out, ntx, ntiles, 0, ptable<T>(H, 2),
+    klaunch(H, kern, grid, Tile::THREADS, smem, map_in, map_out, ntx, ntiles, ptable<T>(H, 2),
             (const double2*)H->ptw64[2], sp, H->derr, skip);
     CKL();
     return CUP_OK;
@@ -1233,7 +1232,6 @@ int launch_advect_sized(cup_handle* H, const char* name, void* const* in, void* 
   for (int f = 0; f < 3; ++f) {
     int rc = make_row_maps<T>(H, &maps.f[f], in[f], TY, G);
     if (rc) return rc;
-    maps.base[f] = maps.f[f].main;
   }
   if (NXC && NXC != H->nx) return fail(H, CUP_ERR_ARG, "advection specialisation mismatch");
   const size_t smem = advect_smem_bytes<T, SCHEME, TY, NS>(H->nx) + 128;
@@ -1272,7 +1270,7 @@ int launch_advect_f2(cup_handle* H, const char* name, void* const* in, void* con
   constexpr int G = 2;
   const int pairs = TY * H->nx / 2;
   if (pairs % PPT || pairs / PPT > 512 || H->ny % TY) return fail(H, CUP_ERR_ARG, "advection tile does not fit the grid");
-  AdvectMaps maps;
+  AdvectF2Maps maps;
   for (int f = 0; f < 3; ++f) {
     int rc = make_row_maps<float>(H, &maps.f[f], in[f], TY, G);
     if (!rc) rc = make_map(H, &maps.base[f], STAGE2 ? base[f] : in[f], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(float),

@@ -422,12 +422,6 @@ __device__ __forceinline__ void dht128_tail(const Acc& a, const AccO& ao, const 
   __syncthreads();
 }
 
-template <int M, typename R, typename R2, class Acc, class Scale = NoScale>
-__device__ __forceinline__ void dht_post(const Acc& a, const R2* twp, int l, int t, bool active,
-                                         const Scale& scale = Scale()) {
-  dht_post_to<M, R, R2>(a, a, twp, l, t, active, scale);
-}
-
 // Full in-place Hartley transform of the lines of `a` (pad: scratch for the
 // first stage's output when USE_PAD). Thread `t` of line `l`, M/8 per line.
 // The packed complex FFT stages of dht_lines (for M = 128 all but the last,
@@ -686,12 +680,11 @@ __device__ __forceinline__ ZColumnFactor z_column_factor(const SpectralParams& s
 template <int M, typename R, int AXIS, bool DIVIDE, int W, int NB, bool T8 = false>
 __global__ void __launch_bounds__(W * (T8 ? 8 : M / 8)) k_dht_cols_pipe(const __grid_constant__ CUtensorMap map,
                                                        int ntiles_x, int ntiles, const typename Cplx<R>::T* tw_g,
-                                                       SpectralParams sp, int* err, const int* skip) {
+                                                       SpectralParams sp, int* err) {
   pdl_entry();
   using R2 = typename Cplx<R>::T;
   static_assert(NB >= 2, "need at least two tile buffers");
   static_assert(!T8 || M == 128, "the 8-thread plan is for 256-long lines");
-  if (skip && *skip) return;
   constexpr int N = 2 * M, TPL = T8 ? 8 : M / 8;
   constexpr int TL = FFTPlan<M>::table_len();
   constexpr uint32_t TILE_BYTES = (uint32_t)(N * W * sizeof(R));

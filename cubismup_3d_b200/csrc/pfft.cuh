@@ -322,7 +322,7 @@ __device__ __forceinline__ void p_factors(float (&f)[N_], double cxy, const doub
 template <int M, typename T, int W, int NB>
 __global__ void __launch_bounds__(PTile<M, T, W>::THREADS)
     k_pfft_z(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_out, int ntiles_x,
-             int ntiles, int rev, const typename Cplx<T>::T* tw_in_g, const double2* tw_g, PSpectral sp, int* err,
+             int ntiles, const typename Cplx<T>::T* tw_in_g, const double2* tw_g, PSpectral sp, int* err,
              const int* skip) {
   pdl_entry();
   if (skip && *skip) return;
@@ -349,8 +349,7 @@ __global__ void __launch_bounds__(PTile<M, T, W>::THREADS)
   }
   __syncthreads();
   auto coords = [&](int i, int& x0, int& y0) {
-    int t = blockIdx.x + i * gridDim.x;
-    if (rev) t = ntiles - 1 - t;
+    const int t = blockIdx.x + i * gridDim.x;
     x0 = (t % ntiles_x) * W;
     y0 = (t / ntiles_x) * P;
   };
@@ -610,8 +609,8 @@ __global__ void __launch_bounds__(32 * WARPS) k_pfft_x(const S* in, S* out, S* o
 // forms the elements m = t + R2 r of its row (cells 2m, 2m+1) from paired loads
 // of u, v, w, straight into stage A's registers. bdelta (may be nullptr): the
 // obstacle's RHS terms on its box, added there.
-template <int M, typename T, int WARPS, int MINB = 1>
-__global__ void __launch_bounds__(32 * WARPS, MINB) k_pfft_x_rhs(const T* __restrict__ u, const T* __restrict__ v_,
+template <int M, typename T, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) k_pfft_x_rhs(const T* __restrict__ u, const T* __restrict__ v_,
                                                           const T* __restrict__ w, double* __restrict__ out, DtArg dt,
                                                           double h, int ny, int nz, int ntiles,
                                                           const double2* tw_g, const Box box, const double* bdelta) {

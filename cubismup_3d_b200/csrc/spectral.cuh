@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(128) k_dht_z_modes(const __grid_constant__ CUt
     const int jj = mode_of(y, mp.ny);
     const double ky = jj * mp.wf[1];
     for (int q = tid; q < N; q += blockDim.x) {
-      const int k = q >> 1, l0 = (q & 1) * 8, k1 = k ? N - k : N / 2, kz1 = k ? k : N / 2;
+      const int k = q >> 1, l0 = (q & 1) * 8, k1 = k ? N - k : N / 2;
       int run = -1;
       double sum = 0.0;
       auto mode = [&](double E, int ii, int kk) {
@@ -122,14 +122,13 @@ __global__ void __launch_bounds__(128) k_dht_z_modes(const __grid_constant__ CUt
         const double Ea = 0.5 * (a[0] * a[0] + a[N * W] * a[N * W] + a[2 * N * W] * a[2 * N * W]);
         const double Eb = 0.5 * (b[0] * b[0] + b[N * W] * b[N * W] + b[2 * N * W] * b[2 * N * W]);
         const bool in = mode(k ? Ea + Eb : Ea, ii, k);
-        const bool in1 = k ? in : mode(Eb, ii, kz1);
+        if (!k) mode(Eb, ii, N / 2);
         if (mp.coef && abs(ii) <= mp.band[0] && abs(jj) <= mp.band[1]) {
           const int n0 = 2 * mp.band[0] + 1, n1 = 2 * mp.band[1] + 1, n2 = 2 * mp.band[2] + 1;
           for (int c = 0; c < 3; ++c) {
             double* o = mp.coef + ((size_t)c * n2 * n1 + jj + mp.band[1]) * n0 + ii + mp.band[0];
             if (k <= mp.band[2]) o[(size_t)(mp.band[2] + k) * n1 * n0] = in ? a[c * N * W] : 0.0;
-            // (the mode N/2 at +N/2 only)
-            if (kz1 <= mp.band[2]) o[(size_t)(k ? mp.band[2] - k : mp.band[2] + kz1) * n1 * n0] = in1 ? b[c * N * W] : 0.0;
+            if (k && k <= mp.band[2]) o[(size_t)(mp.band[2] - k) * n1 * n0] = in ? b[c * N * W] : 0.0;
           }
         }
       }
@@ -147,8 +146,8 @@ __global__ void __launch_bounds__(128) k_dht_z_modes(const __grid_constant__ CUt
   for (int b = tid; b < mp.nbin; b += blockDim.x) partials[(size_t)stride * blockIdx.x + 3 + b] = bins[b];
 }
 
-// The same sums from coefficients in memory, with every mode outside the
-// forcing band zeroed in place: for a band too wide to force mode by mode.
+// Every mode outside the forcing band zeroed in place, for a band too wide to
+// force mode by mode.
 __global__ void k_spectral_filter(double* hu, double* hv, double* hw, int lnx, int lny, int nz, double wfx, double wfy,
                                   double wfz) {
   pdl_entry();
