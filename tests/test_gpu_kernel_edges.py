@@ -329,3 +329,76 @@ def test_whole_solves_refuse_a_spectral_window(precision):
     sim.timestep(1e-3)
     assert np.isfinite(sim.velocity_raw().cpu().numpy()).all()
     sim.close()
+
+
+def graph_pair(cells, precision, sphere):
+    """(graphs on or off, simulation on a stream of torch's, its stream) after the four steps that make FP32-DC's history."""
+    import torch
+    from cubismup_3d_b200 import Sphere
+    u = [0.3 * c for c in np.random.default_rng(6).standard_normal((3,) + cells[::-1])]
+    for graphs in (True, False):
+        sim = make_sim(cells, 1.0, nu=1e-3, precision=precision, scheme="upwind3_rk2", lambda_=1e6,
+                       bImplicitPenalization=True)
+        if sphere:
+            sim.add_obstacle(Sphere(radius=0.1, position=(0.5, 0.25, 0.25), enforcedVelocity=(1.0, 0.0, 0.0),
+                                    bForcedInSimFrame=(True, True, True), bFixFrameOfRef=(True, True, True)))
+        sim.use_graphs(graphs)
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            sim.bind_torch_stream()
+        sim.set_velocity(*u)
+        sim.run_steps(4)
+        yield graphs, sim, stream
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_dc"])
+@pytest.mark.parametrize("sphere", [False, True])
+def test_replayed_runs_match_launched_ones(precision, sphere):
+    """Runs of 20 and 9 steps whose graphs prepare_run has captured (the 6-step
+    one is replayed three times and once, the tails one step at a time), then
+    single steps on cached graphs: the same bits, clock, statistics and launch
+    count as launching every step."""
+    out = []
+    for graphs, sim, _ in graph_pair((64, 32, 32), precision, sphere):
+        got = []
+        for n, captured in ((20, 3), (9, 4)):  # one 6-step graph and the tail's 2 or 3 steps
+            assert sim.prepare_run(n) == (captured if graphs else 0)
+            n0 = sim.launch_count()
+            st = sim.run_steps(n)
+            got += [st.step, st.time, st.dt, st.umax, st.kinetic_energy, list(st.force), sim.launch_count() - n0,
+                    np.stack(sim.velocity()), sim.pressure()]
+        for _ in range(8):
+            st = sim.timestep(sim.calcMaxTimestep())
+            got += [st.time, st.dt, st.kinetic_energy, list(st.force)]
+        out.append(got + [np.stack(sim.velocity())])
+        sim.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_dc"])
+def test_step_inside_a_capture_of_the_callers(precision):
+    """A step inside a capture of the caller's is launched into it, although the
+    handle has a graph of its own for that step; replaying the caller's graph
+    takes the step."""
+    import torch
+    out = []
+    for graphs, sim, stream in graph_pair((64, 32, 32), precision, False):
+        assert (sim.prepare_run(1) > 0) == graphs
+        if graphs:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=stream):
+                sim.timestep(1e-3, stats=False)
+            with torch.cuda.stream(stream):
+                g.replay()
+        else:
+            sim.timestep(1e-3, stats=False)
+        sim.sync()
+        first = sim.velocity()
+        st = sim.run_steps(3)
+        out.append((*first, *sim.velocity(), st.time, st.dt))
+        if graphs:
+            g.reset()
+        sim.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
