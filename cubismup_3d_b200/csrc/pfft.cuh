@@ -609,8 +609,11 @@ __global__ void __launch_bounds__(32 * WARPS) k_pfft_x(const S* in, S* out, S* o
 // forms the elements m = t + R2 r of its row (cells 2m, 2m+1) from paired loads
 // of u, v, w, straight into stage A's registers. bdelta (may be nullptr): the
 // obstacle's RHS terms on its box, added there.
+// The launch bound of one CTA per SM lets the compiler hold all of a row's loads in
+// registers (254 at M = 128); without it, it keeps to 102 and waits for them (12 FP64
+// steps at 256^3 10170 -> 10320 us).
 template <int M, typename T, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS) k_pfft_x_rhs(const T* __restrict__ u, const T* __restrict__ v_,
+__global__ void __launch_bounds__(32 * WARPS, 1) k_pfft_x_rhs(const T* __restrict__ u, const T* __restrict__ v_,
                                                           const T* __restrict__ w, double* __restrict__ out, DtArg dt,
                                                           double h, int ny, int nz, int ntiles,
                                                           const double2* tw_g, const Box box, const double* bdelta) {
