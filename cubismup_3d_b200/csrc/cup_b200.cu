@@ -932,7 +932,7 @@ int launch_rows_rhs_M(cup_handle* H, const char* name, void* const* f, double* o
   if (rc) return rc;
   return launch_named(H, name, [&]() -> int {
     klaunch(H, kern, H->ny * H->nz / lpc, 256, smem, (const T*)f[0], (const T*)f[1], (const T*)f[2], out, dt, H->h, H->ny,
-            H->nz, lpc, (const double2*)H->tw64[0]);
+            H->nz, (const double2*)H->tw64[0]);
     CKL();
     return CUP_OK;
   });
@@ -1149,8 +1149,8 @@ int hartley_finish(cup_handle* H, const char* name_x, double* work, double* out)
 // the packed transforms of the pressure, either alone, moved u by 1e-9 to 5e-7.
 // Such runs keep their arithmetic: the one-sided stencils of both signs
 // (k_advect_zq, SELECT) and the Hartley passes of dht.cuh for the pressure. An
-// upwind3 step takes 55 us then instead of 42 at 64^3, 146 instead of 117 at
-// 128^3, 975 instead of 780 at 256^3. FP32 runs take the same passes either way:
+// upwind3 step takes 48 us then instead of 42 at 64^3, 136 instead of 117 at
+// 128^3, 914 instead of 780 at 256^3. FP32 runs take the same passes either way:
 // their order of arithmetic also depends on how their sums are split.
 bool amplifies_rounding(const cup_handle* H) { return !H->fp32 && H->cfg.CFL > 0.125; }
 

@@ -28,11 +28,11 @@
 //
 // Measured at 256^3 (one B200, passes in sequence) against the Hartley passes
 // of dht.cuh, which every solve ran before and the FP64 handles of
-// amplifies_rounding still run: FP64 RHS + x 187 -> 120 us, y 49 ->
+// amplifies_rounding still run: FP64 RHS + x 187 -> 102 us, y 49 ->
 // 43, z with the divide 80 -> 53, y 49 -> 44, x 53 -> 45; mixed correction solve
 // x 38 -> 27, y 27 -> 22, z 58 -> 45, y 49 -> 44, x + p 74 -> 65.5. The column
 // passes now move their 16 B/cell at 5-6 TB/s (82-95 % of the measured copy
-// bandwidth); RHS + x waits on its loads of u, v, w (32 B/cell, 4.5 TB/s).
+// bandwidth); RHS + x waits on its loads of u, v, w (32 B/cell, 5.3 TB/s).
 #pragma once
 
 #include "common.cuh"
